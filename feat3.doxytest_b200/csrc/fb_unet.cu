@@ -37,6 +37,11 @@ namespace un
 
   __device__ __forceinline__ float bf2f(bf v) { return __uint_as_float(uint32_t(v) << 16); }
   __device__ __forceinline__ bf f2bf(float f) { return __bfloat16_as_ushort(__float2bfloat16_rn(f)); }
+  // all ones in each half of a BF16 pair that is greater than zero
+  __device__ __forceinline__ uint32_t mask2(uint32_t q)
+  {
+    return (bf2f(bf(q)) > 0.f ? 0xFFFFu : 0u) | (bf2f(bf(q >> 16)) > 0.f ? 0xFFFF0000u : 0u);
+  }
 
   constexpr int NLAYER = 10;
   struct LayerDef { int cin, cout, level; bool relu; int dil; };
@@ -62,20 +67,21 @@ namespace un
   template<int N>
   __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
 
-  __device__ __forceinline__ void ldm_x4(uint32_t (&r)[4], const void* p)
+  // ldmatrix from a shared-memory address: each lane points at one 16-byte row
+  __device__ __forceinline__ void ldm_x4a(uint32_t (&r)[4], uint32_t p)
   {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_addr(p)));
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(p));
   }
-  __device__ __forceinline__ void ldm_x4_t(uint32_t (&r)[4], const void* p)
+  __device__ __forceinline__ void ldm_x4a_t(uint32_t (&r)[4], uint32_t p)
   {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_addr(p)));
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(p));
   }
-  __device__ __forceinline__ void ldm_x2_t(uint32_t (&r)[2], const void* p)
+  __device__ __forceinline__ void ldm_x2a_t(uint32_t (&r)[2], uint32_t p)
   {
     asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
-                 : "=r"(r[0]), "=r"(r[1]) : "r"(smem_addr(p)));
+                 : "=r"(r[0]), "=r"(r[1]) : "r"(p));
   }
   __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
   {
@@ -85,291 +91,487 @@ namespace un
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
   }
 
-  // ------------------------------------------------------------------ implicit-GEMM convolution
-  // y[p, n] = act(bias[n] + sum_{tap, c} x[p + off(tap), c] * w[tap*cin + c][n]) for every pixel p of
-  // a B x H x W batch (x NHWC with cin channels, cin % 8 == 0; zero outside the grid).  w: kpad x
-  // n_ld BF16 (rows >= 9*cin are zero, kpad % 32 == 0).  Output BF16 or FP32 at [p * y_ld + y_off].
-  // The same kernel computes the data gradient (x = output gradient, w = flipped transposed weights).
-  struct ConvArgs
+  // ------------------------------------------------------------------ tiles
+  // Every convolution kernel works on T x T pixel tiles of one image (T <= 11, so that a tile's
+  // 121 pixels fill the 128 rows of an MMA tile and 33, 65 and 129 points per side divide into
+  // whole tiles with 1-5% overhang) and stages the tile's input with its halo of `dil` pixels in
+  // shared memory once.  The nine taps then read that one copy at shifted addresses: each ldmatrix
+  // lane points at its own pixel's 16-byte chunk, so no im2col copy of the input is ever made (a
+  // gather per tap reads the input nine times and spends its issue slots on address arithmetic).
+  // Pixel stride: PXC 16-byte chunks, odd, so that the eight rows of an ldmatrix fall into
+  // different banks.
+  constexpr int TMAX = 11;
+  __host__ __device__ constexpr int px_chunks(int c) { return (c / 8) | 1; }
+  __host__ __device__ constexpr int halo_dim(int dil) { return TMAX + 2 * dil; }
+  __host__ __device__ constexpr int halo_bytes(int c, int dil)
   {
-    const bf* x;
-    const bf* w;
-    const float* bias;     // nb entries (columns >= nb get no bias)
-    void* y;
-    int cin, kpad, n, n_ld, nb;
-    int B, H, W, dil;
-    int y_ld, y_off;
-    int relu, out_bf16;
+    return halo_dim(dil) * halo_dim(dil) * px_chunks(c) * 16;
+  }
+
+  struct Tiling
+  {
+    int G, T, nt;        // points per side, tile side, tiles per side
   };
 
-  constexpr int CBM = 128, CBK = 32, CNT = 128;
+  // where a convolution's input comes from
+  enum InMode
+  {
+    IN_PLAIN,            // BF16 [B][G][G][C]
+    IN_SUB,              // injection: every other vertex of BF16 [B][2G-1][2G-1][C]
+    IN_CAT,              // [U(coarse), skip]: the first cu channels are the bilinear vertex
+                         // upsampling of BF16 [B][(G+1)/2][(G+1)/2][cu] (FP32 average rounded
+                         // once), the others BF16 [B][G][G][C - cu]
+    IN_PAIR,             // BF16 pairs [B][G][G][2]: channels 0, 1 of 8 (the others zero)
+    IN_SCALAR            // FP32 [B][G][G]: channel 0 of 8, rounded to BF16
+  };
 
-  template<int BN>
+  struct Input
+  {
+    const void* x;       // IN_CAT: the coarse tensor
+    const bf* skip;      // IN_CAT
+    int cu;              // IN_CAT: upsampled channels
+    int ct;              // channels of the tensor (IN_PLAIN, IN_SUB) or of the concatenation
+    int c0;              // first channel of this kernel's range
+  };
+
+  __device__ __forceinline__ uint32_t avg4(uint32_t a, uint32_t b, uint32_t c, uint32_t d)
+  {
+    const float lo = ((bf2f(bf(a)) + bf2f(bf(b))) + (bf2f(bf(c)) + bf2f(bf(d)))) * 0.25f;
+    const float hi = ((bf2f(bf(a >> 16)) + bf2f(bf(b >> 16))) + (bf2f(bf(c >> 16)) + bf2f(bf(d >> 16)))) * 0.25f;
+    return uint32_t(f2bf(lo)) | (uint32_t(f2bf(hi)) << 16);
+  }
+
+  // The halo tile of channels [c0, c0 + C) around the tile at (y0, x0) of image b into shared
+  // memory, zeros outside the grid.  Asynchronous copies where the data is already BF16.
+  template<int C, int DIL, int IN, int NT>
+  __device__ __forceinline__ void load_halo(const Input& in, const Tiling& t, int b, int y0, int x0, bf* sh)
+  {
+    constexpr int HD = halo_dim(DIL), CH = C / 8, PXC = px_chunks(C);
+    const int hd = t.T + 2 * DIL;
+    const int G = t.G;
+    for(int e = threadIdx.x; e < HD * HD * CH; e += NT)
+    {
+      const int ch = e % CH, p = e / CH;
+      const int hy = p / HD, hx = p - hy * HD;
+      if(hy >= hd || hx >= hd)
+        continue;
+      const int y = y0 + hy - DIL, x = x0 + hx - DIL;
+      const bool ok = y >= 0 && y < G && x >= 0 && x < G;
+      bf* dst = sh + (p * PXC + ch) * 8;
+      if constexpr(IN == IN_PLAIN)
+      {
+        const bf* src = static_cast<const bf*>(in.x);
+        cp16(dst, ok ? src + ((size_t(b) * G + y) * G + x) * in.ct + in.c0 + ch * 8 : src, ok ? 16 : 0);
+      }
+      else if constexpr(IN == IN_SUB)
+      {
+        const bf* src = static_cast<const bf*>(in.x);
+        const int Gf = 2 * G - 1;
+        cp16(dst, ok ? src + ((size_t(b) * Gf + 2 * y) * Gf + 2 * x) * in.ct + in.c0 + ch * 8 : src, ok ? 16 : 0);
+      }
+      else if constexpr(IN == IN_CAT)
+      {
+        const int c = in.c0 + ch * 8;
+        if(c >= in.cu)
+          cp16(dst, ok ? in.skip + ((size_t(b) * G + y) * G + x) * (in.ct - in.cu) + (c - in.cu) : in.skip, ok ? 16 : 0);
+        else
+        {
+          uint4 v = make_uint4(0u, 0u, 0u, 0u);
+          if(ok)
+          {
+            const int Gc = (G + 1) / 2;
+            const int ya = y >> 1, xa = x >> 1, yb = ya + (y & 1), xb = xa + (x & 1);
+            const bf* cb = static_cast<const bf*>(in.x) + size_t(b) * Gc * Gc * in.cu + c;
+            const uint4 v00 = __ldg(reinterpret_cast<const uint4*>(cb + (size_t(ya) * Gc + xa) * in.cu));
+            const uint4 v01 = __ldg(reinterpret_cast<const uint4*>(cb + (size_t(ya) * Gc + xb) * in.cu));
+            const uint4 v10 = __ldg(reinterpret_cast<const uint4*>(cb + (size_t(yb) * Gc + xa) * in.cu));
+            const uint4 v11 = __ldg(reinterpret_cast<const uint4*>(cb + (size_t(yb) * Gc + xb) * in.cu));
+            v.x = avg4(v00.x, v01.x, v10.x, v11.x);
+            v.y = avg4(v00.y, v01.y, v10.y, v11.y);
+            v.z = avg4(v00.z, v01.z, v10.z, v11.z);
+            v.w = avg4(v00.w, v01.w, v10.w, v11.w);
+          }
+          *reinterpret_cast<uint4*>(dst) = v;
+        }
+      }
+      else
+      {
+        uint32_t w = 0u;
+        if(ok)
+        {
+          const size_t q = (size_t(b) * G + y) * G + x;
+          w = IN == IN_PAIR ? __ldg(static_cast<const uint32_t*>(in.x) + q)
+                            : uint32_t(f2bf(__ldg(static_cast<const float*>(in.x) + q)));
+        }
+        *reinterpret_cast<uint4*>(dst) = make_uint4(w, 0u, 0u, 0u);
+      }
+    }
+  }
+
+  // ------------------------------------------------------------------ convolution
+  // y[p, n] = bias[n] + sum_{tap, c} x[p + off(tap), c] * w[tap*C + c][n] for the BN columns from
+  // n0 = blockIdx.y * BN (zero outside the grid); w: BF16 rows of n_ld.  One block of four warps per
+  // tile, persistent over tiles; warp w takes MMA rows 32 w .. 32 w + 31 and all BN columns.  The
+  // same kernel is the data gradient (x = the output gradient, w = flipped transposed weights).
+  // Weights stay in shared memory for all of a block's tiles where the nine taps fit (NST = 9),
+  // otherwise they are streamed tap by tap through two buffers (NST = 2).  Bound by shared-memory
+  // reads: per 16-deep step a warp issues 2 + BN/16 ldmatrix.x4 for BN/4 MMAs.
+  enum OutMode
+  {
+    OUT_RELU,            // BF16 [P][n], max(v + bias, 0)
+    OUT_FIRST,           // FP32 [P]: v + bias of column 0 only
+    OUT_F32,             // FP32, columns < nsplit to y [P][nsplit], the others to y2 [P][n - nsplit]
+    OUT_MASK             // BF16 [P][n]: v where post > 0, else 0
+  };
+
+  struct ConvArgs
+  {
+    Input in;
+    Tiling t;
+    const bf* w;
+    const float* bias;   // n entries (OUT_RELU), 1 (OUT_FIRST)
+    void* y;
+    float* y2;
+    const bf* post;
+    int n, n_ld, nsplit;
+    int ntiles;
+  };
+
+  constexpr int CNT = 128;
+
+  template<int C, int BN, int NST>
+  __host__ __device__ constexpr int conv_wbytes()
+  {
+    return (C == 8 ? 80 : NST * C) * (BN + 8) * 2;
+  }
+  template<int C, int BN, int DIL, int NST>
+  __host__ __device__ constexpr int conv_smem()
+  {
+    return conv_wbytes<C, BN, NST>() + halo_bytes(C, DIL);
+  }
+
+  template<int C, int BN, int DIL, int IN, int OUT, int NST>
   __global__ void __launch_bounds__(CNT) k_conv(const ConvArgs a)
   {
-    constexpr int AST = CBK + 8;          // A row stride (elements): 80 bytes, conflict-free ldmatrix
-    constexpr int BST = BN + 8;
-    constexpr int NT8 = BN / 8;
-    __shared__ __align__(16) bf As[2][CBM * AST];
-    __shared__ __align__(16) bf Bs[2][CBK * BST];
+    constexpr int HD = halo_dim(DIL), PXC = px_chunks(C), NT8 = BN / 8, BST = BN + 8;
+    constexpr int WROWS = C == 8 ? 80 : C;         // weight rows of one stage
+    extern __shared__ __align__(16) unsigned char smem[];
+    bf* sw = reinterpret_cast<bf*>(smem);
+    bf* sx = reinterpret_cast<bf*>(smem + conv_wbytes<C, BN, NST>());
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int P = a.B * a.H * a.W;
-    const int m0 = blockIdx.x * CBM;
+    const int T = a.t.T, G = a.t.G, nt = a.t.nt, TT = T * T;
     const int n0 = blockIdx.y * BN;
-    // this thread's A row (one pixel)
-    const int pm = m0 + tid;
-    const bool prow = pm < P;
-    int pb = 0, py = 0, px = 0;
-    if(prow)
+
+    auto load_w = [&](int stage, int buf)
     {
-      px = pm % a.W;
-      const int t = pm / a.W;
-      py = t % a.H;
-      pb = t / a.H;
-    }
-    const int K9 = 9 * a.cin;
-    auto load = [&](int kt, int buf)
-    {
-      const int k0 = kt * CBK;
-      #pragma unroll
-      for(int c = 0; c < CBK / 8; ++c)
+      constexpr int CHB = BN / 8;
+      for(int q = tid; q < WROWS * CHB; q += CNT)
       {
-        const int k = k0 + c * 8;
-        const bf* src = a.x;
-        int bytes = 0;
-        if(prow && k < K9)
-        {
-          const int tap = k / a.cin, ci = k - tap * a.cin;
-          const int yy = py + (tap / 3 - 1) * a.dil, xx = px + (tap % 3 - 1) * a.dil;
-          if(yy >= 0 && yy < a.H && xx >= 0 && xx < a.W)
-          {
-            src = a.x + ((size_t(pb) * a.H + yy) * a.W + xx) * a.cin + ci;
-            bytes = 16;
-          }
-        }
-        cp16(&As[buf][tid * AST + c * 8], src, bytes);
-      }
-      constexpr int BCH = CBK * BN / 8;   // 16-byte chunks of the B tile
-      for(int q = tid; q < BCH; q += CNT)
-      {
-        const int r = q / (BN / 8), c = q % (BN / 8);
-        const int col = n0 + c * 8;
-        const bf* src = a.w;
-        int bytes = 0;
-        if(col < a.n_ld)
-        {
-          src = a.w + size_t(k0 + r) * a.n_ld + col;
-          bytes = 16;
-        }
-        cp16(&Bs[buf][r * BST + c * 8], src, bytes);
+        const int r = q / CHB, c = q % CHB;
+        cp16(sw + (buf * WROWS + r) * BST + c * 8, a.w + size_t(stage * WROWS + r) * a.n_ld + n0 + c * 8, 16);
       }
     };
-    float acc[2][NT8][4];
+    // shared-memory addresses of this lane's two A rows (pixels outside the tile read pixel 0)
+    uint32_t arow[2];
     #pragma unroll
-    for(int i = 0; i < 2; ++i)
-      #pragma unroll
-      for(int j = 0; j < NT8; ++j)
-        #pragma unroll
-        for(int e = 0; e < 4; ++e)
-          acc[i][j][e] = 0.f;
-    const int nk = a.kpad / CBK;
-    load(0, 0);
-    cp_commit();
-    for(int kt = 0; kt < nk; ++kt)
+    for(int mt = 0; mt < 2; ++mt)
     {
-      const int buf = kt & 1;
-      if(kt + 1 < nk)
-        load(kt + 1, buf ^ 1);
+      int m = warp * 32 + mt * 16 + (lane & 15);
+      if(m >= TT)
+        m = 0;
+      arow[mt] = smem_addr(sx) + uint32_t((m / T * HD + m % T) * PXC * 16);
+    }
+    const uint32_t brow = smem_addr(sw) + uint32_t((lane & 15) * BST + (lane >> 4) * 8) * 2;
+    const int half = lane >> 4;
+
+    bool first = true;
+    for(int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x)
+    {
+      const int b = tile / (nt * nt), r = tile - b * (nt * nt);
+      const int y0 = r / nt * T, x0 = (r - r / nt * nt) * T;
+      if(!first)
+        __syncthreads();                            // the previous tile's reads are done
+      load_halo<C, DIL, IN, CNT>(a.in, a.t, b, y0, x0, sx);
+      if(NST == 9 ? first : true)
+      {
+        if constexpr(C == 8)
+          load_w(0, 0);
+        else
+          for(int s = 0; s < (NST == 9 ? 9 : 1); ++s)
+            load_w(s, s);
+      }
       cp_commit();
-      cp_wait<1>();
-      __syncthreads();
+      float acc[2][NT8][4];
       #pragma unroll
-      for(int kk = 0; kk < CBK; kk += 16)
+      for(int i = 0; i < 2; ++i)
+        #pragma unroll
+        for(int j = 0; j < NT8; ++j)
+          #pragma unroll
+          for(int e = 0; e < 4; ++e)
+            acc[i][j][e] = 0.f;
+      // one 16-deep step: A chunks at aoff (bytes), B rows at boff (bytes)
+      auto step = [&](uint32_t aoff, uint32_t boff)
       {
         uint32_t af[2][4];
         #pragma unroll
         for(int mt = 0; mt < 2; ++mt)
-          ldm_x4(af[mt], &As[buf][(warp * 32 + mt * 16 + (lane & 15)) * AST + kk + (lane >> 4) * 8]);
+          ldm_x4a(af[mt], arow[mt] + aoff);
         #pragma unroll
-        for(int nt = 0; nt < NT8; nt += 2)
+        for(int j = 0; j < NT8; j += 2)
         {
-          if(nt + 1 < NT8)
+          if(j + 1 < NT8)
           {
             uint32_t bfr[4];
-            ldm_x4_t(bfr, &Bs[buf][(kk + (lane & 15)) * BST + nt * 8 + (lane >> 4) * 8]);
+            ldm_x4a_t(bfr, brow + boff + j * 16);
             #pragma unroll
             for(int mt = 0; mt < 2; ++mt)
             {
-              mma16816(acc[mt][nt], af[mt], bfr[0], bfr[1]);
-              mma16816(acc[mt][nt + 1], af[mt], bfr[2], bfr[3]);
+              mma16816(acc[mt][j], af[mt], bfr[0], bfr[1]);
+              mma16816(acc[mt][j + 1], af[mt], bfr[2], bfr[3]);
             }
           }
           else
           {
             uint32_t bfr[2];
-            ldm_x2_t(bfr, &Bs[buf][(kk + (lane & 15)) * BST + nt * 8]);
+            ldm_x2a_t(bfr, brow - half * 16 + boff + j * 16);
             #pragma unroll
             for(int mt = 0; mt < 2; ++mt)
-              mma16816(acc[mt][nt], af[mt], bfr[0], bfr[1]);
+              mma16816(acc[mt][j], af[mt], bfr[0], bfr[1]);
           }
         }
-      }
-      __syncthreads();
-    }
-    // epilogue: bias, activation, store
-    const int g = lane >> 2, tg = lane & 3;
-    #pragma unroll
-    for(int mt = 0; mt < 2; ++mt)
-      #pragma unroll
-      for(int h = 0; h < 2; ++h)
+      };
+      if constexpr(C == 8)
       {
-        const int row = m0 + warp * 32 + mt * 16 + g + h * 8;
-        if(row >= P)
-          continue;
+        cp_wait<0>();
+        __syncthreads();
+        // a 16-deep step holds two taps; the tenth chunk's weight rows are zero
         #pragma unroll
-        for(int nt = 0; nt < NT8; ++nt)
+        for(int s = 0; s < 5; ++s)
         {
-          const int col = n0 + nt * 8 + tg * 2;
-          if(col >= a.n)
-            continue;
-          float v0 = acc[mt][nt][h * 2 + 0], v1 = acc[mt][nt][h * 2 + 1];
-          if(a.bias)
+          const int q0 = 2 * s, q1 = 2 * s + 1 < 9 ? 2 * s + 1 : 0;
+          const int o0 = (q0 / 3 * HD + q0 % 3) * DIL * PXC * 16, o1 = (q1 / 3 * HD + q1 % 3) * DIL * PXC * 16;
+          step(uint32_t(half ? o1 : o0), uint32_t(s * 16 * BST * 2));
+        }
+      }
+      else if constexpr(NST == 9)
+      {
+        cp_wait<0>();
+        __syncthreads();
+        #pragma unroll
+        for(int tap = 0; tap < 9; ++tap)
+          #pragma unroll
+          for(int c = 0; c < C / 16; ++c)
+            step(uint32_t(((tap / 3 * HD + tap % 3) * DIL * PXC + 2 * c + half) * 16),
+              uint32_t((tap * C + c * 16) * BST * 2));
+      }
+      else
+      {
+        for(int tap = 0; tap < 9; ++tap)
+        {
+          if(tap + 1 < 9)
+            load_w(tap + 1, (tap + 1) & 1);
+          cp_commit();
+          cp_wait<1>();
+          __syncthreads();
+          const uint32_t ao = uint32_t(((tap / 3 * HD + tap % 3) * DIL * PXC + half) * 16);
+          const uint32_t bo = uint32_t((tap & 1) * C * BST * 2);
+          #pragma unroll
+          for(int c = 0; c < C / 16; ++c)
+            step(ao + c * 32, bo + c * 16 * BST * 2);
+          __syncthreads();
+        }
+      }
+      first = false;
+      // epilogue: fragment rows g and g + 8 of each 16-row tile, columns 8 j + 2 tg, + 1
+      const int g = lane >> 2, tg = lane & 3;
+      #pragma unroll
+      for(int mt = 0; mt < 2; ++mt)
+        #pragma unroll
+        for(int h = 0; h < 2; ++h)
+        {
+          const int m = warp * 32 + mt * 16 + g + h * 8;
+          const int ty = m / T, y = y0 + ty, x = x0 + m - ty * T;
+          const bool ok = m < TT && y < G && x < G;
+          const size_t p = (size_t(b) * G + y) * G + x;
+          if constexpr(OUT == OUT_FIRST)
           {
-            v0 += col < a.nb ? a.bias[col] : 0.f;
-            v1 += col + 1 < a.nb ? a.bias[col + 1] : 0.f;
+            if(ok && tg == 0)
+              static_cast<float*>(a.y)[p] = acc[mt][0][h * 2] + __ldg(a.bias);
           }
-          if(a.relu)
+          else if constexpr(OUT == OUT_F32)
           {
-            v0 = fmaxf(v0, 0.f);
-            v1 = fmaxf(v1, 0.f);
-          }
-          const size_t o = size_t(row) * a.y_ld + a.y_off + col;
-          if(a.out_bf16)
-          {
-            bf* y = static_cast<bf*>(a.y);
-            const uint32_t pk = uint32_t(f2bf(v0)) | (uint32_t(f2bf(v1)) << 16);
-            *reinterpret_cast<uint32_t*>(y + o) = pk;
+            if(ok)
+              #pragma unroll
+              for(int j = 0; j < NT8; ++j)
+              {
+                const int col = n0 + j * 8 + tg * 2;
+                float* q = col < a.nsplit ? static_cast<float*>(a.y) + p * a.nsplit + col
+                                          : a.y2 + p * (a.n - a.nsplit) + (col - a.nsplit);
+                *reinterpret_cast<float2*>(q) = make_float2(acc[mt][j][h * 2], acc[mt][j][h * 2 + 1]);
+              }
           }
           else
           {
-            float* y = static_cast<float*>(a.y);
-            *reinterpret_cast<float2*>(y + o) = make_float2(v0, v1);
+            // two 8-column groups at a time: the four lanes of a row exchange so that each stores
+            // 8 consecutive bytes of the row's 32 (whole sectors)
+            #pragma unroll
+            for(int j = 0; j < NT8; j += 2)
+            {
+              uint32_t pk[2];
+              #pragma unroll
+              for(int u = 0; u < 2; ++u)
+              {
+                float v0 = acc[mt][j + u][h * 2], v1 = acc[mt][j + u][h * 2 + 1];
+                if constexpr(OUT == OUT_RELU)
+                {
+                  const int col = n0 + (j + u) * 8 + tg * 2;
+                  v0 = fmaxf(v0 + __ldg(a.bias + col), 0.f);
+                  v1 = fmaxf(v1 + __ldg(a.bias + col + 1), 0.f);
+                }
+                pk[u] = uint32_t(f2bf(v0)) | (uint32_t(f2bf(v1)) << 16);
+              }
+              const int s0 = (lane & ~3) | ((tg & 1) * 2);
+              const uint32_t a0 = __shfl_sync(0xffffffffu, pk[0], s0), a1 = __shfl_sync(0xffffffffu, pk[0], s0 + 1);
+              const uint32_t b0 = __shfl_sync(0xffffffffu, pk[1], s0), b1 = __shfl_sync(0xffffffffu, pk[1], s0 + 1);
+              uint2 v = tg < 2 ? make_uint2(a0, a1) : make_uint2(b0, b1);
+              if(ok)
+              {
+                const size_t o = p * a.n + n0 + j * 8 + tg * 4;
+                if constexpr(OUT == OUT_MASK)
+                {
+                  const uint2 q = __ldg(reinterpret_cast<const uint2*>(a.post + o));
+                  v.x &= mask2(q.x);
+                  v.y &= mask2(q.y);
+                }
+                *reinterpret_cast<uint2*>(static_cast<bf*>(a.y) + o) = v;
+              }
+            }
           }
         }
-      }
+    }
   }
 
   // ------------------------------------------------------------------ weight gradient
-  // part[s][m][j] = sum over the pixels of split s of dy[p, m] * x[p + off(tap_j), c_j] with
-  // j = tap*cin + c: M = cout (dy channels, padded to BM), N = 9*cin, K = pixels.
+  // part[block][co][tap*ct + c0 + c] = sum over the block's tiles of dy[p, co] * x[p + off(tap), c],
+  // part_b[block][co] = sum of dy[p, co]: M = output channels, N = 9 C columns, K = the 128 pixel
+  // slots of each tile (slots outside the tile or the grid hold zeros in dy).  Both operands are
+  // read transposed by ldmatrix.trans from the staged tiles; warp w takes GPW groups of 16 columns
+  // and all M rows, so a warp issues MT + GPW ldmatrix.x4 for 2 MT GPW MMAs.  Blocks are
+  // persistent over tiles and write one partial each (FP32), which k_grad_reduce sums in block order.
   struct WgradArgs
   {
-    const bf* dy;        // [P][m_ld]
-    const bf* x;         // [P][cin]
-    float* part;         // [splits][m][n] (m < m_real, n < 9*cin)
-    int m_ld, m_real, cin;
-    int B, H, W, dil;
-    int pix_per_split;
+    Input in;
+    Tiling t;
+    const void* dy;      // BF16 [P][M] or FP32 [P] (SCALAR: M = 16 rows of which row 0 is real)
+    float* part;         // [blocks][m_real * 9 ct]
+    float* part_b;       // [blocks][m_real]
+    int m_real;
+    int ntiles;
   };
 
-  constexpr int WBN = 64, WBK = 32, WNT = 128;
-
-  template<int BM>
-  __global__ void __launch_bounds__(WNT) k_wgrad(const WgradArgs a)
+  template<int C, int M, int DIL>
+  __host__ __device__ constexpr int wgrad_smem()
   {
-    constexpr int AST = BM + 8;     // A stored K-major: [k][m]
-    constexpr int BST = WBN + 8;    // B stored [k][n]
-    constexpr int MT = BM / 16;
-    __shared__ __align__(16) bf As[2][WBK * AST];
-    __shared__ __align__(16) bf Bs[2][WBK * BST];
+    return halo_bytes(C, DIL) + 128 * px_chunks(M) * 16;
+  }
+
+  template<int C, int M, int DIL, int IN, bool SCALAR, int NW>
+  __global__ void __launch_bounds__(NW * 32) k_wgrad(const WgradArgs a)
+  {
+    constexpr int NT = NW * 32, HD = halo_dim(DIL), PXC = px_chunks(C), PXD = px_chunks(M);
+    constexpr int MT = M / 16, CH = C / 8;
+    constexpr int NCH = 9 * CH;                     // 8-column chunks
+    constexpr int GPW = ((NCH + 1) / 2 + NW - 1) / NW;
+    extern __shared__ __align__(16) unsigned char smem[];
+    bf* sx = reinterpret_cast<bf*>(smem);
+    bf* sd = reinterpret_cast<bf*>(smem + halo_bytes(C, DIL));
+    __shared__ int pxo[128];                        // halo offset (bytes) of each pixel slot
+    Input in = a.in;
+    in.c0 += int(blockIdx.y) * C;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int P = a.B * a.H * a.W;
-    const int N9 = 9 * a.cin;
-    const int n0 = blockIdx.x * WBN;
-    const int p_begin = blockIdx.y * a.pix_per_split;
-    const int p_end = min(P, p_begin + a.pix_per_split);
-    auto load = [&](int p0, int buf)
+    const int T = a.t.T, G = a.t.G, nt = a.t.nt, TT = T * T;
+    for(int m = tid; m < 128; m += NT)
+      pxo[m] = m < TT ? (m / T * HD + m % T) * PXC * 16 : 0;
+    // byte offset of this lane's chunk of each column group (chunks past the end read chunk 0)
+    uint32_t goff[GPW];
+    #pragma unroll
+    for(int k = 0; k < GPW; ++k)
     {
-      // A: WBK pixels x BM channels of dy
-      for(int q = tid; q < WBK * (BM / 8); q += WNT)
-      {
-        const int r = q / (BM / 8), c = q % (BM / 8);
-        const int p = p0 + r;
-        const bf* src = a.dy;
-        int bytes = 0;
-        if(p < p_end && c * 8 < a.m_ld)
-        {
-          src = a.dy + size_t(p) * a.m_ld + c * 8;
-          bytes = 16;
-        }
-        cp16(&As[buf][r * AST + c * 8], src, bytes);
-      }
-      // B: WBK pixels x WBN columns of im2col(x)
-      for(int q = tid; q < WBK * (WBN / 8); q += WNT)
-      {
-        const int r = q / (WBN / 8), c = q % (WBN / 8);
-        const int p = p0 + r;
-        const int j = n0 + c * 8;
-        const bf* src = a.x;
-        int bytes = 0;
-        if(p < p_end && j < N9)
-        {
-          const int tap = j / a.cin, ci = j - tap * a.cin;
-          const int px = p % a.W, t = p / a.W;
-          const int py = t % a.H, pb = t / a.H;
-          const int yy = py + (tap / 3 - 1) * a.dil, xx = px + (tap % 3 - 1) * a.dil;
-          if(yy >= 0 && yy < a.H && xx >= 0 && xx < a.W)
-          {
-            src = a.x + ((size_t(pb) * a.H + yy) * a.W + xx) * a.cin + ci;
-            bytes = 16;
-          }
-        }
-        cp16(&Bs[buf][r * BST + c * 8], src, bytes);
-      }
-    };
-    float acc[MT][2][4];
+      int q = 2 * (warp * GPW + k) + (lane >> 4);
+      if(q >= NCH)
+        q = 0;
+      const int tap = q / CH, c = q - tap * CH;
+      goff[k] = smem_addr(sx) + uint32_t(((tap / 3 * HD + tap % 3) * DIL * PXC + c) * 16);
+    }
+    const int lj = lane >> 3, li = lane & 7;
+    const uint32_t drow = smem_addr(sd) + uint32_t(((lj >> 1) * 8 + li) * PXD * 16 + (lj & 1) * 16);
+    float acc[MT][GPW][2][4], accb[MT][4];
     #pragma unroll
     for(int i = 0; i < MT; ++i)
+    {
       #pragma unroll
-      for(int j = 0; j < 2; ++j)
+      for(int j = 0; j < GPW; ++j)
         #pragma unroll
         for(int e = 0; e < 4; ++e)
-          acc[i][j][e] = 0.f;
-    const int nk = (p_end - p_begin + WBK - 1) / WBK;
-    if(nk > 0)
-    {
-      load(p_begin, 0);
-      cp_commit();
-    }
-    for(int kt = 0; kt < nk; ++kt)
-    {
-      const int buf = kt & 1;
-      if(kt + 1 < nk)
-        load(p_begin + (kt + 1) * WBK, buf ^ 1);
-      cp_commit();
-      cp_wait<1>();
-      __syncthreads();
+          acc[i][j][0][e] = acc[i][j][1][e] = 0.f;
       #pragma unroll
-      for(int kk = 0; kk < WBK; kk += 16)
+      for(int e = 0; e < 4; ++e)
+        accb[i][e] = 0.f;
+    }
+    for(int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x)
+    {
+      const int b = tile / (nt * nt), r = tile - b * (nt * nt);
+      const int y0 = r / nt * T, x0 = (r - r / nt * nt) * T;
+      __syncthreads();                              // pxo written; the previous tile's reads are done
+      load_halo<C, DIL, IN, NT>(in, a.t, b, y0, x0, sx);
+      for(int e = tid; e < 128 * (M / 8); e += NT)
       {
-        // B fragments of this warp's 16 columns (two n8 tiles)
-        uint32_t bfr[4];
-        ldm_x4_t(bfr, &Bs[buf][(kk + (lane & 15)) * BST + warp * 16 + (lane >> 4) * 8]);
+        const int ch = e % (M / 8), m = e / (M / 8);
+        const int ty = m / T, y = y0 + ty, x = x0 + m - ty * T;
+        const bool ok = m < TT && y < G && x < G;
+        const size_t p = (size_t(b) * G + y) * G + x;
+        bf* dst = sd + (m * PXD + ch) * 8;
+        if constexpr(SCALAR)
+        {
+          const uint32_t w = ok && ch == 0 ? uint32_t(f2bf(__ldg(static_cast<const float*>(a.dy) + p))) : 0u;
+          *reinterpret_cast<uint4*>(dst) = make_uint4(w, 0u, 0u, 0u);
+        }
+        else
+        {
+          const bf* src = static_cast<const bf*>(a.dy);
+          cp16(dst, ok ? src + p * M + ch * 8 : src, ok ? 16 : 0);
+        }
+      }
+      cp_commit();
+      cp_wait<0>();
+      __syncthreads();
+      #pragma unroll 2
+      for(int k = 0; k < 8; ++k)
+      {
+        const uint32_t px = uint32_t(pxo[k * 16 + (lane & 15)]);
+        uint32_t bfr[GPW][4];
+        #pragma unroll
+        for(int j = 0; j < GPW; ++j)
+          ldm_x4a_t(bfr[j], goff[j] + px);
         #pragma unroll
         for(int mt = 0; mt < MT; ++mt)
         {
-          // A (m x k) from the K-major tile: matrix j covers m-rows (j&1)*8, k-cols (j>>1)*8
           uint32_t af[4];
-          const int j = lane >> 3, i = lane & 7;
-          ldm_x4_t(af, &As[buf][(kk + (j >> 1) * 8 + i) * AST + mt * 16 + (j & 1) * 8]);
-          mma16816(acc[mt][0], af, bfr[0], bfr[1]);
-          mma16816(acc[mt][1], af, bfr[2], bfr[3]);
+          ldm_x4a_t(af, drow + uint32_t(k * 16 * PXD * 16 + mt * 32));
+          #pragma unroll
+          for(int j = 0; j < GPW; ++j)
+          {
+            mma16816(acc[mt][j][0], af, bfr[j][0], bfr[j][1]);
+            mma16816(acc[mt][j][1], af, bfr[j][2], bfr[j][3]);
+          }
+          if(warp == NW - 1)
+            mma16816(accb[mt], af, 0x3F803F80u, 0x3F803F80u);   // times ones: the bias gradient
         }
       }
-      __syncthreads();
     }
     const int g = lane >> 2, tg = lane & 3;
-    float* out = a.part + size_t(blockIdx.y) * a.m_real * N9;
+    const int n9 = 9 * in.ct;
+    float* out = a.part + size_t(blockIdx.x) * a.m_real * n9;
     #pragma unroll
     for(int mt = 0; mt < MT; ++mt)
       #pragma unroll
@@ -379,255 +581,219 @@ namespace un
         if(m >= a.m_real)
           continue;
         #pragma unroll
-        for(int nt = 0; nt < 2; ++nt)
-        {
-          const int n = n0 + warp * 16 + nt * 8 + tg * 2;
-          if(n < N9)
-            out[size_t(m) * N9 + n] = acc[mt][nt][h * 2 + 0];
-          if(n + 1 < N9)
-            out[size_t(m) * N9 + n + 1] = acc[mt][nt][h * 2 + 1];
-        }
+        for(int j = 0; j < GPW; ++j)
+          #pragma unroll
+          for(int u = 0; u < 2; ++u)
+          {
+            const int q = 2 * (warp * GPW + j) + u;
+            if(q < NCH)
+              *reinterpret_cast<float2*>(out + size_t(m) * n9 + q / CH * in.ct + in.c0 + q % CH * 8 + tg * 2) =
+                make_float2(acc[mt][j][u][h * 2], acc[mt][j][u][h * 2 + 1]);
+          }
+        if(warp == NW - 1 && tg == 0 && blockIdx.y == 0)
+          a.part_b[size_t(blockIdx.x) * a.m_real + m] = accb[mt][h * 2];
       }
   }
 
-  // grad W[co][tap][ci] (real channels) = sum over splits of part[s][co][tap*cin_pad + ci], in split
-  // order; grad b[co] = sum_p dy[p, co] (per-block partial sums, then a fixed-order sum)
-  __global__ void k_wgrad_reduce(const float* __restrict__ part, int splits, int m_real, int cin_pad, int cin_real,
-    float* __restrict__ gw, int accumulate)
+  // ------------------------------------------------------------------ parameters
+  // Where each layer's parameters, BF16 GEMM copies and gradient partials lie.
+  struct LayerMap
   {
-    const int N9 = 9 * cin_pad;
-    const int total = m_real * 9 * cin_real;
-    for(int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x)
-    {
-      const int ci = e % cin_real, t = e / cin_real;
-      const int tap = t % 9, co = t / 9;
-      const size_t j = size_t(co) * N9 + tap * cin_pad + ci;
-      float s = 0.f;
-      for(int k = 0; k < splits; ++k)
-        s += part[size_t(k) * m_real * N9 + j];
-      gw[e] = accumulate ? gw[e] + s : s;
-    }
+    int woff, boff, cin, cout, cin_pad, cout_pad;
+    bf *wf, *wd;
+    const float *part, *part_b;
+    int blocks;
+  };
+  struct NetMap
+  {
+    LayerMap l[NLAYER];
+    int n;
+  };
+
+  __device__ __forceinline__ int layer_of(const NetMap& net, int e)
+  {
+    int l = 0;
+    #pragma unroll
+    for(int k = 1; k < NLAYER; ++k)
+      l += e >= net.l[k].woff ? 1 : 0;
+    return l;
   }
 
-  constexpr int BG_NT = 256;
-  __global__ void __launch_bounds__(BG_NT) k_bgrad_part(const bf* __restrict__ dy, int P, int ld, int m_real,
-    int pix_per_block, float* __restrict__ part)
+  // Every parameter's gradient: its partials summed in four groups (group g takes partials g, g + 4,
+  // ...), then the groups in order.  64 parameters per block: a group's loads are whole 128-byte
+  // lines, and four groups keep four times as many of them in flight as one thread per parameter.
+  constexpr int GR_E = 64, GR_G = 4;
+  __global__ void __launch_bounds__(GR_E * GR_G) k_grad_reduce(const __grid_constant__ NetMap net,
+    float* __restrict__ grad, int accumulate)
   {
-    // block b sums pixels [b*ppb, (b+1)*ppb) for every channel; threads: channel-major groups
-    __shared__ float sh[BG_NT];
-    const int p0 = blockIdx.x * pix_per_block, p1 = min(P, p0 + pix_per_block);
-    const int groups = BG_NT / 64;   // 64 channels max per pass
-    const int c = threadIdx.x % 64, gsub = threadIdx.x / 64;
+    __shared__ float sh[GR_G][GR_E];
+    const int x = threadIdx.x % GR_E, grp = threadIdx.x / GR_E;
+    const int e = blockIdx.x * GR_E + x;
     float s = 0.f;
-    if(c < m_real)
-      for(int p = p0 + gsub; p < p1; p += groups)
-        s += bf2f(dy[size_t(p) * ld + c]);
-    sh[threadIdx.x] = s;
+    if(e < net.n)
+    {
+      const LayerMap& L = net.l[layer_of(net, e)];
+      const float* p;
+      int stride;
+      if(e >= L.boff)
+      {
+        p = L.part_b + (e - L.boff);
+        stride = L.cout;
+      }
+      else
+      {
+        const int w = e - L.woff, ci = w % L.cin, t = w / L.cin;
+        p = L.part + t * L.cin_pad + ci;            // t = co * 9 + tap
+        stride = L.cout * 9 * L.cin_pad;
+      }
+      const int blocks = L.blocks;
+      #pragma unroll 8
+      for(int k = grp; k < blocks; k += GR_G)
+        s += __ldg(p + size_t(k) * stride);
+    }
+    sh[grp][x] = s;
     __syncthreads();
-    if(threadIdx.x < 64 && c < m_real)
+    if(grp == 0 && e < net.n)
     {
-      float t = 0.f;
-      for(int k = 0; k < groups; ++k)
-        t += sh[k * 64 + c];
-      part[size_t(blockIdx.x) * m_real + c] = t;
+      const float t = ((s + sh[1][x]) + sh[2][x]) + sh[3][x];
+      grad[e] = accumulate ? grad[e] + t : t;
     }
   }
 
-  __global__ void k_bgrad_reduce(const float* __restrict__ part, int nblk, int m_real, float* __restrict__ gb,
-    int accumulate)
+  // FP32 master -> BF16 GEMM layouts: forward wf[tap*cin_pad + ci][co] (rows of cout_pad) and data
+  // gradient wd[t*cout_pad + co][ci] = W[co][8-t][ci] (rows of cin_pad); padding entries stay zero
+  __device__ __forceinline__ void store_weight(const LayerMap& L, int w, float v)
   {
-    const int c = threadIdx.x;
-    if(c >= m_real)
+    const int ci = w % L.cin, t = w / L.cin, tap = t % 9, co = t / 9;
+    const bf h = f2bf(v);
+    L.wf[(tap * L.cin_pad + ci) * L.cout_pad + co] = h;
+    if(L.wd)
+      L.wd[((8 - tap) * L.cout_pad + co) * L.cin_pad + ci] = h;
+  }
+  __global__ void __launch_bounds__(256) k_prep_weights(const __grid_constant__ NetMap net, const float* __restrict__ p)
+  {
+    const int e = blockIdx.x * 256 + threadIdx.x;
+    if(e >= net.n)
       return;
-    float s = 0.f;
-    for(int k = 0; k < nblk; ++k)
-      s += part[size_t(k) * m_real + c];
-    gb[c] = accumulate ? gb[c] + s : s;
+    const LayerMap& L = net.l[layer_of(net, e)];
+    if(e < L.boff)
+      store_weight(L, e - L.woff, p[e]);
   }
 
-  // ------------------------------------------------------------------ grid transfers and packing
-  // NCHW FP32 input (2 channels) -> NHWC BF16 with 8 channels (6 zero)
-  __global__ void k_pack_input(const float* __restrict__ in, int B, int G, bf* __restrict__ x)
+  // Adam (Kingma & Ba 2015, Algorithm 1) on the FP32 masters, and the BF16 copies of the new weights
+  __global__ void __launch_bounds__(256) k_adam(const __grid_constant__ NetMap net, float* __restrict__ p,
+    const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v, float lr, float b1, float b2, float eps,
+    float c1, float c2)
   {
-    const size_t n = size_t(B) * G * G;
-    for(size_t p = blockIdx.x * size_t(blockDim.x) + threadIdx.x; p < n; p += size_t(gridDim.x) * blockDim.x)
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if(i >= net.n)
+      return;
+    const float gi = g[i];
+    const float mi = b1 * m[i] + (1.f - b1) * gi;
+    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
+    m[i] = mi;
+    v[i] = vi;
+    const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    p[i] = pi;
+    const LayerMap& L = net.l[layer_of(net, i)];
+    if(i < L.boff)
+      store_weight(L, i - L.woff, pi);
+  }
+
+  // ------------------------------------------------------------------ packing and masked gradients
+  // NCHW FP32 input (2 channels) -> BF16 pairs per pixel (kept for the first layer's weight gradient)
+  __global__ void k_pack_input(const float* __restrict__ in, int B, int G, uint32_t* __restrict__ x)
+  {
+    const size_t n = size_t(G) * G;
+    for(size_t p = blockIdx.x * size_t(blockDim.x) + threadIdx.x; p < n * B; p += size_t(gridDim.x) * blockDim.x)
     {
-      const size_t b = p / (size_t(G) * G), r = p % (size_t(G) * G);
-      uint32_t w[4] = {0u, 0u, 0u, 0u};
-      w[0] = uint32_t(f2bf(in[(b * 2 + 0) * G * G + r])) | (uint32_t(f2bf(in[(b * 2 + 1) * G * G + r])) << 16);
-      *reinterpret_cast<uint4*>(x + p * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+      const size_t b = p / n, r = p - b * n;
+      x[p] = uint32_t(f2bf(in[b * 2 * n + r])) | (uint32_t(f2bf(in[(b * 2 + 1) * n + r])) << 16);
     }
   }
 
-  // injection: coarse (i, j) = fine (2i, 2j); C channels, 8 at a time
-  __global__ void k_subsample(const bf* __restrict__ f, int B, int Gf, int C, bf* __restrict__ c)
+  __device__ __forceinline__ void store8(bf* dst, const float (&s)[8], const uint4& post)
+  {
+    const uint32_t q[4] = {post.x, post.y, post.z, post.w};
+    uint32_t o[4];
+    #pragma unroll
+    for(int k = 0; k < 4; ++k)
+      o[k] = (uint32_t(f2bf(s[2 * k])) | (uint32_t(f2bf(s[2 * k + 1])) << 16)) & mask2(q[k]);
+    *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+  __device__ __forceinline__ void load8(const float* p, float (&v)[8])
+  {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p + 4));
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  }
+
+  // adjoint of U for a fine FP32 gradient [B][Gf][Gf][C]: gc(i, j) = sum_{dy,dx in -1..1} w(dy) w(dx)
+  // gf(2i+dy, 2j+dx) (in-grid points), w(0) = 1, w(+-1) = 1/2; the four corner products of a cell
+  // centre carry 1/4 each.  Then dpre = mask(post) * gc as BF16.  Eight channels per thread.
+  __global__ void __launch_bounds__(256) k_upsample_bwd_mask(const float* __restrict__ gf, int C, int B, int Gf,
+    const bf* __restrict__ post, bf* __restrict__ dpre)
   {
     const int Gc = (Gf + 1) / 2, C8 = C / 8;
     const size_t n = size_t(B) * Gc * Gc * C8;
-    for(size_t e = blockIdx.x * size_t(blockDim.x) + threadIdx.x; e < n; e += size_t(gridDim.x) * blockDim.x)
+    for(size_t e = blockIdx.x * size_t(256) + threadIdx.x; e < n; e += size_t(gridDim.x) * 256)
     {
       const int ch = int(e % C8);
       const size_t p = e / C8;
       const int x = int(p % Gc), y = int((p / Gc) % Gc);
       const size_t b = p / (size_t(Gc) * Gc);
-      const size_t src = ((b * Gf + 2 * y) * Gf + 2 * x) * C + ch * 8;
-      *reinterpret_cast<uint4*>(c + p * C + ch * 8) = *reinterpret_cast<const uint4*>(f + src);
-    }
-  }
-
-  // out[:, :, :, 0:Cu] = U(coarse) (bilinear vertex upsampling, FP32 average rounded once),
-  // out[:, :, :, Cu:Cu+Cs] = skip
-  __global__ void k_upsample_cat(const bf* __restrict__ coarse, int Cu, const bf* __restrict__ skip, int Cs, int B,
-    int Gf, bf* __restrict__ out)
-  {
-    const int Gc = (Gf + 1) / 2, Ct = Cu + Cs;
-    const size_t n = size_t(B) * Gf * Gf * Ct;
-    for(size_t e = blockIdx.x * size_t(blockDim.x) + threadIdx.x; e < n; e += size_t(gridDim.x) * blockDim.x)
-    {
-      const int ch = int(e % Ct);
-      const size_t p = e / Ct;
-      const int x = int(p % Gf), y = int((p / Gf) % Gf);
-      const size_t b = p / (size_t(Gf) * Gf);
-      bf v;
-      if(ch >= Cu)
-        v = skip[p * Cs + (ch - Cu)];
-      else
-      {
-        const int y0 = y >> 1, x0 = x >> 1, y1 = y0 + (y & 1), x1 = x0 + (x & 1);
-        const bf* cb = coarse + b * size_t(Gc) * Gc * Cu + ch;
-        const float a00 = bf2f(cb[(size_t(y0) * Gc + x0) * Cu]);
-        const float a01 = bf2f(cb[(size_t(y0) * Gc + x1) * Cu]);
-        const float a10 = bf2f(cb[(size_t(y1) * Gc + x0) * Cu]);
-        const float a11 = bf2f(cb[(size_t(y1) * Gc + x1) * Cu]);
-        v = f2bf(((a00 + a01) + (a10 + a11)) * 0.25f);
-      }
-      out[e] = v;
-    }
-  }
-
-  // adjoint of U for channel range [c0, c0+C) of a fine gradient (FP32, row stride ld):
-  // gc(i, j) = sum_{dy,dx in -1..1} w(dy) w(dx) gf(2i+dy, 2j+dx) (in-grid points), w(0) = 1,
-  // w(+-1) = 1/2; the four corner products of a cell centre carry 1/4 each.  Then dpre = mask(post)
-  // * gc as BF16 ([B][Gc][Gc][C]).
-  __global__ void k_upsample_bwd_mask(const float* __restrict__ gf, int ld, int c0, int C, int B, int Gf,
-    const bf* __restrict__ post, bf* __restrict__ dpre)
-  {
-    const int Gc = (Gf + 1) / 2;
-    const size_t n = size_t(B) * Gc * Gc * C;
-    for(size_t e = blockIdx.x * size_t(blockDim.x) + threadIdx.x; e < n; e += size_t(gridDim.x) * blockDim.x)
-    {
-      const int ch = int(e % C);
-      const size_t p = e / C;
-      const int x = int(p % Gc), y = int((p / Gc) % Gc);
-      const size_t b = p / (size_t(Gc) * Gc);
-      float s = 0.f;
+      float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      #pragma unroll
       for(int dy = -1; dy <= 1; ++dy)
-      {
-        const int yf = 2 * y + dy;
-        if(yf < 0 || yf >= Gf)
-          continue;
+        #pragma unroll
         for(int dx = -1; dx <= 1; ++dx)
         {
-          const int xf = 2 * x + dx;
-          if(xf < 0 || xf >= Gf)
+          const int yf = 2 * y + dy, xf = 2 * x + dx;
+          if(yf < 0 || yf >= Gf || xf < 0 || xf >= Gf)
             continue;
           const float w = (dy == 0 ? 1.f : 0.5f) * (dx == 0 ? 1.f : 0.5f);
-          s += w * gf[((b * Gf + yf) * Gf + xf) * ld + c0 + ch];
+          float v[8];
+          load8(gf + ((b * Gf + yf) * Gf + xf) * C + ch * 8, v);
+          #pragma unroll
+          for(int k = 0; k < 8; ++k)
+            s[k] += w * v[k];
         }
-      }
-      dpre[e] = f2bf(bf2f(post[e]) > 0.f ? s : 0.f);
+      store8(dpre + e * 8, s, __ldg(reinterpret_cast<const uint4*>(post + e * 8)));
     }
   }
 
-  // dpre = mask(post) * (g1[p, c1+c] (optional) + (even-even p ? g2[p/2 coarse, c] : 0) (optional))
-  __global__ void k_grad_mask(const bf* __restrict__ post, int C, int B, int G, const float* __restrict__ g1, int ld1,
-    int c1, const float* __restrict__ g2, int ld2, bf* __restrict__ dpre)
+  // dpre = mask(post) * (g1 + (even-even pixel ? g2 of the coarse vertex : 0)): the gradient through
+  // the skip connection and through the injection.  Eight channels per thread.
+  __global__ void __launch_bounds__(256) k_grad_mask(const bf* __restrict__ post, int C, int B, int G,
+    const float* __restrict__ g1, const float* __restrict__ g2, bf* __restrict__ dpre)
   {
-    const int Gc = (G + 1) / 2;
-    const size_t n = size_t(B) * G * G * C;
-    for(size_t e = blockIdx.x * size_t(blockDim.x) + threadIdx.x; e < n; e += size_t(gridDim.x) * blockDim.x)
+    const int Gc = (G + 1) / 2, C8 = C / 8;
+    const size_t n = size_t(B) * G * G * C8;
+    for(size_t e = blockIdx.x * size_t(256) + threadIdx.x; e < n; e += size_t(gridDim.x) * 256)
     {
-      const int ch = int(e % C);
-      const size_t p = e / C;
-      float s = 0.f;
-      if(g1)
-        s += g1[p * ld1 + c1 + ch];
-      if(g2)
+      const int ch = int(e % C8);
+      const size_t p = e / C8;
+      const int x = int(p % G), y = int((p / G) % G);
+      float s[8];
+      load8(g1 + e * 8, s);
+      if(!(x & 1) && !(y & 1))
       {
-        const int x = int(p % G), y = int((p / G) % G);
-        if(!(x & 1) && !(y & 1))
-        {
-          const size_t b = p / (size_t(G) * G);
-          s += g2[((b * Gc + y / 2) * Gc + x / 2) * ld2 + ch];
-        }
+        const size_t b = p / (size_t(G) * G);
+        float v[8];
+        load8(g2 + ((b * Gc + y / 2) * Gc + x / 2) * C + ch * 8, v);
+        #pragma unroll
+        for(int k = 0; k < 8; ++k)
+          s[k] += v[k];
       }
-      dpre[e] = f2bf(bf2f(post[e]) > 0.f ? s : 0.f);
+      store8(dpre + e * 8, s, __ldg(reinterpret_cast<const uint4*>(post + e * 8)));
     }
   }
 
-  // output gradient (FP32 [B][G][G]) -> BF16 [P][8], channel 0
-  __global__ void k_pack_dout(const float* __restrict__ g, size_t P, bf* __restrict__ dy)
-  {
-    for(size_t p = blockIdx.x * size_t(blockDim.x) + threadIdx.x; p < P; p += size_t(gridDim.x) * blockDim.x)
-      *reinterpret_cast<uint4*>(dy + p * 8) = make_uint4(uint32_t(f2bf(g[p])), 0u, 0u, 0u);
-  }
-
-  // output [P][8] FP32 channel 0 -> [B][G][G]
-  __global__ void k_unpack_out(const float* __restrict__ y, size_t P, float* __restrict__ out)
-  {
-    for(size_t p = blockIdx.x * size_t(blockDim.x) + threadIdx.x; p < P; p += size_t(gridDim.x) * blockDim.x)
-      out[p] = y[p * 8];
-  }
-
-  // FP32 master -> BF16 GEMM layouts: forward wf[tap*cin_pad + ci][co] (kpad x cout_pad) and data
-  // gradient wd[t*cout_pad + co][ci] = W[co][8-t][ci] (kpad_d x cin_pad)
-  __global__ void k_prep_weights(const float* __restrict__ W, int cin, int cout, int cin_pad, int cout_pad, int kpad,
-    int kpad_d, bf* __restrict__ wf, bf* __restrict__ wd)
-  {
-    const int nf = kpad * cout_pad, nd = kpad_d * cin_pad;
-    for(int e = blockIdx.x * blockDim.x + threadIdx.x; e < nf + nd; e += gridDim.x * blockDim.x)
-    {
-      if(e < nf)
-      {
-        const int co = e % cout_pad, k = e / cout_pad;
-        const int tap = k / cin_pad, ci = k % cin_pad;
-        float v = 0.f;
-        if(tap < 9 && ci < cin && co < cout)
-          v = W[(co * 9 + tap) * cin + ci];
-        wf[e] = f2bf(v);
-      }
-      else if(wd)
-      {
-        const int f = e - nf;
-        const int ci = f % cin_pad, k = f / cin_pad;
-        const int t = k / cout_pad, co = k % cout_pad;
-        float v = 0.f;
-        if(t < 9 && ci < cin && co < cout)
-          v = W[(co * 9 + (8 - t)) * cin + ci];
-        wd[f] = f2bf(v);
-      }
-    }
-  }
-
-  // Adam (Kingma & Ba 2015, Algorithm 1) on the FP32 masters
-  __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-    size_t n, float lr, float b1, float b2, float eps, float c1, float c2)
-  {
-    for(size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
-    {
-      const float gi = g[i];
-      const float mi = b1 * m[i] + (1.f - b1) * gi;
-      const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-      m[i] = mi;
-      v[i] = vi;
-      p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    }
-  }
-
-  // loss = sum (y - t)^2 / n over [n]; grad = 2 (y - t) / n (per-block partials, fixed-order sum)
+  // loss = sum (y - t)^2 / n over [n]; grad = 2 (y - t) / n (per-block partials, summed in block
+  // order by the last block)
   constexpr int MSE_NT = 256;
   __global__ void __launch_bounds__(MSE_NT) k_mse(const float* __restrict__ y, const float* __restrict__ t, size_t n,
-    float* __restrict__ grad, double* __restrict__ part)
+    float* __restrict__ grad, RedSlot slot, double* __restrict__ loss)
   {
     __shared__ double sh[32];
     double s = 0.0;
@@ -639,16 +805,9 @@ namespace un
         grad[i] = 2.f * d * inv;
       s += double(d) * double(d);
     }
-    const double tot = block_sum<MSE_NT>(s, sh);
-    if(threadIdx.x == 0)
-      part[blockIdx.x] = tot;
-  }
-  __global__ void k_mse_final(const double* __restrict__ part, int nb, size_t n, double* __restrict__ loss)
-  {
-    double s = 0.0;
-    for(int k = 0; k < nb; ++k)
-      s += part[k];
-    *loss = s / double(n);
+    double total;
+    if(grid_sum_last<MSE_NT>(s, slot, sh, total))
+      *loss = total / double(n);
   }
 } // namespace un
 } // namespace fb
@@ -663,37 +822,30 @@ struct fb_unet
   size_t nparam = 0;
   size_t woff[NLAYER], boff[NLAYER];
   int cin_pad[NLAYER], cout_pad[NLAYER], kpad[NLAYER], kpad_d[NLAYER];
-  std::vector<void*> allocs;
+  void* arena = nullptr;       // every device buffer of the network
   float *param = nullptr, *grad = nullptr, *adam_m = nullptr, *adam_v = nullptr;
   bf* wf[NLAYER] = {};
   bf* wd[NLAYER] = {};
-  // activations (BF16 NHWC): x8 (input), e1..e4, s1..s3, c3, c2, c1, d3, d2, d1
-  bf *x8 = nullptr, *e[4] = {}, *s[3] = {}, *c[3] = {}, *d[3] = {};
+  // activations (BF16 NHWC): xp (input pairs), e1..e4, the two further bottleneck outputs, d3, d2, d1
+  uint32_t* xp = nullptr;
+  bf *e[4] = {}, *d[3] = {};
   bf* b4[2] = {};              // bottleneck: outputs of the dilation-2 and dilation-4 convolutions
-  float* yout = nullptr;       // [P1][8] FP32 pre-activation output of L8
-  // backward scratch: BF16 output gradient and pre-activation gradient (one layer at a time);
-  // FP32 data gradients of the concatenated inputs (dc1 @G1 48 ch, dc2 @G2 96, dc3 @G3 128) and of
-  // the other inputs (gs: d1, then s3, s2, s1 in turn)
-  bf *dy8 = nullptr, *dpre = nullptr;
-  float* dc[3] = {};
-  float* gs = nullptr;
-  float* wpart = nullptr;
-  size_t wpart_n = 0;
-  float* bpart = nullptr;
-  size_t bpart_n = 0;
+  // backward scratch: BF16 pre-activation gradients (two, used in turn); FP32 data gradients of the
+  // concatenated inputs, upsampled channels du and skip channels dk, and of the subsampled ones (gs)
+  bf* dpre[2] = {};
+  float *du[3] = {}, *dk[3] = {}, *gs = nullptr;
+  float* part[NLAYER] = {};    // weight- and bias-gradient partials, one per block
+  float* part_b[NLAYER] = {};
+  int blocks_max[NLAYER] = {};
   double* mse_part = nullptr;
-  double* mse_loss = nullptr;
+  unsigned int* mse_counter = nullptr;
   bool weights_ready = false;
 };
 
 namespace
 {
-  fb_status ualloc(fb_unet* u, void** p, size_t bytes)
-  {
-    FB_CUDA(cudaMalloc(p, std::max<size_t>(bytes, 256)));
-    u->allocs.push_back(*p);
-    return FB_OK;
-  }
+  constexpr int SMS = 148;
+
 #define UN_TRY(x)                      \
   do {                                 \
     fb_status t_ = (x);                \
@@ -702,144 +854,136 @@ namespace
 
   unsigned grid_for(size_t n, int nt = 256)
   {
-    return unsigned(std::min<size_t>(std::max<size_t>((n + nt - 1) / nt, 1), 148 * 16));
+    return unsigned(std::min<size_t>(std::max<size_t>((n + nt - 1) / nt, 1), SMS * 16));
+  }
+
+  // tiles of at most TMAX x TMAX points, as even as they come
+  Tiling tiling(int G)
+  {
+    Tiling t;
+    t.G = G;
+    t.nt = (G + TMAX - 1) / TMAX;
+    t.T = (G + t.nt - 1) / t.nt;
+    return t;
+  }
+  int tiles(const Tiling& t, int B) { return B * t.nt * t.nt; }
+
+  // resolution level of each layer, and the blocks of its weight-gradient kernel: enough to fill the
+  // SMs where there are that many tiles; where a layer's partials are large (64 x 576 values and
+  // more) every block takes at least two tiles, which halves what the reduction has to read
+  int wgrad_blocks(const fb_unet* u, int l, int B)
+  {
+    const int nt = tiles(tiling(u->G[LAYERS[l].level]), B);
+    const int big = LAYERS[l].cin * LAYERS[l].cout >= 64 * 64;
+    const int cap = l == 6 ? SMS / 2 : big ? SMS : 2 * SMS;
+    return std::max(1, std::min(big ? (nt + 1) / 2 : nt, cap));
+  }
+
+  NetMap net_map(const fb_unet* u, int B)
+  {
+    NetMap m;
+    m.n = int(u->nparam);
+    for(int l = 0; l < NLAYER; ++l)
+    {
+      LayerMap& L = m.l[l];
+      L.woff = int(u->woff[l]);
+      L.boff = int(u->boff[l]);
+      L.cin = LAYERS[l].cin;
+      L.cout = LAYERS[l].cout;
+      L.cin_pad = u->cin_pad[l];
+      L.cout_pad = u->cout_pad[l];
+      L.wf = u->wf[l];
+      L.wd = u->wd[l];
+      L.part = u->part[l];
+      L.part_b = u->part_b[l];
+      L.blocks = B > 0 ? wgrad_blocks(u, l, B) : 0;
+    }
+    return m;
+  }
+
+  template<int C, int BN, int DIL, int IN, int OUT, int NST>
+  fb_status launch_conv(const ConvArgs& a, cudaStream_t st)
+  {
+    constexpr int smem = conv_smem<C, BN, DIL, NST>();
+    if(smem > 48 * 1024)
+      FB_CUDA(cudaFuncSetAttribute(k_conv<C, BN, DIL, IN, OUT, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // resident blocks per SM by shared memory, at most 8 (32 warps)
+    constexpr int occ = std::min(8, 227 * 1024 / (smem + 1024));
+    const int ny = a.n / BN;
+    dim3 grid(unsigned(std::min(a.ntiles, std::max(1, SMS * occ / ny))), unsigned(ny));
+    k_conv<C, BN, DIL, IN, OUT, NST><<<grid, CNT, smem, st>>>(a);
+    FB_LAUNCHED(1);
+    return FB_OK;
+  }
+
+  Input plain(const bf* x, int c) { return Input{x, nullptr, 0, c, 0}; }
+  Input concat(const bf* coarse, int cu, const bf* skip, int cs) { return Input{coarse, skip, cu, cu + cs, 0}; }
+
+  // layer l's convolution of `in` at its grid; y BF16 with ReLU, or FP32 [P] for the last layer.
+  // NARROW: 16 output columns per block instead of all, for grids of few tiles: the blocks of one
+  // tile share its pixels, so a batch of one (4 to 36 tiles on the coarse grids) spreads over four
+  // times as many SMs, and each streams a quarter of the weights.
+  template<int C, int BN, int DIL, int IN, int OUT, int NST, int NARROW_NST = 9>
+  fb_status conv_fwd(fb_unet* u, int l, const Input& in, int B, void* y, cudaStream_t st)
+  {
+    ConvArgs a{};
+    a.in = in;
+    a.t = tiling(u->G[LAYERS[l].level]);
+    a.w = u->wf[l];
+    a.bias = u->param + u->boff[l];
+    a.y = y;
+    a.n = a.n_ld = u->cout_pad[l];
+    a.ntiles = tiles(a.t, B);
+    if constexpr(BN > 16)
+      if(a.ntiles * (a.n / BN) < SMS)
+        return launch_conv<C, 16, DIL, IN, OUT, NARROW_NST>(a, st);
+    return launch_conv<C, BN, DIL, IN, OUT, NST>(a, st);
+  }
+
+  // data gradient of layer l: from dpre (`in`, cout_pad channels) to its input's cin_pad channels
+  template<int C, int BN, int DIL, int IN, int OUT, int NST>
+  fb_status conv_bwd(fb_unet* u, int l, const Input& in, int B, void* y, float* y2, int nsplit, const bf* post,
+    cudaStream_t st)
+  {
+    ConvArgs a{};
+    a.in = in;
+    a.t = tiling(u->G[LAYERS[l].level]);
+    a.w = u->wd[l];
+    a.y = y;
+    a.y2 = y2;
+    a.post = post;
+    a.n = a.n_ld = u->cin_pad[l];
+    a.nsplit = nsplit;
+    a.ntiles = tiles(a.t, B);
+    return launch_conv<C, BN, DIL, IN, OUT, NST>(a, st);
+  }
+
+  // weight- and bias-gradient partials of layer l (cin_pad = C * ny channels, ny halves)
+  template<int C, int M, int DIL, int IN, bool SCALAR, int NW>
+  fb_status wgrad(fb_unet* u, int l, const void* dy, const Input& in, int B, cudaStream_t st)
+  {
+    constexpr int smem = wgrad_smem<C, M, DIL>();
+    if(smem > 48 * 1024 - 1024)
+      FB_CUDA(cudaFuncSetAttribute(k_wgrad<C, M, DIL, IN, SCALAR, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    WgradArgs a{};
+    a.in = in;
+    a.t = tiling(u->G[LAYERS[l].level]);
+    a.dy = dy;
+    a.part = u->part[l];
+    a.part_b = u->part_b[l];
+    a.m_real = LAYERS[l].cout;
+    a.ntiles = tiles(a.t, B);
+    const dim3 grid(unsigned(wgrad_blocks(u, l, B)), unsigned(u->cin_pad[l] / C));
+    k_wgrad<C, M, DIL, IN, SCALAR, NW><<<grid, NW * 32, smem, st>>>(a);
+    FB_LAUNCHED(1);
+    return FB_OK;
   }
 
   fb_status prep_weights(fb_unet* u, cudaStream_t st)
   {
-    for(int l = 0; l < NLAYER; ++l)
-    {
-      const LayerDef& L = LAYERS[l];
-      const int nf = u->kpad[l] * u->cout_pad[l] + (u->wd[l] ? u->kpad_d[l] * u->cin_pad[l] : 0);
-      k_prep_weights<<<grid_for(size_t(nf)), 256, 0, st>>>(u->param + u->woff[l], L.cin, L.cout, u->cin_pad[l],
-        u->cout_pad[l], u->kpad[l], u->kpad_d[l], u->wf[l], u->wd[l]);
-    }
-    FB_LAUNCHED(NLAYER);
+    k_prep_weights<<<unsigned((u->nparam + 255) / 256), 256, 0, st>>>(net_map(u, 0), u->param);
+    FB_LAUNCHED(1);
     u->weights_ready = true;
-    return FB_OK;
-  }
-
-  // y = conv(x) of layer l at grid G (B images); bf16 output with ReLU or FP32 without
-  fb_status conv_fwd(fb_unet* u, int l, const bf* x, int B, int G, void* y, int y_ld, bool out_bf16, bool relu,
-    cudaStream_t st)
-  {
-    ConvArgs a;
-    a.x = x;
-    a.w = u->wf[l];
-    a.bias = u->param + u->boff[l];
-    a.y = y;
-    a.cin = u->cin_pad[l];
-    a.kpad = u->kpad[l];
-    a.n = u->cout_pad[l];
-    a.n_ld = u->cout_pad[l];
-    a.nb = LAYERS[l].cout;
-    a.B = B;
-    a.dil = LAYERS[l].dil;
-    a.H = G;
-    a.W = G;
-    a.y_ld = y_ld;
-    a.y_off = 0;
-    a.relu = relu ? 1 : 0;
-    a.out_bf16 = out_bf16 ? 1 : 0;
-    const int P = B * G * G;
-    const int bn = std::min(64, a.n);
-    dim3 grid((P + CBM - 1) / CBM, (a.n + bn - 1) / bn);
-    switch(bn)
-    {
-      case 8: k_conv<8><<<grid, CNT, 0, st>>>(a); break;
-      case 16: k_conv<16><<<grid, CNT, 0, st>>>(a); break;
-      case 32: k_conv<32><<<grid, CNT, 0, st>>>(a); break;
-      default: k_conv<64><<<grid, CNT, 0, st>>>(a); break;
-    }
-    FB_LAUNCHED(1);
-    return FB_OK;
-  }
-
-  // data gradient of layer l: gx[p][ci] (FP32, ci < cin_pad) from dpre [P][cout_pad]
-  fb_status conv_bwd_data(fb_unet* u, int l, const bf* dpre, int B, int G, float* gx, cudaStream_t st)
-  {
-    ConvArgs a;
-    a.x = dpre;
-    a.w = u->wd[l];
-    a.bias = nullptr;
-    a.y = gx;
-    a.cin = u->cout_pad[l];
-    a.kpad = u->kpad_d[l];
-    a.n = u->cin_pad[l];
-    a.n_ld = u->cin_pad[l];
-    a.nb = 0;
-    a.B = B;
-    a.dil = LAYERS[l].dil;
-    a.H = G;
-    a.W = G;
-    a.y_ld = u->cin_pad[l];
-    a.y_off = 0;
-    a.relu = 0;
-    a.out_bf16 = 0;
-    const int P = B * G * G;
-    const int bn = std::min(64, a.n);
-    dim3 grid((P + CBM - 1) / CBM, (a.n + bn - 1) / bn);
-    switch(bn)
-    {
-      case 8: k_conv<8><<<grid, CNT, 0, st>>>(a); break;
-      case 16: k_conv<16><<<grid, CNT, 0, st>>>(a); break;
-      case 32: k_conv<32><<<grid, CNT, 0, st>>>(a); break;
-      default: k_conv<64><<<grid, CNT, 0, st>>>(a); break;
-    }
-    FB_LAUNCHED(1);
-    return FB_OK;
-  }
-
-  // weight and bias gradients of layer l from dpre [P][cout_pad] and its input x [P][cin_pad]
-  fb_status conv_bwd_weight(fb_unet* u, int l, const bf* dpre, const bf* x, int B, int G, int acc, cudaStream_t st)
-  {
-    const LayerDef& L = LAYERS[l];
-    const int P = B * G * G;
-    const int N9 = 9 * u->cin_pad[l];
-    const int ntile = (N9 + WBN - 1) / WBN;
-    // splits: about 4 waves of 148 SMs, at least 64 pixels each
-    int splits = std::max(1, std::min((148 * 8) / ntile, (P + 63) / 64));
-    const int pps = ((P + splits - 1) / splits + WBK - 1) / WBK * WBK;
-    splits = (P + pps - 1) / pps;
-    const size_t need = size_t(splits) * L.cout * N9;
-    if(need > u->wpart_n)
-    {
-      set_error("unet: weight-gradient scratch too small");
-      return FB_ERR_STATE;
-    }
-    WgradArgs a;
-    a.dy = dpre;
-    a.x = x;
-    a.part = u->wpart;
-    a.m_ld = u->cout_pad[l];
-    a.m_real = L.cout;
-    a.cin = u->cin_pad[l];
-    a.B = B;
-    a.H = G;
-    a.W = G;
-    a.dil = L.dil;
-    a.pix_per_split = pps;
-    dim3 grid(ntile, splits);
-    const int bm = u->cout_pad[l] <= 16 ? 16 : (u->cout_pad[l] <= 32 ? 32 : 64);
-    switch(bm)
-    {
-      case 16: k_wgrad<16><<<grid, WNT, 0, st>>>(a); break;
-      case 32: k_wgrad<32><<<grid, WNT, 0, st>>>(a); break;
-      default: k_wgrad<64><<<grid, WNT, 0, st>>>(a); break;
-    }
-    const int tot = L.cout * 9 * L.cin;
-    k_wgrad_reduce<<<grid_for(size_t(tot)), 256, 0, st>>>(u->wpart, splits, L.cout, u->cin_pad[l], L.cin,
-      u->grad + u->woff[l], acc);
-    const int ppb = 2048;
-    const int nblk = (P + ppb - 1) / ppb;
-    if(size_t(nblk) * L.cout > u->bpart_n)
-    {
-      set_error("unet: bias-gradient scratch too small");
-      return FB_ERR_STATE;
-    }
-    k_bgrad_part<<<nblk, BG_NT, 0, st>>>(dpre, P, u->cout_pad[l], L.cout, ppb, u->bpart);
-    k_bgrad_reduce<<<1, 64, 0, st>>>(u->bpart, nblk, L.cout, u->grad + u->boff[l], acc);
-    FB_LAUNCHED(4);
     return FB_OK;
   }
 } // namespace
@@ -868,62 +1012,72 @@ fb_status fb_unet_create(fb_unet** out, int grid, int max_batch)
     off += size_t(L.cout);
     u->cin_pad[l] = pad8(L.cin);
     u->cout_pad[l] = pad8(L.cout);
-    u->kpad[l] = (9 * u->cin_pad[l] + CBK - 1) / CBK * CBK;
-    u->kpad_d[l] = (9 * u->cout_pad[l] + CBK - 1) / CBK * CBK;
+    // GEMM depth rounded up to whole 32-deep steps (the rows past 9 channels stay zero)
+    u->kpad[l] = (9 * u->cin_pad[l] + 31) / 32 * 32;
+    u->kpad_d[l] = (9 * u->cout_pad[l] + 31) / 32 * 32;
   }
   u->nparam = off;
   fb_unet* p = u.get();
-  auto fail = [&](fb_status e) { for(void* a : p->allocs) cudaFree(a); return e; };
-  fb_status e;
-#define UN_A(ptr, bytes) do { e = ualloc(p, (void**)&(ptr), (bytes)); if(e != FB_OK) return fail(e); } while(0)
-  UN_A(p->param, sizeof(float) * off);
-  UN_A(p->grad, sizeof(float) * off);
-  UN_A(p->adam_m, sizeof(float) * off);
-  UN_A(p->adam_v, sizeof(float) * off);
-  FB_CUDA(cudaMemset(p->param, 0, sizeof(float) * off));
-  FB_CUDA(cudaMemset(p->grad, 0, sizeof(float) * off));
-  FB_CUDA(cudaMemset(p->adam_m, 0, sizeof(float) * off));
-  FB_CUDA(cudaMemset(p->adam_v, 0, sizeof(float) * off));
+  // one allocation for all buffers (an allocation each takes the driver longer than their use in a
+  // short training step); the zeroed ones first
+  std::vector<std::pair<void**, size_t>> want;
+  size_t total = 0;
+  auto take = [&](auto*& ptr, size_t bytes)
+  {
+    want.emplace_back(reinterpret_cast<void**>(&ptr), total);
+    total += (std::max<size_t>(bytes, 256) + 255) & ~size_t(255);
+  };
+  take(p->param, sizeof(float) * off);
+  take(p->grad, sizeof(float) * off);
+  take(p->adam_m, sizeof(float) * off);
+  take(p->adam_v, sizeof(float) * off);
   for(int l = 0; l < NLAYER; ++l)
   {
-    UN_A(p->wf[l], sizeof(bf) * p->kpad[l] * p->cout_pad[l]);
+    take(p->wf[l], sizeof(bf) * p->kpad[l] * p->cout_pad[l]);
     if(l > 0)
-      UN_A(p->wd[l], sizeof(bf) * p->kpad_d[l] * p->cin_pad[l]);
+      take(p->wd[l], sizeof(bf) * p->kpad_d[l] * p->cin_pad[l]);
+  }
+  take(p->mse_counter, sizeof(unsigned int));
+  const size_t zeroed = total;
+  for(int l = 0; l < NLAYER; ++l)
+  {
+    const size_t nb = size_t(wgrad_blocks(p, l, max_batch));
+    take(p->part[l], sizeof(float) * nb * LAYERS[l].cout * 9 * p->cin_pad[l]);
+    take(p->part_b[l], sizeof(float) * nb * LAYERS[l].cout);
   }
   const size_t B = size_t(max_batch);
   auto pix = [&](int lv) { return B * size_t(p->G[lv]) * p->G[lv]; };
-  UN_A(p->x8, sizeof(bf) * pix(0) * 8);
+  take(p->xp, sizeof(uint32_t) * pix(0));
   const int ech[4] = {16, 32, 64, 64};
   for(int i = 0; i < 4; ++i)
-    UN_A(p->e[i], sizeof(bf) * pix(i) * ech[i]);
-  for(int i = 0; i < 3; ++i)
-    UN_A(p->s[i], sizeof(bf) * pix(i + 1) * ech[i]);
+    take(p->e[i], sizeof(bf) * pix(i) * ech[i]);
   for(int i = 0; i < 2; ++i)
-    UN_A(p->b4[i], sizeof(bf) * pix(3) * 64);
-  // c[0] = [U(d2), e1] @G1 (48), c[1] = [U(d3), e2] @G2 (96), c[2] = [U(e4), e3] @G3 (128)
-  UN_A(p->c[0], sizeof(bf) * pix(0) * 48);
-  UN_A(p->c[1], sizeof(bf) * pix(1) * 96);
-  UN_A(p->c[2], sizeof(bf) * pix(2) * 128);
+    take(p->b4[i], sizeof(bf) * pix(3) * 64);
   // d[0] = d1 @G1 (16), d[1] = d2 @G2 (32), d[2] = d3 @G3 (64)
-  UN_A(p->d[0], sizeof(bf) * pix(0) * 16);
-  UN_A(p->d[1], sizeof(bf) * pix(1) * 32);
-  UN_A(p->d[2], sizeof(bf) * pix(2) * 64);
-  UN_A(p->yout, sizeof(float) * pix(0) * 8);
-  UN_A(p->dy8, sizeof(bf) * pix(0) * 8);
-  // largest dpre: G1 x 16 or G2 x 32 or G3 x 64 channels
-  size_t dmax = std::max(std::max(pix(0) * 16, pix(1) * 32), std::max(pix(2) * 64, pix(3) * 64));
-  UN_A(p->dpre, sizeof(bf) * dmax);
-  UN_A(p->dc[0], sizeof(float) * pix(0) * 48);
-  UN_A(p->dc[1], sizeof(float) * pix(1) * 96);
-  UN_A(p->dc[2], sizeof(float) * pix(2) * 128);
-  UN_A(p->gs, sizeof(float) * std::max(std::max(pix(0) * 16, pix(3) * 64), std::max(pix(2) * 32, pix(1) * 16)));
-  p->wpart_n = size_t(148) * 8 * 64 * WBN;   // splits * cout * 9 cin_pad <= (1184 / ntile) * 64 * ntile * WBN
-  UN_A(p->wpart, sizeof(float) * p->wpart_n);
-  p->bpart_n = (pix(0) + 2047) / 2048 * 64 + 64;
-  UN_A(p->bpart, sizeof(float) * p->bpart_n);
-  UN_A(p->mse_part, sizeof(double) * 1024);
-  UN_A(p->mse_loss, sizeof(double));
-#undef UN_A
+  for(int i = 0; i < 3; ++i)
+    take(p->d[i], sizeof(bf) * pix(i) * ech[i]);
+  // largest pre-activation gradient: G1 x 16, G2 x 32, G3 x 64 or G4 x 64 channels
+  const size_t dmax = std::max(std::max(pix(0) * 16, pix(1) * 32), std::max(pix(2) * 64, pix(3) * 64));
+  for(int i = 0; i < 2; ++i)
+    take(p->dpre[i], sizeof(bf) * dmax);
+  // data gradients of [U(d2), e1] @G1, [U(d3), e2] @G2, [U(e4), e3] @G3
+  const int uch[3] = {32, 64, 64};
+  for(int i = 0; i < 3; ++i)
+  {
+    take(p->du[i], sizeof(float) * pix(i) * uch[i]);
+    take(p->dk[i], sizeof(float) * pix(i) * ech[i]);
+  }
+  take(p->gs, sizeof(float) * std::max(pix(3) * 64, std::max(pix(2) * 32, pix(1) * 16)));
+  take(p->mse_part, sizeof(double) * 1024);
+  FB_CUDA(cudaMalloc(&p->arena, total));
+  const cudaError_t z = cudaMemset(p->arena, 0, zeroed);
+  if(z != cudaSuccess)
+  {
+    cudaFree(p->arena);
+    return cuda_fail(z, "cudaMemset");
+  }
+  for(const auto& w : want)
+    *w.first = static_cast<unsigned char*>(p->arena) + w.second;
   *out = u.release();
   return FB_OK;
 }
@@ -932,8 +1086,7 @@ void fb_unet_destroy(fb_unet* u)
 {
   if(!u)
     return;
-  for(void* a : u->allocs)
-    cudaFree(a);
+  cudaFree(u->arena);
   delete u;
 }
 
@@ -997,40 +1150,20 @@ fb_status fb_unet_forward(fb_unet* u, const float* in, float* out, int batch, vo
   }
   cudaStream_t st = as_stream(stream);
   const int B = batch;
-  const int* G = u->G;
-  const size_t P0 = size_t(B) * G[0] * G[0];
-  k_pack_input<<<grid_for(P0), 256, 0, st>>>(in, B, G[0], u->x8);
+  k_pack_input<<<grid_for(size_t(B) * u->G[0] * u->G[0]), 256, 0, st>>>(in, B, u->G[0], u->xp);
   FB_LAUNCHED(1);
-  UN_TRY(conv_fwd(u, 0, u->x8, B, G[0], u->e[0], 16, true, true, st));
-  const int ech[4] = {16, 32, 64, 64};
-  for(int i = 0; i < 3; ++i)
-  {
-    const size_t nc = size_t(B) * G[i + 1] * G[i + 1] * (ech[i] / 8);
-    k_subsample<<<grid_for(nc), 256, 0, st>>>(u->e[i], B, G[i], ech[i], u->s[i]);
-    FB_LAUNCHED(1);
-    UN_TRY(conv_fwd(u, i + 1, u->s[i], B, G[i + 1], u->e[i + 1], ech[i + 1], true, true, st));
-  }
+  UN_TRY((conv_fwd<8, 16, 1, IN_PAIR, OUT_RELU, 9>(u, 0, Input{u->xp, nullptr, 0, 8, 0}, B, u->e[0], st)));
+  UN_TRY((conv_fwd<16, 32, 1, IN_SUB, OUT_RELU, 9>(u, 1, plain(u->e[0], 16), B, u->e[1], st)));
+  UN_TRY((conv_fwd<32, 64, 1, IN_SUB, OUT_RELU, 9>(u, 2, plain(u->e[1], 32), B, u->e[2], st)));
+  UN_TRY((conv_fwd<64, 64, 1, IN_SUB, OUT_RELU, 2>(u, 3, plain(u->e[2], 64), B, u->e[3], st)));
   // bottleneck: dilation 2 and 4
-  UN_TRY(conv_fwd(u, 4, u->e[3], B, G[3], u->b4[0], 64, true, true, st));
-  UN_TRY(conv_fwd(u, 5, u->b4[0], B, G[3], u->b4[1], 64, true, true, st));
+  UN_TRY((conv_fwd<64, 64, 2, IN_PLAIN, OUT_RELU, 2>(u, 4, plain(u->e[3], 64), B, u->b4[0], st)));
+  UN_TRY((conv_fwd<64, 64, 4, IN_PLAIN, OUT_RELU, 2>(u, 5, plain(u->b4[0], 64), B, u->b4[1], st)));
   // decoder
-  {
-    const size_t n3 = size_t(B) * G[2] * G[2] * 128;
-    k_upsample_cat<<<grid_for(n3), 256, 0, st>>>(u->b4[1], 64, u->e[2], 64, B, G[2], u->c[2]);
-    FB_LAUNCHED(1);
-    UN_TRY(conv_fwd(u, 6, u->c[2], B, G[2], u->d[2], 64, true, true, st));
-    const size_t n2 = size_t(B) * G[1] * G[1] * 96;
-    k_upsample_cat<<<grid_for(n2), 256, 0, st>>>(u->d[2], 64, u->e[1], 32, B, G[1], u->c[1]);
-    FB_LAUNCHED(1);
-    UN_TRY(conv_fwd(u, 7, u->c[1], B, G[1], u->d[1], 32, true, true, st));
-    const size_t n1 = size_t(B) * G[0] * G[0] * 48;
-    k_upsample_cat<<<grid_for(n1), 256, 0, st>>>(u->d[1], 32, u->e[0], 16, B, G[0], u->c[0]);
-    FB_LAUNCHED(1);
-    UN_TRY(conv_fwd(u, 8, u->c[0], B, G[0], u->d[0], 16, true, true, st));
-    UN_TRY(conv_fwd(u, 9, u->d[0], B, G[0], u->yout, 8, false, false, st));
-  }
-  k_unpack_out<<<grid_for(P0), 256, 0, st>>>(u->yout, P0, out);
-  FB_LAUNCHED(1);
+  UN_TRY((conv_fwd<128, 64, 1, IN_CAT, OUT_RELU, 2>(u, 6, concat(u->b4[1], 64, u->e[2], 64), B, u->d[2], st)));
+  UN_TRY((conv_fwd<96, 32, 1, IN_CAT, OUT_RELU, 2>(u, 7, concat(u->d[2], 64, u->e[1], 32), B, u->d[1], st)));
+  UN_TRY((conv_fwd<48, 16, 1, IN_CAT, OUT_RELU, 9>(u, 8, concat(u->d[1], 32, u->e[0], 16), B, u->d[0], st)));
+  UN_TRY((conv_fwd<16, 8, 1, IN_PLAIN, OUT_FIRST, 9>(u, 9, plain(u->d[0], 16), B, out, st)));
   return FB_OK;
 }
 
@@ -1046,58 +1179,58 @@ fb_status fb_unet_backward(fb_unet* u, const float* dout, int batch, int accumul
   cudaStream_t st = as_stream(stream);
   const int B = batch;
   const int* G = u->G;
-  const int acc = accumulate ? 1 : 0;
-  const size_t P0 = size_t(B) * G[0] * G[0];
-  auto n_at = [&](int lv, int C) { return size_t(B) * G[lv] * G[lv] * C; };
-  // L8 (input d1): dy8 = dout
-  k_pack_dout<<<grid_for(P0), 256, 0, st>>>(dout, P0, u->dy8);
+  bf *p0 = u->dpre[0], *p1 = u->dpre[1];
+  auto n8 = [&](int lv, int C) { return size_t(B) * G[lv] * G[lv] * (C / 8); };
+  // dpre = mask(post) * U^T(du) at level lv + 1 (C channels)
+  auto up_bwd = [&](int lv, int C, const bf* post, bf* dpre)
+  {
+    k_upsample_bwd_mask<<<grid_for(n8(lv + 1, C)), 256, 0, st>>>(u->du[lv], C, B, G[lv], post, dpre);
+    FB_LAUNCHED(1);
+    return fb_status(FB_OK);
+  };
+  // dpre = mask(e[lv]) * (skip gradient + S^T(gs))
+  auto skip_bwd = [&](int lv, int C, bf* dpre)
+  {
+    k_grad_mask<<<grid_for(n8(lv, C)), 256, 0, st>>>(u->e[lv], C, B, G[lv], u->dk[lv], u->gs, dpre);
+    FB_LAUNCHED(1);
+    return fb_status(FB_OK);
+  };
+  // L8 (input d1)
+  const Input dy8{dout, nullptr, 0, 8, 0};
+  UN_TRY((wgrad<16, 16, 1, IN_PLAIN, true, 9>(u, 9, dout, plain(u->d[0], 16), B, st)));
+  UN_TRY((conv_bwd<8, 16, 1, IN_SCALAR, OUT_MASK, 9>(u, 9, dy8, B, p0, nullptr, 0, u->d[0], st)));
+  // L7 (input [U(d2), e1])
+  UN_TRY((wgrad<48, 16, 1, IN_CAT, false, 9>(u, 8, p0, concat(u->d[1], 32, u->e[0], 16), B, st)));
+  UN_TRY((conv_bwd<16, 48, 1, IN_PLAIN, OUT_F32, 9>(u, 8, plain(p0, 16), B, u->du[0], u->dk[0], 32, nullptr, st)));
+  UN_TRY(up_bwd(0, 32, u->d[1], p1));
+  // L6 (input [U(d3), e2])
+  UN_TRY((wgrad<96, 32, 1, IN_CAT, false, 9>(u, 7, p1, concat(u->d[2], 64, u->e[1], 32), B, st)));
+  UN_TRY((conv_bwd<32, 48, 1, IN_PLAIN, OUT_F32, 9>(u, 7, plain(p1, 32), B, u->du[1], u->dk[1], 64, nullptr, st)));
+  UN_TRY(up_bwd(1, 64, u->d[2], p0));
+  // L5 (input [U(e4), e3])
+  UN_TRY((wgrad<64, 64, 1, IN_CAT, false, 12>(u, 6, p0, concat(u->b4[1], 64, u->e[2], 64), B, st)));
+  UN_TRY((conv_bwd<64, 64, 1, IN_PLAIN, OUT_F32, 2>(u, 6, plain(p0, 64), B, u->du[2], u->dk[2], 64, nullptr, st)));
+  UN_TRY(up_bwd(2, 64, u->b4[1], p1));
+  // bottleneck: dilation 4 (input b4[0]), dilation 2 (input e4 = e[3]), L4 (input S(e3))
+  UN_TRY((wgrad<64, 64, 4, IN_PLAIN, false, 12>(u, 5, p1, plain(u->b4[0], 64), B, st)));
+  UN_TRY((conv_bwd<64, 64, 4, IN_PLAIN, OUT_MASK, 2>(u, 5, plain(p1, 64), B, p0, nullptr, 0, u->b4[0], st)));
+  UN_TRY((wgrad<64, 64, 2, IN_PLAIN, false, 12>(u, 4, p0, plain(u->e[3], 64), B, st)));
+  UN_TRY((conv_bwd<64, 64, 2, IN_PLAIN, OUT_MASK, 2>(u, 4, plain(p0, 64), B, p1, nullptr, 0, u->e[3], st)));
+  UN_TRY((wgrad<64, 64, 1, IN_SUB, false, 12>(u, 3, p1, plain(u->e[2], 64), B, st)));
+  UN_TRY((conv_bwd<64, 64, 1, IN_PLAIN, OUT_F32, 2>(u, 3, plain(p1, 64), B, u->gs, nullptr, 64, nullptr, st)));
+  // L3 (input S(e2))
+  UN_TRY(skip_bwd(2, 64, p0));
+  UN_TRY((wgrad<32, 64, 1, IN_SUB, false, 9>(u, 2, p0, plain(u->e[1], 32), B, st)));
+  UN_TRY((conv_bwd<64, 32, 1, IN_PLAIN, OUT_F32, 2>(u, 2, plain(p0, 64), B, u->gs, nullptr, 32, nullptr, st)));
+  // L2 (input S(e1))
+  UN_TRY(skip_bwd(1, 32, p1));
+  UN_TRY((wgrad<16, 32, 1, IN_SUB, false, 9>(u, 1, p1, plain(u->e[0], 16), B, st)));
+  UN_TRY((conv_bwd<32, 16, 1, IN_PLAIN, OUT_F32, 9>(u, 1, plain(p1, 32), B, u->gs, nullptr, 16, nullptr, st)));
+  // L1 (input f, log kappa)
+  UN_TRY(skip_bwd(0, 16, p0));
+  UN_TRY((wgrad<8, 16, 1, IN_PAIR, false, 5>(u, 0, p0, Input{u->xp, nullptr, 0, 8, 0}, B, st)));
+  k_grad_reduce<<<unsigned((u->nparam + GR_E - 1) / GR_E), GR_E * GR_G, 0, st>>>(net_map(u, B), u->grad, accumulate ? 1 : 0);
   FB_LAUNCHED(1);
-  UN_TRY(conv_bwd_weight(u, 9, u->dy8, u->d[0], B, G[0], acc, st));
-  UN_TRY(conv_bwd_data(u, 9, u->dy8, B, G[0], u->gs, st));                       // d1 grad [P0][16]
-  // L7 (input c1 = [U(d2), e1]): dpre = mask(d1) * gs
-  k_grad_mask<<<grid_for(n_at(0, 16)), 256, 0, st>>>(u->d[0], 16, B, G[0], u->gs, 16, 0, nullptr, 0, u->dpre);
-  FB_LAUNCHED(1);
-  UN_TRY(conv_bwd_weight(u, 8, u->dpre, u->c[0], B, G[0], acc, st));
-  UN_TRY(conv_bwd_data(u, 8, u->dpre, B, G[0], u->dc[0], st));                   // dc1 [P0][48]
-  // L6 (input c2 = [U(d3), e2]): dpre = mask(d2) * U^T(dc1[:, 0:32])
-  k_upsample_bwd_mask<<<grid_for(n_at(1, 32)), 256, 0, st>>>(u->dc[0], 48, 0, 32, B, G[0], u->d[1], u->dpre);
-  FB_LAUNCHED(1);
-  UN_TRY(conv_bwd_weight(u, 7, u->dpre, u->c[1], B, G[1], acc, st));
-  UN_TRY(conv_bwd_data(u, 7, u->dpre, B, G[1], u->dc[1], st));                   // dc2 [P1][96]
-  // L5 (input c3 = [U(e4), e3]): dpre = mask(d3) * U^T(dc2[:, 0:64])
-  k_upsample_bwd_mask<<<grid_for(n_at(2, 64)), 256, 0, st>>>(u->dc[1], 96, 0, 64, B, G[1], u->d[2], u->dpre);
-  FB_LAUNCHED(1);
-  UN_TRY(conv_bwd_weight(u, 6, u->dpre, u->c[2], B, G[2], acc, st));
-  UN_TRY(conv_bwd_data(u, 6, u->dpre, B, G[2], u->dc[2], st));                   // dc3 [P2][128]
-  // bottleneck, dilation 4 (input b4[0]): dpre = mask(e4) * U^T(dc3[:, 0:64])
-  k_upsample_bwd_mask<<<grid_for(n_at(3, 64)), 256, 0, st>>>(u->dc[2], 128, 0, 64, B, G[2], u->b4[1], u->dpre);
-  FB_LAUNCHED(1);
-  UN_TRY(conv_bwd_weight(u, 5, u->dpre, u->b4[0], B, G[3], acc, st));
-  UN_TRY(conv_bwd_data(u, 5, u->dpre, B, G[3], u->gs, st));                      // b4[0] grad [P3][64]
-  // bottleneck, dilation 2 (input e4a = e[3])
-  k_grad_mask<<<grid_for(n_at(3, 64)), 256, 0, st>>>(u->b4[0], 64, B, G[3], u->gs, 64, 0, nullptr, 0, u->dpre);
-  FB_LAUNCHED(1);
-  UN_TRY(conv_bwd_weight(u, 4, u->dpre, u->e[3], B, G[3], acc, st));
-  UN_TRY(conv_bwd_data(u, 4, u->dpre, B, G[3], u->gs, st));                      // e[3] grad [P3][64]
-  // L4 (input s3 = S(e3))
-  k_grad_mask<<<grid_for(n_at(3, 64)), 256, 0, st>>>(u->e[3], 64, B, G[3], u->gs, 64, 0, nullptr, 0, u->dpre);
-  FB_LAUNCHED(1);
-  UN_TRY(conv_bwd_weight(u, 3, u->dpre, u->s[2], B, G[3], acc, st));
-  UN_TRY(conv_bwd_data(u, 3, u->dpre, B, G[3], u->gs, st));                      // s3 grad [P3][64]
-  // L3 (input s2): dpre = mask(e3) * (dc3[:, 64:128] + S^T(gs))
-  k_grad_mask<<<grid_for(n_at(2, 64)), 256, 0, st>>>(u->e[2], 64, B, G[2], u->dc[2], 128, 64, u->gs, 64, u->dpre);
-  FB_LAUNCHED(1);
-  UN_TRY(conv_bwd_weight(u, 2, u->dpre, u->s[1], B, G[2], acc, st));
-  UN_TRY(conv_bwd_data(u, 2, u->dpre, B, G[2], u->gs, st));                      // s2 grad [P2][32]
-  // L2 (input s1): dpre = mask(e2) * (dc2[:, 64:96] + S^T(gs))
-  k_grad_mask<<<grid_for(n_at(1, 32)), 256, 0, st>>>(u->e[1], 32, B, G[1], u->dc[1], 96, 64, u->gs, 32, u->dpre);
-  FB_LAUNCHED(1);
-  UN_TRY(conv_bwd_weight(u, 1, u->dpre, u->s[0], B, G[1], acc, st));
-  UN_TRY(conv_bwd_data(u, 1, u->dpre, B, G[1], u->gs, st));                      // s1 grad [P1][16]
-  // L1 (input x8): dpre = mask(e1) * (dc1[:, 32:48] + S^T(gs))
-  k_grad_mask<<<grid_for(n_at(0, 16)), 256, 0, st>>>(u->e[0], 16, B, G[0], u->dc[0], 48, 32, u->gs, 16, u->dpre);
-  FB_LAUNCHED(1);
-  UN_TRY(conv_bwd_weight(u, 0, u->dpre, u->x8, B, G[0], acc, st));
   return FB_OK;
 }
 
@@ -1112,10 +1245,11 @@ fb_status fb_unet_adam(fb_unet* u, float lr, float beta1, float beta2, float eps
   }
   cudaStream_t st = as_stream(stream);
   const float c1 = 1.f - std::pow(beta1, float(t)), c2 = 1.f - std::pow(beta2, float(t));
-  k_adam<<<grid_for(u->nparam), 256, 0, st>>>(u->param, u->grad, u->adam_m, u->adam_v, u->nparam, lr, beta1, beta2,
-    eps, c1, c2);
+  k_adam<<<unsigned((u->nparam + 255) / 256), 256, 0, st>>>(net_map(u, 0), u->param, u->grad, u->adam_m, u->adam_v, lr,
+    beta1, beta2, eps, c1, c2);
   FB_LAUNCHED(1);
-  return prep_weights(u, st);
+  u->weights_ready = true;
+  return FB_OK;
 }
 
 // Mean squared error over n entries (DEVICE arrays): *loss (DEVICE double) = sum (y - t)^2 / n;
@@ -1129,9 +1263,8 @@ fb_status fb_unet_mse(fb_unet* u, const float* y, const float* t, uint64_t n, fl
   }
   cudaStream_t st = as_stream(stream);
   const int nb = int(std::min<uint64_t>(1024, (n + MSE_NT - 1) / MSE_NT));
-  k_mse<<<nb, MSE_NT, 0, st>>>(y, t, size_t(n), grad, u->mse_part);
-  k_mse_final<<<1, 1, 0, st>>>(u->mse_part, nb, size_t(n), loss);
-  FB_LAUNCHED(2);
+  k_mse<<<nb, MSE_NT, 0, st>>>(y, t, size_t(n), grad, RedSlot{u->mse_part, u->mse_counter}, loss);
+  FB_LAUNCHED(1);
   return FB_OK;
 }
 

@@ -62,6 +62,25 @@ def test_forward_backward_match_oracle(featlib, cuda, G, B):
         assert _rel(g[sl], go[sl]) <= GRAD_TOL, (sl, _rel(g[sl], go[sl]))
 
 
+@pytest.mark.parametrize("G,B", [(9, 2), (17, 150), (65, 3)])
+def test_tile_edges_match_oracle(featlib, cuda, G, B):
+    """Grids of one partial tile (9, 5, 3, 2 points per side), a batch with enough tiles on every
+    grid for the kernels that take all output channels per block (150), and whole tiles with a
+    ragged last one (65 = 6 x 11 - 1): the tolerances of the comparison above."""
+    torch = cuda
+    net, theta, inp, tgt, inp_d, tgt_d = _setup(torch, G, B, seed=G)
+    y = net.forward(inp_d)
+    grad = torch.empty_like(y)
+    net.mse(y, tgt_d, grad)
+    net.backward(grad)
+    yo, cache = UO.forward(theta.astype(np.float64), inp, exact=False)
+    assert _rel(y.cpu().numpy(), yo) <= FWD_TOL
+    go = UO.backward(cache, grad.cpu().numpy().astype(np.float64), exact=False)
+    g = net.get_grads()
+    for sl in _layer_slices():
+        assert _rel(g[sl], go[sl]) <= GRAD_TOL, (sl, _rel(g[sl], go[sl]))
+
+
 def test_backward_accumulates(featlib, cuda):
     torch = cuda
     net, theta, inp, tgt, inp_d, tgt_d = _setup(torch, 17, 2, seed=5)
