@@ -7,13 +7,15 @@
 //
 // kappa = exp(g), g(x, y) = s * sum_{i,j} (xi_ij cos t + eta_ij sin t) / (kx_i^2 + ky_j^2),
 // t = 2 pi (kx_i x + ky_j y), kx = ky = -K/2 .. K/2-1 (the (0,0) mode excluded); f = sum of
-// Gaussians a * exp(-|x - c|^2 / (2 w^2)).  Pass 1 computes every cell's 4x4 element matrix and
-// 4 load contributions (one thread per cell); pass 2 sums them per matrix entry / vertex (one
-// thread per vertex, cells in ascending index order), so no atomics are needed and the result is
-// deterministic.
+// Gaussians a * exp(-|x - c|^2 / (2 w^2)).  Both are separable: pass 1 tabulates their factors per
+// quadrature coordinate; pass 2 computes, for every tile of vertices, the 4x4 element matrices and
+// load contributions of the cells around it in shared memory (one thread per cell) and sums them per
+// matrix entry / vertex (one thread per vertex, cells in ascending index order), so no atomics are
+// needed and the result is deterministic.
 #include "fb_common.cuh"
 
 #include <cmath>
+#include <mutex>
 #include <vector>
 
 namespace fb
@@ -57,104 +59,154 @@ namespace as
     return s * acc;
   }
 
-  // Separable tables of the field at the quadrature coordinates (3 per cell and direction, index
-  // 3*cell + q): ex[t][i] = e^{2 pi i kx_i x_t} and hy[t][i] = sum_j c_ij e^{2 pi i ky_j y_t}, so that
-  // g(x_t, y_u) = s * sum_i Re(ex[t][i] * hy[u][i]): K complex products per point instead of K^2
-  // sine/cosine pairs.
-  __global__ void k_field_tables(int N, double h, int K, const double* __restrict__ xi,
-    const double* __restrict__ eta, double2* __restrict__ ex, double2* __restrict__ hy)
+  // Separable tables at the quadrature coordinates (3 per cell and direction, index 3*cell + q):
+  //   field: ex[t][i] = e^{2 pi i kx_i x_t} and hy[t][i] = sum_j c_ij e^{2 pi i ky_j y_t}, so that
+  //     g(x_t, y_u) = s * sum_i Re(ex[t][i] * hy[u][i]): K complex products per point instead of K^2
+  //     sine/cosine pairs (kx = ky, so hy's exponentials are ex's, formed once per block);
+  //   Gaussians: gx[t][g] = a exp(-(x_t - c_x)^2 / (2 w^2)), gy[t][g] = exp(-(y_t - c_y)^2 / (2 w^2)):
+  //     one product per Gaussian and point instead of an exponential (72 per cell for 8 Gaussians).
+  // One block per T coordinates; K <= 64.
+  constexpr int FT_T = 8;
+  __global__ void __launch_bounds__(128) k_tables(int N, double h, int K, const double* __restrict__ xi,
+    const double* __restrict__ eta, double2* __restrict__ ex, double2* __restrict__ hy, int ng,
+    const double* __restrict__ gauss, double* __restrict__ gx, double* __restrict__ gy)
   {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if(e >= 3 * N * K)
-      return;
+    __shared__ double2 se[FT_T][64];
     const double tp = 6.283185307179586476925286766559;
-    const int i = e % K, t = e / K;
-    const double c = (double(t / 3) + (1.0 + c_ref.xq[t % 3]) / 2.0) * h;   // x_t = y_t
-    const double kx = double(i - K / 2);
-    double sx, cx;
-    sincos(tp * kx * c, &sx, &cx);
-    ex[e] = make_double2(cx, sx);
-    double hr = 0.0, hi = 0.0;
-    for(int j = 0; j < K; ++j)
+    const int t0 = blockIdx.x * FT_T, nt = min(FT_T, 3 * N - t0);
+    for(int e = threadIdx.x; e < nt * K; e += 128)
     {
-      const double ky = double(j - K / 2);
-      const double den = kx * kx + ky * ky;
-      if(den == 0.0)
-        continue;
-      double sy, cy;
-      sincos(tp * ky * c, &sy, &cy);
-      const double a = __ldg(xi + i * K + j) / den, b = __ldg(eta + i * K + j) / den;
-      hr += a * cy + b * sy;
-      hi += a * sy - b * cy;
+      const int i = e % K, t = t0 + e / K;
+      const double c = (double(t / 3) + (1.0 + c_ref.xq[t % 3]) / 2.0) * h;   // x_t = y_t
+      const double kx = double(i - K / 2);
+      double sx, cx;
+      sincos(tp * kx * c, &sx, &cx);
+      se[e / K][i] = make_double2(cx, sx);
+      ex[size_t(t) * K + i] = make_double2(cx, sx);
     }
-    hy[e] = make_double2(hr, hi);
+    for(int e = threadIdx.x; e < nt * ng; e += 128)
+    {
+      const int g = e % ng, t = t0 + e / ng;
+      const double c = (double(t / 3) + (1.0 + c_ref.xq[t % 3]) / 2.0) * h;
+      const double dx = c - gauss[4 * g + 0], dy = c - gauss[4 * g + 1], w = gauss[4 * g + 2];
+      gx[size_t(t) * ng + g] = gauss[4 * g + 3] * exp(-(dx * dx) / (2.0 * w * w));
+      gy[size_t(t) * ng + g] = exp(-(dy * dy) / (2.0 * w * w));
+    }
+    __syncthreads();
+    for(int e = threadIdx.x; e < nt * K; e += 128)
+    {
+      const int i = e % K, t = e / K;
+      const double kx = double(i - K / 2);
+      double hr = 0.0, hi = 0.0;
+      for(int j = 0; j < K; ++j)
+      {
+        const double ky = double(j - K / 2);
+        const double den = kx * kx + ky * ky;
+        if(den == 0.0)
+          continue;
+        const double cy = se[t][j].x, sy = se[t][j].y;
+        const double a = __ldg(xi + i * K + j) / den, b = __ldg(eta + i * K + j) / den;
+        hr += a * cy + b * sy;
+        hi += a * sy - b * cy;
+      }
+      hy[size_t(t0 + t) * K + i] = make_double2(hr, hi);
+    }
   }
 
-  // per cell: the 4x4 element matrix (kappa-weighted) and the 4 load-vector contributions
-  __global__ void k_cells(int N, double h, int K, const double2* __restrict__ ex, const double2* __restrict__ hy,
-    double s, int ng, const double* __restrict__ gauss, double* __restrict__ ke, double* __restrict__ fe)
-  {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if(c >= N * N)
-      return;
-    const int cx = c % N, cy = c / N;
-    double kq[9], fq[9];
-    for(int qy = 0; qy < 3; ++qy)
-      for(int qx = 0; qx < 3; ++qx)
-      {
-        const int q = qx * 3 + qy;   // reference order: x index slowest (meshgrid "ij" over (x, y))
-        const double x = (double(cx) + (1.0 + c_ref.xq[qx]) / 2.0) * h;
-        const double y = (double(cy) + (1.0 + c_ref.xq[qy]) / 2.0) * h;
-        double kv = 1.0;
-        if(K > 0 && ke)
-        {
-          const double2* exr = ex + size_t(cx * 3 + qx) * K;
-          const double2* hyr = hy + size_t(cy * 3 + qy) * K;
-          double g = 0.0;
-          for(int i = 0; i < K; ++i)
-          {
-            const double2 a = __ldg(exr + i), b = __ldg(hyr + i);
-            g += b.x * a.x - b.y * a.y;
-          }
-          kv = exp(s * g);
-        }
-        kq[q] = kv;
-        double f = 0.0;
-        for(int g = 0; g < ng && fe; ++g)
-        {
-          const double dx = x - gauss[4 * g + 0], dy = y - gauss[4 * g + 1], w = gauss[4 * g + 2];
-          f += gauss[4 * g + 3] * exp(-(dx * dx + dy * dy) / (2.0 * w * w));
-        }
-        fq[q] = f;
-      }
-    if(ke)
-      for(int a = 0; a < 4; ++a)
-        for(int b = 0; b < 4; ++b)
-        {
-          double v = 0.0;
-          for(int q = 0; q < 9; ++q)
-            v += kq[q] * (c_ref.wq[q / 3] * c_ref.wq[q % 3]) * c_ref.gg[q][a][b];
-          ke[size_t(c) * 16 + a * 4 + b] = v;
-        }
-    if(fe)
-      for(int a = 0; a < 4; ++a)
-      {
-        double v = 0.0;
-        for(int q = 0; q < 9; ++q)
-          v += fq[q] * (c_ref.wq[q / 3] * c_ref.wq[q % 3]) * c_ref.val[q][a];
-        fe[size_t(c) * 4 + a] = (h / 2.0) * (h / 2.0) * v;
-      }
-  }
-
-  // per vertex: stiffness row (sorted neighbours) and load entry, summing cells in ascending order
-  __global__ void k_vertices(int N, const double* __restrict__ ke, const double* __restrict__ fe,
+  // One block per AT x AT vertices: the (AT + 1)^2 = 256 cells around them, one thread each (the
+  // kappa-weighted 4x4 element matrix and the 4 load contributions, in shared memory), then one
+  // thread per vertex (its stiffness row, sorted neighbours, and its load entry, cells in ascending
+  // order).  The cells on a tile's rim are computed by up to four blocks (1.14 cells per vertex); in
+  // exchange the element matrices (33 MB at level 9) never leave the SM.
+  constexpr int AT = 15, AC = AT + 1;
+  __global__ void __launch_bounds__(AC * AC) k_assemble(int N, double h, int K, const double2* __restrict__ ex,
+    const double2* __restrict__ hy, double s, int ng, const double* __restrict__ gx, const double* __restrict__ gy,
     const uint64_t* __restrict__ rp, double* __restrict__ vals, double* __restrict__ rhs)
   {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n1 = N + 1;
-    if(v >= n1 * n1)
+    __shared__ double ke[16][AC * AC];
+    __shared__ double fe[4][AC * AC];
+    const int vx0 = blockIdx.x * AT, vy0 = blockIdx.y * AT;   // first vertex; cells from (vx0 - 1, vy0 - 1)
+    const int tid = threadIdx.x;
+    {
+      const int cx = vx0 - 1 + tid % AC, cy = vy0 - 1 + tid / AC;
+      if(cx >= 0 && cy >= 0 && cx < N && cy < N)
+      {
+        if(vals)
+        {
+          double kq[9];
+          #pragma unroll
+          for(int q = 0; q < 9; ++q)
+            kq[q] = c_ref.wq[q / 3] * c_ref.wq[q % 3];
+          if(K > 0)
+          {
+            // reference order of the points: x index slowest (meshgrid "ij" over (x, y))
+            double g[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            const double2* exr = ex + size_t(cx) * 3 * K;
+            const double2* hyr = hy + size_t(cy) * 3 * K;
+            for(int i = 0; i < K; ++i)
+            {
+              double2 a[3], b[3];
+              #pragma unroll
+              for(int q = 0; q < 3; ++q)
+              {
+                a[q] = __ldg(exr + q * K + i);
+                b[q] = __ldg(hyr + q * K + i);
+              }
+              #pragma unroll
+              for(int q = 0; q < 9; ++q)
+                g[q] += b[q % 3].x * a[q / 3].x - b[q % 3].y * a[q / 3].y;
+            }
+            #pragma unroll
+            for(int q = 0; q < 9; ++q)
+              kq[q] *= exp(s * g[q]);
+          }
+          for(int a = 0; a < 4; ++a)
+            for(int b = 0; b < 4; ++b)
+            {
+              double v = 0.0;
+              #pragma unroll
+              for(int q = 0; q < 9; ++q)
+                v += kq[q] * c_ref.gg[q][a][b];
+              ke[a * 4 + b][tid] = v;
+            }
+        }
+        if(rhs)
+        {
+          double fq[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+          const double* xr = gx + size_t(cx) * 3 * ng;
+          const double* yr = gy + size_t(cy) * 3 * ng;
+          for(int g = 0; g < ng; ++g)
+          {
+            double a[3], b[3];
+            #pragma unroll
+            for(int q = 0; q < 3; ++q)
+            {
+              a[q] = __ldg(xr + q * ng + g);
+              b[q] = __ldg(yr + q * ng + g);
+            }
+            #pragma unroll
+            for(int q = 0; q < 9; ++q)
+              fq[q] += a[q / 3] * b[q % 3];
+          }
+          #pragma unroll
+          for(int a = 0; a < 4; ++a)
+          {
+            double v = 0.0;
+            #pragma unroll
+            for(int q = 0; q < 9; ++q)
+              v += fq[q] * (c_ref.wq[q / 3] * c_ref.wq[q % 3]) * c_ref.val[q][a];
+            fe[a][tid] = (h / 2.0) * (h / 2.0) * v;
+          }
+        }
+      }
+    }
+    __syncthreads();
+    const int ix = vx0 + tid % AC, iy = vy0 + tid / AC;
+    if(tid % AC >= AT || tid / AC >= AT || ix > N || iy > N)
       return;
-    const int ix = v % n1, iy = v / n1;
+    const int n1 = N + 1;
+    const size_t v = size_t(iy) * n1 + ix;
+    auto cell = [&](int cx, int cy) { return (cy - vy0 + 1) * AC + (cx - vx0 + 1); };
     if(vals)
     {
       uint64_t pos = rp[v];
@@ -164,25 +216,25 @@ namespace as
           const int jx = ix + dx, jy = iy + dy;
           if(jx < 0 || jy < 0 || jx > N || jy > N)
             continue;
-          double s = 0.0;
+          double t = 0.0;
           for(int cy = max(max(iy, jy) - 1, 0); cy <= min(min(iy, jy), N - 1); ++cy)
             for(int cx = max(max(ix, jx) - 1, 0); cx <= min(min(ix, jx), N - 1); ++cx)
             {
               const int a = (ix - cx) + 2 * (iy - cy);
               const int b = (jx - cx) + 2 * (jy - cy);
-              s += ke[(size_t(cy) * N + cx) * 16 + a * 4 + b];
+              t += ke[a * 4 + b][cell(cx, cy)];
             }
-          vals[pos++] = s;
+          vals[pos++] = t;
         }
     }
     if(rhs)
     {
-      double s = 0.0;
+      double t = 0.0;
       for(int cy = max(iy - 1, 0); cy <= min(iy, N - 1); ++cy)
         for(int cx = max(ix - 1, 0); cx <= min(ix, N - 1); ++cx)
-          s += fe[(size_t(cy) * N + cx) * 4 + (ix - cx) + 2 * (iy - cy)];
+          t += fe[(ix - cx) + 2 * (iy - cy)][cell(cx, cy)];
       const bool boundary = ix == 0 || iy == 0 || ix == N || iy == N;
-      rhs[v] = boundary ? 0.0 : s;
+      rhs[v] = boundary ? 0.0 : t;
     }
   }
 
@@ -357,6 +409,50 @@ namespace as
         }
   }
 
+  // Stream-ordered workspace from a pool of the library's own per device.  The device's default pool
+  // gives its memory back at every synchronisation, and assembly calls end with one: each call then
+  // mapped and unmapped its workspace anew (5 ms of the 9 ms that assembling, updating and solving a
+  // level-9 instance took).  The pool keeps at most POOL_KEEP bytes; what a call needs beyond that is
+  // given back at its synchronisation.
+  constexpr uint64_t POOL_KEEP = uint64_t(64) << 20;
+  static fb_status workspace(void** p, size_t bytes, cudaStream_t st)
+  {
+    static std::mutex mu;
+    static cudaMemPool_t pools[64] = {};
+    int dev = 0;
+    FB_CUDA(cudaGetDevice(&dev));
+    if(dev < 0 || dev >= 64)
+    {
+      FB_CUDA(cudaMallocAsync(p, bytes, st));
+      return FB_OK;
+    }
+    cudaMemPool_t pool;
+    {
+      std::lock_guard<std::mutex> lock(mu);
+      if(!pools[dev])
+      {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t np;
+        FB_CUDA(cudaMemPoolCreate(&np, &props));
+        uint64_t keep = POOL_KEEP;
+        const cudaError_t ke = cudaMemPoolSetAttribute(np, cudaMemPoolAttrReleaseThreshold, &keep);
+        if(ke != cudaSuccess)
+        {
+          cudaMemPoolDestroy(np);
+          return cuda_fail(ke, "cudaMemPoolSetAttribute");
+        }
+        pools[dev] = np;
+      }
+      pool = pools[dev];
+    }
+    FB_CUDA(cudaMallocFromPoolAsync(p, bytes, pool, st));
+    return FB_OK;
+  }
+
   static bool ref3_ready[64] = {};
   static fb_status upload_ref3()
   {
@@ -504,32 +600,29 @@ fb_status fb_q1_assemble_2d(int level, int kmodes, const double* xi, const doubl
   const int N = 1 << level;
   const double h = 1.0 / N;
   cudaStream_t st = as_stream(stream);
-  double *ke = nullptr, *fe = nullptr;
+  const int K = values ? kmodes : 0, ng = rhs ? ngauss : 0;
+  // the tables: ex, hy [3N][K] complex, gx, gy [3N][ng]
+  const size_t nt = 3 * size_t(N), bytes = nt * (size_t(K) * 2 * sizeof(double2) + size_t(ng) * 2 * sizeof(double));
+  void* ws = nullptr;
   double2 *ex = nullptr, *hy = nullptr;
-  const int K = values ? kmodes : 0;
-  if(values)
-    FB_CUDA(cudaMallocAsync((void**)&ke, sizeof(double) * 16 * size_t(N) * N, st));
-  if(rhs)
-    FB_CUDA(cudaMallocAsync((void**)&fe, sizeof(double) * 4 * size_t(N) * N, st));
-  if(K)
+  double *gx = nullptr, *gy = nullptr;
+  if(bytes)
   {
-    FB_CUDA(cudaMallocAsync((void**)&ex, sizeof(double2) * 3 * size_t(N) * K, st));
-    FB_CUDA(cudaMallocAsync((void**)&hy, sizeof(double2) * 3 * size_t(N) * K, st));
-    as::k_field_tables<<<(3 * N * K + 127) / 128, 128, 0, st>>>(N, h, K, xi, eta, ex, hy);
+    e = as::workspace(&ws, bytes, st);
+    if(e != FB_OK)
+      return e;
+    ex = static_cast<double2*>(ws);
+    hy = ex + nt * size_t(K);
+    gx = reinterpret_cast<double*>(hy + nt * size_t(K));
+    gy = gx + nt * size_t(ng);
+    as::k_tables<<<unsigned((nt + as::FT_T - 1) / as::FT_T), 128, 0, st>>>(N, h, K, xi, eta, ex, hy, ng, gauss, gx, gy);
     FB_LAUNCHED(1);
   }
-  const int cells = N * N, verts = (N + 1) * (N + 1);
-  as::k_cells<<<(cells + 127) / 128, 128, 0, st>>>(N, h, K, ex, hy, s, rhs ? ngauss : 0, gauss, ke, fe);
-  as::k_vertices<<<(verts + 255) / 256, 256, 0, st>>>(N, ke, fe, row_ptr, values, rhs);
-  FB_LAUNCHED(2);
-  if(ke)
-    FB_CUDA(cudaFreeAsync(ke, st));
-  if(fe)
-    FB_CUDA(cudaFreeAsync(fe, st));
-  if(ex)
-    FB_CUDA(cudaFreeAsync(ex, st));
-  if(hy)
-    FB_CUDA(cudaFreeAsync(hy, st));
+  const unsigned tiles = unsigned((N + as::AT) / as::AT);   // (N + 1) vertices per side
+  as::k_assemble<<<dim3(tiles, tiles), as::AC * as::AC, 0, st>>>(N, h, K, ex, hy, s, ng, gx, gy, row_ptr, values, rhs);
+  FB_LAUNCHED(1);
+  if(ws)
+    FB_CUDA(cudaFreeAsync(ws, st));
   FB_CUDA(cudaStreamSynchronize(st));
   return FB_OK;
 }
@@ -610,7 +703,9 @@ fb_status fb_q1_assemble_3d(int level, int ngauss, const double* gauss, const ui
   const long long cells = (long long)N * N * N, verts = (long long)(N + 1) * (N + 1) * (N + 1);
   if(rhs)
   {
-    FB_CUDA(cudaMallocAsync((void**)&fe, sizeof(double) * 8 * size_t(cells), st));
+    e = as::workspace((void**)&fe, sizeof(double) * 8 * size_t(cells), st);
+    if(e != FB_OK)
+      return e;
     as::k_cells3<<<unsigned((cells + 127) / 128), 128, 0, st>>>(N, h, ngauss, gauss, fe);
     FB_LAUNCHED(1);
   }

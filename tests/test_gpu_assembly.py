@@ -51,6 +51,29 @@ def test_assembly_matches_host(featlib, cuda, level, with_field):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("level,modes,sources", [(1, 2, 1), (4, 64, 40), (6, 3, 5)])
+def test_assembly_modes_and_sources(featlib, cuda, level, modes, sources):
+    """The tables' extremes (64 modes, many Gaussians, one partial tile of 3 x 3 vertices, a last tile
+    of 2 and of 5): within the tolerance of the comparison above."""
+    torch = cuda
+    from featb200.assembly_gpu import Q1Assembler2D
+    fp = AS.field_params(60 + level, modes)
+    gp = AS.gauss_params(70 + level, 2, sources)
+    vals, b = Q1Assembler2D(level).assemble(fp, gp)
+    torch.cuda.synchronize()
+
+    def kappa(x, y):
+        xs, ys = np.unique(x), np.unique(y)
+        return np.exp(AS.field_eval_grid(fp, xs, ys)[np.searchsorted(ys, y), np.searchsorted(xs, x)])
+
+    A = AS.stiffness(level, 2, kappa)
+    b_ref = AS.load_vector(level, lambda *xs: AS.gauss_eval(gp, *xs), 2)
+    b_ref[AS.boundary_dofs(level, 2).astype(np.int64)] = 0.0
+    assert np.abs(vals.cpu().numpy() - A.data).max() <= TOL * np.abs(A.data).max()
+    assert np.abs(b.cpu().numpy() - b_ref).max() <= TOL * max(np.abs(b_ref).max(), 1e-300)
+
+
+@pytest.mark.gpu
 def test_assembly_values_only_and_rhs_only(featlib, cuda):
     torch = cuda
     from featb200.assembly_gpu import Q1Assembler2D
