@@ -16,11 +16,17 @@
 
 namespace fb
 {
-  // Op::block_done() exists: the epilogue finishes each block itself (instead of the grid reduction)
+  // Op::Acc exists: the epilogue carries a per-thread accumulator through the block's rows (passed to
+  // op(i, sum, pre, acc)) and finishes each block itself (op.block_done(acc)) instead of the grid
+  // reduction.  Such a pass gives every block one contiguous range of chunks, so that consecutive
+  // chunks mostly belong to one instance and the accumulator is handed over a few times per block.
   template<class T, class = void>
-  struct HasBlockDone : std::false_type {};
+  struct HasAcc : std::false_type {};
   template<class T>
-  struct HasBlockDone<T, std::void_t<decltype(std::declval<const T&>().block_done())>> : std::true_type {};
+  struct HasAcc<T, std::void_t<typename T::Acc>> : std::true_type {};
+  struct NoAcc {};
+  template<class T, bool H> struct AccOf { typedef NoAcc type; };
+  template<class T> struct AccOf<T, true> { typedef typename T::Acc type; };
 
   constexpr int TMA_NT = 256;          // threads = rows per chunk
   constexpr int TMA_STAGES = 3;   // pipeline depth, at most
@@ -178,6 +184,18 @@ namespace fb
     const uint32_t sb = mb + (xlo && xstage ? xw * uint32_t(sizeof(S)) : 0u);
     const uint32_t nsl = padded_rows / 32u;
     const uint32_t nch = (padded_rows + TMA_NT - 1) / TMA_NT;
+    // this block's chunks: cfirst, cfirst + cstep, ... (ccount of them)
+    constexpr bool ACC = HasAcc<Op>::value;
+    uint32_t cfirst = blockIdx.x, cstep = gridDim.x, ccount;
+    if constexpr(ACC)
+    {
+      const uint32_t per = nch / gridDim.x, rem = nch % gridDim.x;
+      cfirst = blockIdx.x * per + min(blockIdx.x, rem);
+      ccount = per + (blockIdx.x < rem ? 1u : 0u);
+      cstep = 1u;
+    }
+    else
+      ccount = blockIdx.x < nch ? (nch - blockIdx.x + gridDim.x - 1u) / gridDim.x : 0u;
     auto issue = [&](uint32_t c, int s)
     {
       uint32_t e0, ne;
@@ -235,11 +253,8 @@ namespace fb
     {
       if(threadIdx.x == 0)
         for(int s = 0; s < NS; ++s)
-        {
-          const uint32_t c = blockIdx.x + uint32_t(s) * gridDim.x;
-          if(c < nch)
-            issue(c, s);
-        }
+          if(uint32_t(s) < ccount)
+            issue(cfirst + uint32_t(s) * cstep, s);
     };
     if(!xlo)
       issue_first();
@@ -251,14 +266,22 @@ namespace fb
       // drain the first copies (bounded) before the block exits
       if(threadIdx.x == 0)
         for(int s = 0; s < NS; ++s)
-          if(blockIdx.x + uint32_t(s) * gridDim.x < nch)
+          if(uint32_t(s) < ccount)
             mbar_wait(&bar[s], 0u);
       return;
     }
     double part = 0.0;
+    typename AccOf<Op, ACC>::type acc{};
+    auto row = [&](uint32_t i, Ac sum, const typename Op::Pre& pre)
+    {
+      if constexpr(ACC)
+        op(i, sum, pre, acc);
+      else
+        part += op(i, sum, pre);
+    };
     bool failed = false;
     uint32_t it = 0;
-    for(uint32_t c = blockIdx.x; c < nch; c += gridDim.x, ++it)
+    for(uint32_t c = cfirst; it < ccount; c += cstep, ++it)
     {
       const int s = int(it % NS);
       const uint32_t par = (it / NS) & 1u;
@@ -288,11 +311,10 @@ namespace fb
       // every thread is past the previous chunk: refill its stage (NS - 1 chunks ahead)
       if(threadIdx.x == 0 && it > 0)
       {
-        const uint32_t c2 = c - gridDim.x + uint32_t(NS) * gridDim.x;
-        if(c2 < nch)
+        if(it - 1 + uint32_t(NS) < ccount)
         {
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          issue(c2, int((it - 1) % NS));
+          issue(c + (uint32_t(NS) - 1u) * cstep, int((it - 1) % NS));
         }
       }
       const unsigned char* st = tma_smem + size_t(s) * sb;
@@ -308,7 +330,7 @@ namespace fb
           #pragma unroll
           for(int u = 0; u < (DG ? KC : 1); ++u)
             sum = add(sum, mul(to_acc(sv[base + uint32_t(u) * 32u]), xv[u]));
-          part += op(i, sum, dpre);
+          row(i, sum, dpre);
         }
       }
       else if(i < A.rows)
@@ -338,7 +360,7 @@ namespace fb
         }
         const auto sum = staged_row_sum<V, S, KC>(sv, narrow ? reinterpret_cast<const int16_t*>(scol) : nullptr,
           narrow ? nullptr : reinterpret_cast<const uint32_t*>(scol), kr, base, i, x, sx, x0, xl);
-        part += op(i, sum, pre);
+        row(i, sum, pre);
       }
     }
     if(failed)
@@ -353,8 +375,7 @@ namespace fb
         for(uint32_t k = 0; k < pending; ++k)
         {
           const uint32_t jt = it + k;
-          const uint32_t c = blockIdx.x + jt * gridDim.x;
-          if(c < nch)
+          if(jt < ccount)
             mbar_wait(&bar[jt % NS], (jt / NS) & 1u);
         }
       }
@@ -362,9 +383,9 @@ namespace fb
     }
     // an epilogue with its own end of block (the batched solver's per-instance reductions): every
     // thread of every block that ran the loop calls it once
-    if constexpr(HasBlockDone<Op>::value)
+    if constexpr(ACC)
     {
-      op.block_done();
+      op.block_done(acc);
       return;
     }
     if(!Op::REDUCES)

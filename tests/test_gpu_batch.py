@@ -105,3 +105,24 @@ def test_batch_rows_per_block(featlib, cuda, rows_per_block):
         assert fb.solve(s, x, fb.DenseVector(b)) == fb.Status.success
         assert bat.iterations()[k] == s.get_num_iter()
         assert rel_err(X[k], x.elements) <= 1e-12
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+def test_batch_many_instances_per_block(featlib, cuda, precision):
+    """Enough small instances (300 of levels 3 to 5) that a block's range of rows holds several of
+    them: the per-instance sums are handed over between warps of one instance and the next.  Equal
+    instances (every third) must take the same iterations, and FP64 solutions match single solves."""
+    fb = featlib
+    inst = _family([5, 3, 4])
+    hs = [fb.build_hierarchy(lv) for lv, _ in inst]
+    bat = fb.BatchPCG(hs * 100, precision=precision)
+    rhs = np.concatenate([b for _, b in inst] * 100)
+    X = bat.split(bat.solve(np.zeros_like(rhs), rhs))
+    assert all(st == fb.Status.success for st in bat.statuses())
+    for k, (lv, b) in enumerate(inst):
+        s = fb.build_pcg_multigrid(lv)
+        x = fb.DenseVector(b.size)
+        assert fb.solve(s, x, fb.DenseVector(b)) == fb.Status.success
+        assert len(set(bat.iterations()[k::3])) == 1
+        for j in (k, 150 + k, 297 + k):
+            assert rel_err(X[j], x.elements) <= (1e-12 if precision == "f64" else 1e-7)
