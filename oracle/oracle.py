@@ -28,6 +28,7 @@ FEAT_B200_BIN = os.path.join(REF_DIR, "feat_b200")
 FEAT_CUDA_BIN = os.path.join(REF_DIR, "feat_cuda")
 # the reference source tree the reference binary is compiled from (only where it exists)
 REF_SRC = os.environ.get("FEAT_REF", "/root/reference")
+HAVE_REF_SRC = os.path.exists(os.path.join(REF_SRC, "kernel", "runtime.hpp"))   # an empty folder is none
 
 STATUS = {0: "progress", 1: "success", 2: "aborted", 3: "diverged", 4: "max_iter"}
 
@@ -45,13 +46,13 @@ class _LevelIn(C.Structure):
 def build():
     """Compile the C restatement (and the reference driver when the reference tree exists)."""
     targets = ["port"]
-    if os.path.isdir(REF_SRC):
+    if HAVE_REF_SRC:
         targets.append("ref")
         # the FEAT build on the library's binding links the built library
         if os.path.exists(os.path.join(os.path.dirname(HERE), "feat3.doxytest_b200", "featb200", "libfeatb200.so")):
             targets.append("b200")
     subprocess.run(["make", "-s", "-j8", "-C", HERE, f"FEAT_REF={REF_SRC}"] + targets, check=True)
-    if os.path.isdir(REF_SRC):
+    if HAVE_REF_SRC:
         # FEAT on its own CUDA backend: only a timing column beside the library, so a failure to
         # build it (e.g. without the toolkit's cuSPARSE) leaves the checkers usable
         r = subprocess.run(["make", "-s", "-j8", "-C", HERE, f"FEAT_REF={REF_SRC}", "cuda"], capture_output=True,
