@@ -220,7 +220,12 @@ typedef struct
                            of 32 up to 512; 0 = picked per level by the autotuner at creation */
   int tail_rows;        /* levels (below the finest) with at most this many rows, down to the
                            coarsest, run in one single-block kernel per visit of the cycle (a
-                           V-cycle bottom, or an F/W sub-cycle with its peak smoothing); 0 = off */
+                           V-cycle bottom, or an F/W sub-cycle with its peak smoothing); 0 = off.
+                           With tail_rows, cluster_rows, fused, streamed, tma_rows and tma_window at
+                           their defaults a V-cycle with Jacobi smoothing and the fixed coarse-grid
+                           correction takes neither: its levels from the finest that fits the shared
+                           memory of 16 SMs run in one kernel on a cluster of 16 thread blocks, and
+                           where all levels fit the whole solve does */
   int tma_rows;         /* levels with at least this many rows use the TMA-staged persistent
                            passes (bulk copies into shared memory); 0 = off */
   int cluster_rows;     /* levels (below the finest) with at most this many rows, down to the
