@@ -8,11 +8,12 @@
 // (K/32 per lane): the row's entries are read once, coalesced, and broadcast by shuffles, and every
 // gather of x[col][0..K) is one coalesced K*sizeof(S) access -- the matrix traffic is shared by all
 // right-hand sides (the reference's multi-vector CSR kernel, apply.cu:109-135, covers K <= 3).
-// With the configuration's `diagonal` set, system matrices of lexicographically numbered Q1 grids
-// run in a stencil form instead: values by diagonal, one warp per strip of consecutive rows, each x
-// row gathered once for all the strip's rows it enters (strip_rows).  Rows are summed in stored entry order without FMA, per right-hand
-// side, as in the single-RHS kernels, in both forms.  Dot products and norms are reduced per block and then with FP64 atomics (their
-// summation order is not fixed; results agree with the single-RHS path to rounding).
+// System matrices of lexicographically numbered Q1 grids with enough rows to fill the SMs (with the
+// configuration's `diagonal` set: of any size) run in a stencil form instead: values by diagonal, one
+// warp per strip of consecutive rows, each x row gathered once for all the strip's rows it enters
+// (strip_rows).  Rows are summed in stored entry order without FMA, per right-hand side, as in the
+// single-RHS kernels, in both forms.  Dot products and norms are reduced per block and then with FP64
+// atomics (their summation order is not fixed; results agree with the single-RHS path to rounding).
 #include "fb_common.cuh"
 #include "fb_setup.h"
 
@@ -27,9 +28,33 @@ namespace fb
 {
 namespace mr
 {
-  constexpr int MNT = 256;               // threads per block
-  constexpr int MW = MNT / 32;            // warps (rows in flight) per block
+  // Threads per block.  Passes over a matrix: every block takes one contiguous range of rows, its warps
+  // interleaved, so the rows in flight on an SM lie together and find each other's x rows in L1; large
+  // levels run one block of 1,024 threads per SM, levels with fewer rows than fill those blocks of 256
+  // threads on as many SMs as there are.  Passes without a matrix run blocks of 256 (64 right-hand
+  // sides, 274,625 rows: p = z + beta p 64 us against 69 in blocks of 1,024).
+  constexpr int MNT = 256, MNT_BIG = 1024;
+  constexpr int MW = MNT / 32;
+  constexpr int MW_MAX = MNT_BIG / 32;
   constexpr int KMAX = 64;
+
+  // this block's rows (or strips) of n
+  struct Range
+  {
+    uint32_t first, end;
+    __device__ explicit Range(uint32_t n)
+    {
+      const uint32_t per = n / gridDim.x, rem = n % gridDim.x;
+      first = blockIdx.x * per + min(blockIdx.x, rem);
+      end = first + per + (blockIdx.x < rem ? 1u : 0u);
+    }
+  };
+  __device__ __forceinline__ uint32_t warp_id() { return threadIdx.x >> 5; }
+  __device__ __forceinline__ uint32_t warps() { return blockDim.x >> 5; }
+
+  // 64 right-hand sides in FP64: an x row is 512 bytes and the x rows around an SM's rows outgrow its
+  // L1, so the rows are swept twice, 32 right-hand sides each time
+  template<typename S, int R> struct Half { static constexpr bool value = sizeof(S) == 8 && R == 2; };
 
   // A matrix in CSR form and, for a system matrix whose stored rows all share one pattern of 9 or
   // 27 column offsets made of triplets (o-1, o, o+1) -- the Q1 stencil of a lexicographically
@@ -50,8 +75,10 @@ namespace mr
   };
 
   // rows per warp in the stencil form: the strip's rows share their x gathers (M + 2 row loads per
-  // triplet for M rows instead of 3 M); 4 for FP64 values to bound the registers
-  template<typename V> struct StripRows { static constexpr int value = sizeof(V) == 8 ? 4 : 8; };
+  // triplet for M rows instead of 3 M).  Latency bounds the form, not the gathers: 8 rows per warp hold
+  // twice the registers, so half the warps are resident (FP32, 64 right-hand sides, 274,625 rows, a
+  // defect pass 115 us with 4 rows in 1,024 threads, 138 us with 8 in 512)
+  constexpr int STRIP = 4;
 
   struct MScal
   {
@@ -103,6 +130,46 @@ namespace mr
     }
   }
 
+  // streaming accesses of the row-wise vectors (read or written once per pass: kept out of the way of
+  // the x rows in L1), in one access where the width allows
+  template<typename S, int R>
+  __device__ __forceinline__ void ld_vec(const S* p, S (&v)[R])
+  {
+    if constexpr(R == 2 && sizeof(S) == 4)
+    {
+      const float2 t = __ldcs(reinterpret_cast<const float2*>(p));
+      v[0] = S(t.x);
+      v[1] = S(t.y);
+    }
+    else if constexpr(R == 2)
+    {
+      const double2 t = __ldcs(reinterpret_cast<const double2*>(p));
+      v[0] = S(t.x);
+      v[1] = S(t.y);
+    }
+    else
+      v[0] = __ldcs(p);
+  }
+  template<typename S, int R>
+  __device__ __forceinline__ void st_vec(S* p, const S (&v)[R])
+  {
+    if constexpr(R == 2 && sizeof(S) == 4)
+      *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
+    else if constexpr(R == 2)
+      *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
+    else
+      *p = v[0];
+  }
+
+  // part[k] += v with k known only by its range (a select each: the array stays in registers)
+  template<int R>
+  __device__ __forceinline__ void sum_to(double (&part)[R], int k, double v)
+  {
+    #pragma unroll
+    for(int r = 0; r < R; ++r)
+      part[r] += k == r ? v : 0.0;
+  }
+
   template<typename S> __device__ __forceinline__ double epsq();
   template<> __device__ __forceinline__ double epsq<double>() { return EPS64 * EPS64; }
   template<> __device__ __forceinline__ double epsq<float>() { return double(EPS32) * double(EPS32); }
@@ -111,9 +178,9 @@ namespace mr
     return (!isfinite(nrm) || nrm <= epsq<S>()) ? 1 : 0;
   }
 
-  // sum[r] = (A x)[row][lane*R + r], entries in stored order
-  template<typename V, typename S, int R>
-  __device__ __forceinline__ void mrow(const MCsr<V>& M, uint32_t row, const S* __restrict__ x,
+  // sum[r] = (A x)[row][rhs0 + r] (K right-hand sides in all), entries in stored order
+  template<typename V, typename S, int R, int K>
+  __device__ __forceinline__ void mrow(const MCsr<V>& M, uint32_t row, const S* __restrict__ x, int rhs0,
     typename ValueTraits<V>::acc (&sum)[R])
   {
     typedef typename ValueTraits<V>::acc A;
@@ -138,7 +205,7 @@ namespace mr
       {
         const A vk = A(shfl_v(v, int(k)));
         const uint32_t ck = __shfl_sync(0xffffffffu, c, int(k));
-        const S* xr = x + size_t(ck) * (32 * R) + lane * R;
+        const S* xr = x + size_t(ck) * K + rhs0;
         S xv[R];
         ldg_row<S, R>(xr, xv);
         #pragma unroll
@@ -179,17 +246,56 @@ namespace mr
   // to three) rows whose entry it is.  Row m receives its entries in ascending column order
   // (triplets in order, then o-1, o, o+1), which is the stored CSR order, so every row sum equals
   // mrow's bit for bit.  x rows outside [0, rows) are read only by rows stored empty (their values
-  // are zero); they are not loaded.  epi(row, sum) runs for every row < rows.
-  template<typename V, typename S, int R, int G, class Epi>
-  __device__ __forceinline__ void strip_rows(const MCsr<V>& A, const S* __restrict__ x, Epi& epi)
+  // are zero); they are not loaded (INSIDE: there are none).
+  template<typename V, typename S, int R, int K, int G, bool INSIDE, int M>
+  __device__ __forceinline__ void strip_sums(const MCsr<V>& A, const S* __restrict__ x, int j0, uint32_t r0,
+    typename ValueTraits<V>::acc (&sum)[M][R])
   {
     typedef typename ValueTraits<V>::acc Ac;
-    constexpr int M = StripRows<V>::value;
-    constexpr int K = 32 * R;
-    const int lane = threadIdx.x & 31;
+    #pragma unroll
+    for(int g = 0; g < G; ++g)
+    {
+      V v[3][M];
+      #pragma unroll
+      for(int dx = 0; dx < 3; ++dx)
+        ldg_diag<M>(A.dval + size_t(3 * g + dx) * A.dn + r0, v[dx]);
+      const int64_t base = int64_t(r0) - 1 + A.goff[g];
+      const S* xg = x + base * K + j0;
+      #pragma unroll
+      for(int t = 0; t < M + 2; ++t)
+      {
+        S xv[R];
+        if(INSIDE || (base + t >= 0 && base + t < int64_t(A.rows)))
+          ldg_row<S, R>(xg + t * K, xv);
+        else
+        {
+          #pragma unroll
+          for(int r = 0; r < R; ++r)
+            xv[r] = S(0);
+        }
+        #pragma unroll
+        for(int m = t - 2; m <= t; ++m)
+        {
+          if(m < 0 || m >= M)
+            continue;
+          const Ac vk = Ac(v[t - m][m]);
+          #pragma unroll
+          for(int r = 0; r < R; ++r)
+            sum[m][r] = add(sum[m][r], mul(vk, Ac(xv[r])));
+        }
+      }
+    }
+  }
+
+  // epi(row, sum) for every row < rows
+  template<typename V, typename S, int R, int K, int G, class Epi>
+  __device__ __forceinline__ void strip_rows(const MCsr<V>& A, const S* __restrict__ x, int j0, Epi& epi)
+  {
+    typedef typename ValueTraits<V>::acc Ac;
+    constexpr int M = STRIP;
     const uint32_t n = A.rows;
-    const uint32_t nstrips = (n + M - 1) / M;
-    for(uint32_t st = blockIdx.x * MW + (threadIdx.x >> 5); st < nstrips; st += gridDim.x * MW)
+    const Range rg((n + M - 1) / M);
+    for(uint32_t st = rg.first + warp_id(); st < rg.end; st += warps())
     {
       const uint32_t r0 = st * M;
       Ac sum[M][R];
@@ -198,39 +304,10 @@ namespace mr
         #pragma unroll
         for(int r = 0; r < R; ++r)
           sum[m][r] = Ac(0);
-      #pragma unroll
-      for(int g = 0; g < G; ++g)
-      {
-        V v[3][M];
-        #pragma unroll
-        for(int dx = 0; dx < 3; ++dx)
-          ldg_diag<M>(A.dval + size_t(3 * g + dx) * A.dn + r0, v[dx]);
-        const int64_t base = int64_t(r0) - 1 + A.goff[g];
-        #pragma unroll
-        for(int t = 0; t < M + 2; ++t)
-        {
-          const int64_t xr = base + t;
-          S xv[R];
-          if(xr >= 0 && xr < int64_t(n))
-            ldg_row<S, R>(x + size_t(xr) * K + lane * R, xv);
-          else
-          {
-            #pragma unroll
-            for(int r = 0; r < R; ++r)
-              xv[r] = S(0);
-          }
-          #pragma unroll
-          for(int m = t - 2; m <= t; ++m)
-          {
-            if(m < 0 || m >= M)
-              continue;
-            const Ac vk = Ac(v[t - m][m]);
-            #pragma unroll
-            for(int r = 0; r < R; ++r)
-              sum[m][r] = add(sum[m][r], mul(vk, Ac(xv[r])));
-          }
-        }
-      }
+      if(int64_t(r0) - 1 + A.goff[0] >= 0 && int64_t(r0) + M + A.goff[G - 1] < int64_t(n))
+        strip_sums<V, S, R, K, G, true, M>(A, x, j0, r0, sum);
+      else
+        strip_sums<V, S, R, K, G, false, M>(A, x, j0, r0, sum);
       #pragma unroll
       for(int m = 0; m < M; ++m)
         if(r0 + uint32_t(m) < n)
@@ -238,42 +315,56 @@ namespace mr
     }
   }
 
-  // epi(row, sum) for every row of A with sum = (A x)[row]: in the stencil form with G = 9 or 3
-  // triplets per row, in the CSR form for G = 0.  The form is a template parameter of every matrix
-  // pass, so the CSR instances keep the registers (and the resident warps) of the row kernel.
+  // epi(row, j0, q, sum) for every row of A, with sum[r] = (A x)[row][j0 + r] and q the first of the
+  // thread's partial sums they go to: in the stencil form with G = 9 or 3 triplets per row, in the CSR
+  // form for G = 0.  The form is a template parameter of every matrix pass, so the CSR instances keep
+  // the registers (and the resident warps) of the row kernel.
   template<typename V, typename S, int R, int G, class Epi>
   __device__ __forceinline__ void for_rows(const MCsr<V>& A, const S* __restrict__ x, Epi epi)
   {
     typedef typename ValueTraits<V>::acc Ac;
-    if constexpr(G > 0)
-      strip_rows<V, S, R, G>(A, x, epi);
-    else
-      for(uint32_t row = blockIdx.x * MW + (threadIdx.x >> 5); row < A.rows; row += gridDim.x * MW)
+    constexpr int K = 32 * R;
+    constexpr bool H = Half<S, R>::value;
+    constexpr int RR = H ? 1 : R;
+    const int lane = threadIdx.x & 31;
+    #pragma unroll 1
+    for(int h = 0; h < (H ? 2 : 1); ++h)
+    {
+      const int j0 = H ? 32 * h + lane : lane * R;
+      auto one = [&](uint32_t row, const Ac (&sum)[RR]) { epi(row, j0, h, sum); };
+      if constexpr(G > 0)
+        strip_rows<V, S, RR, K, G>(A, x, j0, one);
+      else
       {
-        Ac sum[R];
-        mrow<V, S, R>(A, row, x, sum);
-        epi(row, sum);
+        const Range rg(A.rows);
+        for(uint32_t row = rg.first + warp_id(); row < rg.end; row += warps())
+        {
+          Ac sum[RR];
+          mrow<V, S, RR, K>(A, row, x, j0, sum);
+          one(row, sum);
+        }
       }
+    }
   }
 
   // block partials per right-hand side (smem), atomically added to sc->acc; the last block calls
-  // fin(j, total) for every j < K and clears the accumulators.  Returns true in the last block.
-  template<int R, class Fin>
+  // fin(j, total) for every j < K and clears the accumulators.  part[r] belongs to right-hand side
+  // lane R + r, or with H (Half) to 32 r + lane.
+  template<int R, bool H = false, class Fin>
   __device__ __forceinline__ void reduce_per_rhs(const double (&part)[R], MScal* sc, Fin fin)
   {
     constexpr int K = 32 * R;
-    __shared__ double red[MW][K];
+    __shared__ double red[MW_MAX][K];
     __shared__ bool last;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     #pragma unroll
     for(int r = 0; r < R; ++r)
-      red[warp][lane * R + r] = part[r];
+      red[warp][H ? 32 * r + lane : lane * R + r] = part[r];
     __syncthreads();
     if(threadIdx.x < K)
     {
       double s = 0.0;
-      #pragma unroll
-      for(int w = 0; w < MW; ++w)
+      for(int w = 0; w < nw; ++w)
         s += red[w][threadIdx.x];
       atomicAdd(&sc->acc[threadIdx.x], s);
     }
@@ -296,10 +387,11 @@ namespace mr
   }
 
 #define MR_ROWS(n) \
-  for(uint32_t row = blockIdx.x * MW + (threadIdx.x >> 5); row < (n); row += gridDim.x * MW)
+  const Range rg_(n); \
+  for(uint32_t row = rg_.first + warp_id(); row < rg_.end; row += warps())
 
   template<typename V, typename S, int R, int G>
-  __global__ void __launch_bounds__(MNT) km_smooth(MCsr<V> A, const S* __restrict__ b, const S* __restrict__ x,
+  __global__ void __launch_bounds__(MNT_BIG, 1) km_smooth(MCsr<V> A, const S* __restrict__ b, const S* __restrict__ x,
     S* __restrict__ xo, const S* __restrict__ dinv, const uint8_t* __restrict__ dm, const int* __restrict__ skip,
     const MScal* __restrict__ sc)
   {
@@ -307,50 +399,50 @@ namespace mr
     constexpr int K = 32 * R;
     if(closed(sc))
       return;
-    const int lane = threadIdx.x & 31;
-    for_rows<V, S, R, G>(A, x, [&](uint32_t row, const Ac (&sum)[R])
+    constexpr int RR = Half<S, R>::value ? 1 : R;
+    for_rows<V, S, R, G>(A, x, [&](uint32_t row, int j0, int, const Ac (&sum)[RR])
     {
       const bool d = __ldg(dm + row) != 0;
       const Ac di = Ac(__ldg(dinv + row));
+      const size_t e = size_t(row) * K + j0;
+      S bv[RR], xv[RR], out[RR];
+      ld_vec<S, RR>(b + e, bv);
+      ldg_row<S, RR>(x + e, xv);
       #pragma unroll
-      for(int r = 0; r < R; ++r)
+      for(int r = 0; r < RR; ++r)
       {
-        const size_t e = size_t(row) * K + lane * R + r;
-        S out = S(0);
-        if(!skip[lane * R + r])
-        {
-          const Ac d1 = d ? Ac(0) : sub(Ac(b[e]), sum[r]);
-          const Ac c = d ? Ac(0) : mul(di, d1);
-          out = S(add(Ac(x[e]), c));
-        }
-        xo[e] = out;
+        const Ac d1 = d ? Ac(0) : sub(Ac(bv[r]), sum[r]);
+        const Ac c = d ? Ac(0) : mul(di, d1);
+        out[r] = skip[j0 + r] ? S(0) : S(add(Ac(xv[r]), c));
       }
+      st_vec<S, RR>(xo + e, out);
     });
   }
 
   template<typename V, typename S, int R, int G>
-  __global__ void __launch_bounds__(MNT) km_defect(MCsr<V> A, const S* __restrict__ b, const S* __restrict__ x,
+  __global__ void __launch_bounds__(MNT_BIG, 1) km_defect(MCsr<V> A, const S* __restrict__ b, const S* __restrict__ x,
     S* __restrict__ dv, const uint8_t* __restrict__ dm, const MScal* __restrict__ sc)
   {
     typedef typename ValueTraits<V>::acc Ac;
     constexpr int K = 32 * R;
     if(closed(sc))
       return;
-    const int lane = threadIdx.x & 31;
-    for_rows<V, S, R, G>(A, x, [&](uint32_t row, const Ac (&sum)[R])
+    constexpr int RR = Half<S, R>::value ? 1 : R;
+    for_rows<V, S, R, G>(A, x, [&](uint32_t row, int j0, int, const Ac (&sum)[RR])
     {
       const bool d = __ldg(dm + row) != 0;
+      const size_t e = size_t(row) * K + j0;
+      S bv[RR], out[RR];
+      ld_vec<S, RR>(b + e, bv);
       #pragma unroll
-      for(int r = 0; r < R; ++r)
-      {
-        const size_t e = size_t(row) * K + lane * R + r;
-        dv[e] = d ? S(0) : S(sub(Ac(b[e]), sum[r]));
-      }
+      for(int r = 0; r < RR; ++r)
+        out[r] = d ? S(0) : S(sub(Ac(bv[r]), sum[r]));
+      st_vec<S, RR>(dv + e, out);
     });
   }
 
   template<typename V, typename S, int R>
-  __global__ void __launch_bounds__(MNT) km_restrict(MCsr<V> Rm, const S* __restrict__ dv, S* __restrict__ bc,
+  __global__ void __launch_bounds__(MNT_BIG, 1) km_restrict(MCsr<V> Rm, const S* __restrict__ dv, S* __restrict__ bc,
     S* __restrict__ xc, const S* __restrict__ dinvc, const uint8_t* __restrict__ dmc, int* __restrict__ skipc,
     MScal* __restrict__ sc)
   {
@@ -366,21 +458,22 @@ namespace mr
     MR_ROWS(Rm.rows)
     {
       Ac sum[R];
-      mrow<V, S, R>(Rm, row, dv, sum);
+      mrow<V, S, R, K>(Rm, row, dv, lane * R, sum);
       const bool d = __ldg(dmc + row) != 0;
+      const size_t e = size_t(row) * K + lane * R;
+      S bo[R], xo[R];
       #pragma unroll
       for(int r = 0; r < R; ++r)
       {
-        const size_t e = size_t(row) * K + lane * R + r;
         const Ac v = d ? Ac(0) : add(sum[r], Ac(0));
-        bc[e] = S(v);
-        if(xc)
-        {
-          const Ac c = d ? Ac(0) : mul(Ac(__ldg(dinvc + row)), v);
-          xc[e] = S(add(Ac(0), c));
-        }
+        bo[r] = S(v);
+        const Ac c = d || !xc ? Ac(0) : mul(Ac(__ldg(dinvc + row)), v);
+        xo[r] = S(add(Ac(0), c));
         part[r] += double(v) * double(v);
       }
+      st_vec<S, R>(bc + e, bo);
+      if(xc)
+        st_vec<S, R>(xc + e, xo);
     }
     if(!xc)
       return;
@@ -408,7 +501,7 @@ namespace mr
   }
 
   template<typename V, typename S, int R>
-  __global__ void __launch_bounds__(MNT) km_prolong(MCsr<V> P, const S* __restrict__ xc, S* __restrict__ x,
+  __global__ void __launch_bounds__(MNT_BIG, 1) km_prolong(MCsr<V> P, const S* __restrict__ xc, S* __restrict__ x,
     const uint8_t* __restrict__ dm, const MScal* __restrict__ sc)
   {
     typedef typename ValueTraits<V>::acc Ac;
@@ -419,20 +512,23 @@ namespace mr
     MR_ROWS(P.rows)
     {
       Ac sum[R];
-      mrow<V, S, R>(P, row, xc, sum);
+      S xv[R];
+      const size_t e = size_t(row) * K + lane * R;
+      ld_vec<S, R>(x + e, xv);
+      mrow<V, S, R, K>(P, row, xc, lane * R, sum);
       const bool d = __ldg(dm + row) != 0;
       #pragma unroll
       for(int r = 0; r < R; ++r)
       {
-        const size_t e = size_t(row) * K + lane * R + r;
         const Ac c = d ? Ac(0) : add(sum[r], Ac(0));
-        x[e] = S(add(Ac(x[e]), c));
+        xv[r] = S(add(Ac(xv[r]), c));
       }
+      st_vec<S, R>(x + e, xv);
     }
   }
 
   template<typename V, typename S, int R, int G>
-  __global__ void __launch_bounds__(MNT) km_post1(MCsr<V> A, const S* __restrict__ b, const S* __restrict__ x,
+  __global__ void __launch_bounds__(MNT_BIG, 1) km_post1(MCsr<V> A, const S* __restrict__ b, const S* __restrict__ x,
     S* __restrict__ dv, S* __restrict__ cv, const S* __restrict__ dinv, const uint8_t* __restrict__ dm,
     int* __restrict__ skip, MScal* __restrict__ sc)
   {
@@ -445,26 +541,31 @@ namespace mr
     #pragma unroll
     for(int r = 0; r < R; ++r)
       part[r] = 0.0;
-    for_rows<V, S, R, G>(A, x, [&](uint32_t row, const Ac (&sum)[R])
+    constexpr int RR = Half<S, R>::value ? 1 : R;
+    for_rows<V, S, R, G>(A, x, [&](uint32_t row, int j0, int q, const Ac (&sum)[RR])
     {
       const bool d = __ldg(dm + row) != 0;
       const Ac di = Ac(__ldg(dinv + row));
+      const size_t e = size_t(row) * K + j0;
+      S bv[RR], dvo[RR], cvo[RR];
+      ld_vec<S, RR>(b + e, bv);
       #pragma unroll
-      for(int r = 0; r < R; ++r)
+      for(int r = 0; r < RR; ++r)
       {
-        const size_t e = size_t(row) * K + lane * R + r;
-        const Ac dd = d ? Ac(0) : sub(Ac(b[e]), sum[r]);
-        dv[e] = S(dd);
+        const Ac dd = d ? Ac(0) : sub(Ac(bv[r]), sum[r]);
+        dvo[r] = S(dd);
         const Ac c = d ? Ac(0) : mul(di, dd);
-        cv[e] = S(add(Ac(0), c));
-        part[r] += double(dd) * double(dd);
+        cvo[r] = S(add(Ac(0), c));
+        sum_to(part, q + r, double(dd) * double(dd));
       }
+      st_vec<S, RR>(dv + e, dvo);
+      st_vec<S, RR>(cv + e, cvo);
     });
-    reduce_per_rhs<R>(part, sc, [&](int j, double tot) { skip[j] = skip_of<S>(sqrt(tot)); });
+    reduce_per_rhs<R, Half<S, R>::value>(part, sc, [&](int j, double tot) { skip[j] = skip_of<S>(sqrt(tot)); });
   }
 
   template<typename V, typename S, int R, bool LAST, bool TOP, int G>
-  __global__ void __launch_bounds__(MNT) km_post2(MCsr<V> A, const S* __restrict__ dv, const S* __restrict__ cv,
+  __global__ void __launch_bounds__(MNT_BIG, 1) km_post2(MCsr<V> A, const S* __restrict__ dv, const S* __restrict__ cv,
     S* __restrict__ co, S* __restrict__ x, double* __restrict__ z, const double* __restrict__ rr,
     const S* __restrict__ dinv, const uint8_t* __restrict__ dm, const int* __restrict__ skip, MScal* __restrict__ sc)
   {
@@ -477,41 +578,49 @@ namespace mr
     #pragma unroll
     for(int r = 0; r < R; ++r)
       part[r] = 0.0;
-    for_rows<V, S, R, G>(A, cv, [&](uint32_t row, const Ac (&sum)[R])
+    constexpr int RR = Half<S, R>::value ? 1 : R;
+    for_rows<V, S, R, G>(A, cv, [&](uint32_t row, int j0, int q, const Ac (&sum)[RR])
     {
       const bool d = __ldg(dm + row) != 0;
       const Ac di = Ac(__ldg(dinv + row));
+      const size_t e = size_t(row) * K + j0;
+      S dvv[RR], cvv[RR], out[RR];
+      double rv[RR], zo[RR];
+      ld_vec<S, RR>(dv + e, dvv);
+      ldg_row<S, RR>(cv + e, cvv);
+      if constexpr(LAST)
+        ld_vec<S, RR>(x + e, out);
+      if constexpr(LAST && TOP)
+        ld_vec<double, RR>(rr + e, rv);
       #pragma unroll
-      for(int r = 0; r < R; ++r)
+      for(int r = 0; r < RR; ++r)
       {
-        const int j = lane * R + r;
-        const size_t e = size_t(row) * K + j;
-        Ac cn = Ac(0);
-        if(!skip[j])
-        {
-          const Ac dk = d ? Ac(0) : sub(Ac(dv[e]), sum[r]);
-          const Ac ck = d ? Ac(0) : mul(di, dk);
-          cn = add(Ac(cv[e]), ck);
-        }
-        if(!LAST)
-          co[e] = S(cn);
+        const Ac dk = d ? Ac(0) : sub(Ac(dvv[r]), sum[r]);
+        const Ac ck = d ? Ac(0) : mul(di, dk);
+        const Ac cn = skip[j0 + r] ? Ac(0) : add(Ac(cvv[r]), ck);
+        if constexpr(!LAST)
+          out[r] = S(cn);
         else
         {
-          const S xn = S(add(Ac(x[e]), cn));
-          if(TOP)
+          const S xn = S(add(Ac(out[r]), cn));
+          out[r] = xn;
+          if constexpr(TOP)
           {
-            const double zi = mul(double(xn), sc->inv_scale[j]);
-            z[e] = zi;
-            part[r] += mul(rr[e], zi);
+            zo[r] = mul(double(xn), sc->inv_scale[j0 + r]);
+            sum_to(part, q + r, mul(rv[r], zo[r]));
           }
-          else
-            x[e] = xn;
         }
       }
+      if constexpr(!LAST)
+        st_vec<S, RR>(co + e, out);
+      else if constexpr(TOP)
+        st_vec<double, RR>(z + e, zo);
+      else
+        st_vec<S, RR>(x + e, out);
     });
     if(!(LAST && TOP))
       return;
-    reduce_per_rhs<R>(part, sc, [&](int j, double tot)
+    reduce_per_rhs<R, Half<S, R>::value>(part, sc, [&](int j, double tot)
     {
       sc->gamma_prev[j] = sc->gamma[j];
       sc->gamma[j] = tot;
@@ -530,7 +639,7 @@ namespace mr
 
   // r = F(rhs - A x), norms -> def_init, status; FP64 mode: sol1 = F(D .* r)
   template<typename S, int R, int G>
-  __global__ void __launch_bounds__(MNT) km_pcg_init(MCsr<double> A, const double* __restrict__ rhs,
+  __global__ void __launch_bounds__(MNT_BIG, 1) km_pcg_init(MCsr<double> A, const double* __restrict__ rhs,
     const double* __restrict__ x, double* __restrict__ rr, const uint8_t* __restrict__ dm, S* __restrict__ x1,
     const S* __restrict__ dinv, int* __restrict__ skip_top, MScal* __restrict__ sc)
   {
@@ -540,24 +649,28 @@ namespace mr
     #pragma unroll
     for(int r = 0; r < R; ++r)
       part[r] = 0.0;
-    for_rows<double, double, R, G>(A, x, [&](uint32_t row, const double (&sum)[R])
+    constexpr int RR = Half<double, R>::value ? 1 : R;
+    for_rows<double, double, R, G>(A, x, [&](uint32_t row, int j0, int q, const double (&sum)[RR])
     {
       const bool d = __ldg(dm + row) != 0;
+      const size_t e = size_t(row) * K + j0;
+      double bv[RR];
+      S xo[RR];
+      ld_vec<double, RR>(rhs + e, bv);
       #pragma unroll
-      for(int r = 0; r < R; ++r)
+      for(int r = 0; r < RR; ++r)
       {
-        const size_t e = size_t(row) * K + lane * R + r;
-        const double rv = d ? 0.0 : sub(rhs[e], sum[r]);
-        rr[e] = rv;
-        if(x1)
-        {
-          const S c = d ? S(0) : mul(__ldg(dinv + row), S(rv));
-          x1[e] = add(S(0), c);
-        }
-        part[r] += mul(rv, rv);
+        const double rv = d ? 0.0 : sub(bv[r], sum[r]);
+        bv[r] = rv;
+        const S c = d || !x1 ? S(0) : mul(__ldg(dinv + row), S(rv));
+        xo[r] = add(S(0), c);
+        sum_to(part, q + r, mul(rv, rv));
       }
+      st_vec<double, RR>(rr + e, bv);
+      if(x1)
+        st_vec<S, RR>(x1 + e, xo);
     });
-    reduce_per_rhs<R>(part, sc, [&](int j, double tot)
+    reduce_per_rhs<R, Half<double, R>::value>(part, sc, [&](int j, double tot)
     {
       const double d0 = sqrt(tot);
       sc->def_init[j] = d0;
@@ -596,7 +709,7 @@ namespace mr
 
   // FP32 modes: b = S(r * scale_j), sol1 = F(D .* b), ||b|| -> skip flags of the top level
   template<typename S, int R>
-  __global__ void __launch_bounds__(MNT) km_prep(const double* __restrict__ rr, S* __restrict__ bt,
+  __global__ void __launch_bounds__(MNT_BIG, 1) km_prep(const double* __restrict__ rr, S* __restrict__ bt,
     S* __restrict__ x1, const S* __restrict__ dinv, const uint8_t* __restrict__ dm, int* __restrict__ skip_top,
     uint32_t n, MScal* __restrict__ sc)
   {
@@ -614,16 +727,20 @@ namespace mr
     MR_ROWS(n)
     {
       const bool d = __ldg(dm + row) != 0;
+      const size_t e = size_t(row) * K + lane * R;
+      double rv[R];
+      S bo[R], xo[R];
+      ld_vec<double, R>(rr + e, rv);
       #pragma unroll
       for(int r = 0; r < R; ++r)
       {
-        const size_t e = size_t(row) * K + lane * R + r;
-        const S b = S(mul(rr[e], scale[r]));
-        bt[e] = b;
-        const S c = d ? S(0) : mul(__ldg(dinv + row), b);
-        x1[e] = add(S(0), c);
-        part[r] += double(b) * double(b);
+        bo[r] = S(mul(rv[r], scale[r]));
+        const S c = d ? S(0) : mul(__ldg(dinv + row), bo[r]);
+        xo[r] = add(S(0), c);
+        part[r] += double(bo[r]) * double(bo[r]);
       }
+      st_vec<S, R>(bt + e, bo);
+      st_vec<S, R>(x1 + e, xo);
     }
     reduce_per_rhs<R>(part, sc, [&](int j, double tot)
     {
@@ -636,7 +753,7 @@ namespace mr
 
   // q = F(A p), q.p -> alpha
   template<int R, int G>
-  __global__ void __launch_bounds__(MNT) km_pcg_q(MCsr<double> A, const double* __restrict__ p, double* __restrict__ q,
+  __global__ void __launch_bounds__(MNT_BIG, 1) km_pcg_q(MCsr<double> A, const double* __restrict__ p, double* __restrict__ q,
     const uint8_t* __restrict__ dm, MScal* __restrict__ sc)
   {
     constexpr int K = 32 * R;
@@ -647,25 +764,28 @@ namespace mr
     #pragma unroll
     for(int r = 0; r < R; ++r)
       part[r] = 0.0;
-    for_rows<double, double, R, G>(A, p, [&](uint32_t row, const double (&sum)[R])
+    constexpr int RR = Half<double, R>::value ? 1 : R;
+    for_rows<double, double, R, G>(A, p, [&](uint32_t row, int j0, int qi, const double (&sum)[RR])
     {
       const bool d = __ldg(dm + row) != 0;
+      const size_t e = size_t(row) * K + j0;
+      double pv[RR], qo[RR];
+      ldg_row<double, RR>(p + e, pv);
       #pragma unroll
-      for(int r = 0; r < R; ++r)
+      for(int r = 0; r < RR; ++r)
       {
-        const size_t e = size_t(row) * K + lane * R + r;
-        const double qv = d ? 0.0 : add(sum[r], 0.0);
-        q[e] = qv;
-        part[r] += mul(qv, p[e]);
+        qo[r] = d ? 0.0 : add(sum[r], 0.0);
+        sum_to(part, qi + r, mul(qo[r], pv[r]));
       }
+      st_vec<double, RR>(q + e, qo);
     });
-    reduce_per_rhs<R>(part, sc, [&](int j, double tot) { sc->alpha[j] = sc->gamma[j] / tot; });
+    reduce_per_rhs<R, Half<double, R>::value>(part, sc, [&](int j, double tot) { sc->alpha[j] = sc->gamma[j] / tot; });
   }
 
   // per right-hand side still in progress: x += alpha p, r -= alpha q; ||r||, stopping test; the
   // next V-cycle input (FP64: sol1 = F(D .* r); FP32: b = S(r * scale), sol1 = F(D .* b))
   template<typename S, int R, bool CONVERT>
-  __global__ void __launch_bounds__(MNT) km_pcg_x(double* __restrict__ x, double* __restrict__ rr,
+  __global__ void __launch_bounds__(MNT_BIG, 1) km_pcg_x(double* __restrict__ x, double* __restrict__ rr,
     const double* __restrict__ p, const double* __restrict__ q, const uint8_t* __restrict__ dm, S* __restrict__ bt,
     S* __restrict__ x1, const S* __restrict__ dinv, int* __restrict__ skip_top, double* __restrict__ hist,
     uint32_t n, int hist_stride, MScal* __restrict__ sc)
@@ -688,24 +808,30 @@ namespace mr
     MR_ROWS(n)
     {
       const bool d = __ldg(dm + row) != 0;
+      const S di = __ldg(dinv + row);
+      const size_t e = size_t(row) * K + lane * R;
+      double xv[R], rv[R], pv[R], qv[R];
+      S bo[R], xo[R];
+      ld_vec<double, R>(x + e, xv);
+      ld_vec<double, R>(rr + e, rv);
+      ld_vec<double, R>(p + e, pv);
+      ld_vec<double, R>(q + e, qv);
       #pragma unroll
       for(int r = 0; r < R; ++r)
       {
-        const size_t e = size_t(row) * K + lane * R + r;
-        double rv = rr[e];
-        if(act[r])
-        {
-          x[e] = add(x[e], mul(alpha[r], p[e]));
-          rv = add(rv, mul(-alpha[r], q[e]));
-          rr[e] = rv;
-        }
-        const S b = S(mul(rv, scale[r]));
-        if(CONVERT)
-          bt[e] = b;
-        const S c = d ? S(0) : mul(__ldg(dinv + row), b);
-        x1[e] = add(S(0), c);
-        part[r] += mul(rv, rv);
+        // a finished right-hand side keeps its x and r
+        xv[r] = act[r] ? add(xv[r], mul(alpha[r], pv[r])) : xv[r];
+        rv[r] = act[r] ? add(rv[r], mul(-alpha[r], qv[r])) : rv[r];
+        bo[r] = S(mul(rv[r], scale[r]));
+        const S c = d ? S(0) : mul(di, bo[r]);
+        xo[r] = add(S(0), c);
+        part[r] += mul(rv[r], rv[r]);
       }
+      st_vec<double, R>(x + e, xv);
+      st_vec<double, R>(rr + e, rv);
+      if(CONVERT)
+        st_vec<S, R>(bt + e, bo);
+      st_vec<S, R>(x1 + e, xo);
     }
     reduce_per_rhs<R>(part, sc, [&](int j, double tot)
     {
@@ -736,7 +862,7 @@ namespace mr
   }
 
   template<int R>
-  __global__ void __launch_bounds__(MNT) km_pcg_p(double* __restrict__ p, const double* __restrict__ z, uint32_t n,
+  __global__ void __launch_bounds__(MNT_BIG, 1) km_pcg_p(double* __restrict__ p, const double* __restrict__ z, uint32_t n,
     int first, const MScal* __restrict__ sc)
   {
     constexpr int K = 32 * R;
@@ -745,13 +871,15 @@ namespace mr
     const int lane = threadIdx.x & 31;
     MR_ROWS(n)
     {
+      const size_t e = size_t(row) * K + lane * R;
+      double zv[R], pv[R];
+      ld_vec<double, R>(z + e, zv);
+      if(!first)
+        ld_vec<double, R>(p + e, pv);
       #pragma unroll
       for(int r = 0; r < R; ++r)
-      {
-        const int j = lane * R + r;
-        const size_t e = size_t(row) * K + j;
-        p[e] = first ? z[e] : add(mul(p[e], sc->beta[j]), z[e]);
-      }
+        pv[r] = first ? zv[r] : add(mul(pv[r], sc->beta[lane * R + r]), zv[r]);
+      st_vec<double, R>(p + e, pv);
     }
   }
 
@@ -768,6 +896,18 @@ namespace mr
     const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if(i < size_t(n) * K)
       out[size_t(perm[i / K]) * K + i % K] = in[i];
+  }
+  // the values of the stencil form (zero-filled before) from the CSR rows
+  template<typename V>
+  __global__ void km_stencil_values(const uint32_t* __restrict__ rp, const V* __restrict__ val, uint32_t rows,
+    V* __restrict__ dval, uint32_t dn)
+  {
+    const uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
+    if(row >= rows)
+      return;
+    const uint32_t j0 = rp[row], len = rp[row + 1] - j0;
+    for(uint32_t k = 0; k < len; ++k)
+      dval[size_t(k) * dn + row] = val[j0 + k];
   }
   __global__ void km_open(MScal* sc, int K)
   {
@@ -845,7 +985,7 @@ namespace mr
   } while(0)
 
   static fb_status upload_stencil(fb_msolver* s, fb_msolver::Mat& d, const std::vector<uint32_t>& rp,
-    const std::vector<uint32_t>& col, const std::vector<double>& val, int prec, bool use);
+    const std::vector<uint32_t>& col, int prec);
 
   static fb_status upload(fb_msolver* s, fb_msolver::Mat& d, const HostCsr& M, int prec,
     const std::vector<uint8_t>* empty, bool stencil = false)
@@ -882,17 +1022,21 @@ namespace mr
         FB_CUDA(cudaMemcpy(d.val, f.data(), 4 * f.size(), cudaMemcpyHostToDevice));
       }
     }
-    return upload_stencil(s, d, rp, col, val, prec, stencil);
+    return stencil ? upload_stencil(s, d, rp, col, prec) : FB_OK;
   }
 
   // The stencil form of a system matrix (see MCsr): every stored row has the same column offsets,
   // 9 or 27 of them in triplets (o-1, o, o+1) with increasing centres.  Leaves d.nd = 0 when the
-  // pattern does not hold (another numbering, another element) or use is 0.
+  // pattern does not hold (another numbering, another element).
   static fb_status upload_stencil(fb_msolver* s, fb_msolver::Mat& d, const std::vector<uint32_t>& rp,
-    const std::vector<uint32_t>& col, const std::vector<double>& val, int prec, bool use)
+    const std::vector<uint32_t>& col, int prec)
   {
     d.nd = 0;
-    if(!use)
+    // whether a pass runs in this form: every SM has a block of strips to run (18,944 rows on 148 SMs),
+    // or the configuration asks.  Ten iterations, CSR against stencil form: 2D 16,641 rows, 64 right-hand
+    // sides FP64 2,547 against 2,906 us; 3D 4,913 rows, 64 FP32 1,223 against 1,353; above the line 2D
+    // 66,049 rows, 64 FP32 4,377 against 3,832; 3D 35,937 rows, 64 FP64 4,305 against 3,899
+    if(!s->cfg.diagonal && d.rows < s->grid / 8u * uint32_t(MW_MAX * STRIP))
       return FB_OK;
     std::vector<int64_t> off;
     for(uint32_t r = 0; r < d.rows; ++r)
@@ -927,19 +1071,14 @@ namespace mr
       return FB_OK;
     const int nd = int(off.size());
     const uint32_t dn = (d.rows + 7u) & ~7u;
-    std::vector<double> dv(size_t(nd) * dn, 0.0);
-    for(uint32_t r = 0; r < d.rows; ++r)
-      for(uint32_t j = rp[r], k = 0; j < rp[r + 1]; ++j, ++k)
-        dv[size_t(k) * dn + r] = val[j];
     const size_t vb = prec == FB_PREC_F64 ? 8 : 4;
-    MR_TRY(malloc0(s, &d.dval, vb * dv.size()));
+    MR_TRY(malloc0(s, &d.dval, vb * size_t(nd) * dn));
     if(prec == FB_PREC_F64)
-      FB_CUDA(cudaMemcpy(d.dval, dv.data(), 8 * dv.size(), cudaMemcpyHostToDevice));
+      km_stencil_values<double><<<(d.rows + 255) / 256, 256>>>(d.rp, (const double*)d.val, d.rows, (double*)d.dval, dn);
     else
-    {
-      std::vector<float> f(dv.begin(), dv.end());
-      FB_CUDA(cudaMemcpy(d.dval, f.data(), 4 * f.size(), cudaMemcpyHostToDevice));
-    }
+      km_stencil_values<float><<<(d.rows + 255) / 256, 256>>>(d.rp, (const float*)d.val, d.rows, (float*)d.dval, dn);
+    FB_CUDA(cudaGetLastError());
+    FB_CUDA(cudaStreamSynchronize(nullptr));   // (the solves run on another stream)
     d.dn = dn;
     d.nd = nd;
     for(int g = 0; g < nd / 3; ++g)
@@ -965,26 +1104,41 @@ namespace mr
     double bytes = 0;
     static constexpr int K = 32 * R;
 
-    unsigned int g(uint32_t rows) const
+    // grid and block of a pass of one warp per row
+    struct Shape { unsigned int g, t; };
+    Shape shape(uint32_t rows) const
     {
-      return std::max(1u, std::min(s->grid, (rows + MW - 1) / MW));
+      const uint32_t nsm = s->grid / 8u;
+      if(rows >= nsm * uint32_t(2 * MW_MAX))
+        return Shape{nsm, unsigned(MNT_BIG)};
+      return flat(rows);
     }
-    // blocks of a pass over a system matrix: one warp per row, or per strip in the stencil form
-    template<typename W> unsigned int ga(const fb_msolver::Mat& m) const
+    // of a pass without a matrix
+    Shape flat(uint32_t rows) const
     {
-      constexpr uint32_t M = StripRows<W>::value;
-      return g(m.nd ? (m.rows + M - 1) / M : m.rows);
+      return Shape{std::max(1u, std::min(s->grid, (rows + MW - 1) / MW)), unsigned(MNT)};
+    }
+    // of a pass over a system matrix: one warp per row, or per strip in the stencil form
+    template<typename W> Shape ga(const fb_msolver::Mat& m) const
+    {
+      if(!m.nd)
+        return shape(m.rows);
+      constexpr uint32_t M = STRIP;
+      const uint32_t nsm = s->grid / 8u, n = (m.rows + M - 1) / M;
+      if(n >= nsm * uint32_t(MNT_BIG / 32))
+        return Shape{nsm, unsigned(MNT_BIG)};
+      return Shape{std::max(1u, std::min(nsm * 2u, (n + MW - 1) / MW)), unsigned(MNT)};
     }
     // matrix bytes read by one pass, as stored
-    static double mbytes(const fb_msolver::Mat& m, double vsize)
+    template<typename W> double mbytes(const fb_msolver::Mat& m) const
     {
       if(m.nd)
-        return double(m.nd) * m.dn * vsize;
-      return double(m.nnz) * (vsize + 4.0) + double(m.rows + 1) * 4.0;
+        return double(m.nd) * m.dn * sizeof(W);
+      return double(m.nnz) * (sizeof(W) + 4.0) + double(m.rows + 1) * 4.0;
     }
-    double mb(const fb_msolver::Mat& m) const { return mbytes(m, sizeof(V)); }
+    double mb(const fb_msolver::Mat& m) const { return mbytes<V>(m); }
     // f(std::integral_constant<int, G>) with G the stored form of m: 9 or 3 stencil triplets, 0 = CSR
-    template<class F> static void by_form(const fb_msolver::Mat& m, F&& f)
+    template<typename W, class F> void by_form(const fb_msolver::Mat& m, F&& f) const
     {
       if(m.nd == 27)
         f(std::integral_constant<int, 9>());
@@ -1008,8 +1162,8 @@ namespace mr
         for(int k = 1; k < s->cfg.smooth_steps; ++k)
         {
           if(!dry)
-            by_form(f.A, [&](auto gc) {
-              km_smooth<V, S, R, decltype(gc)::value><<<ga<V>(f.A), MNT, 0, st>>>(mv<V>(f.A), (const S*)f.b,
+            by_form<V>(f.A, [&](auto gc) {
+              km_smooth<V, S, R, decltype(gc)::value><<<ga<V>(f.A).g, ga<V>(f.A).t, 0, st>>>(mv<V>(f.A), (const S*)f.b,
                 (const S*)xa, (S*)xb, (const S*)f.dinv, f.dm, f.skip_pre, s->sc);
             });
           ++launches;
@@ -1018,15 +1172,15 @@ namespace mr
         }
         xcur[size_t(l)] = xa;
         if(!dry)
-          by_form(f.A, [&](auto gc) {
-            km_defect<V, S, R, decltype(gc)::value><<<ga<V>(f.A), MNT, 0, st>>>(mv<V>(f.A), (const S*)f.b,
+          by_form<V>(f.A, [&](auto gc) {
+            km_defect<V, S, R, decltype(gc)::value><<<ga<V>(f.A).g, ga<V>(f.A).t, 0, st>>>(mv<V>(f.A), (const S*)f.b,
               (const S*)xa, (S*)f.d, f.dm, s->sc);
           });
         ++launches;
         bytes += mb(f.A) + vb(f.n, 3);
         const bool coarsest = (l + 2 == nl);
         if(!dry)
-          km_restrict<V, S, R><<<g(c.n), MNT, 0, st>>>(mv<V>(f.R), (const S*)f.d, (S*)c.b,
+          km_restrict<V, S, R><<<shape(c.n).g, shape(c.n).t, 0, st>>>(mv<V>(f.R), (const S*)f.d, (S*)c.b,
             coarsest ? (S*)nullptr : (S*)c.x, (const S*)c.dinv, c.dm, c.skip_pre, s->sc);
         ++launches;
         bytes += mb(f.R) + vb(f.n, 1) + vb(c.n, 2);
@@ -1044,10 +1198,10 @@ namespace mr
         fb_msolver::Level& f = s->lv[size_t(l)];
         void* xf = xcur[size_t(l)];
         if(!dry)
-          km_prolong<V, S, R><<<g(f.n), MNT, 0, st>>>(mv<V>(f.P), (const S*)xcur[size_t(l + 1)], (S*)xf, f.dm, s->sc);
+          km_prolong<V, S, R><<<shape(f.n).g, shape(f.n).t, 0, st>>>(mv<V>(f.P), (const S*)xcur[size_t(l + 1)], (S*)xf, f.dm, s->sc);
         if(!dry)
-          by_form(f.A, [&](auto gc) {
-            km_post1<V, S, R, decltype(gc)::value><<<ga<V>(f.A), MNT, 0, st>>>(mv<V>(f.A), (const S*)f.b,
+          by_form<V>(f.A, [&](auto gc) {
+            km_post1<V, S, R, decltype(gc)::value><<<ga<V>(f.A).g, ga<V>(f.A).t, 0, st>>>(mv<V>(f.A), (const S*)f.b,
               (const S*)xf, (S*)f.d, (S*)f.c, (const S*)f.dinv, f.dm, f.skip_post, s->sc);
           });
         launches += 2;
@@ -1059,16 +1213,16 @@ namespace mr
         {
           const bool last = (k == s->cfg.smooth_steps);
           if(!dry)
-            by_form(f.A, [&](auto gc) {
+            by_form<V>(f.A, [&](auto gc) {
               constexpr int G = decltype(gc)::value;
               if(!last)
-                km_post2<V, S, R, false, false, G><<<ga<V>(f.A), MNT, 0, st>>>(mv<V>(f.A), (const S*)f.d,
+                km_post2<V, S, R, false, false, G><<<ga<V>(f.A).g, ga<V>(f.A).t, 0, st>>>(mv<V>(f.A), (const S*)f.d,
                   (const S*)ca, (S*)cb, (S*)xf, nullptr, nullptr, (const S*)f.dinv, f.dm, f.skip_post, s->sc);
               else if(top)
-                km_post2<V, S, R, true, true, G><<<ga<V>(f.A), MNT, 0, st>>>(mv<V>(f.A), (const S*)f.d,
+                km_post2<V, S, R, true, true, G><<<ga<V>(f.A).g, ga<V>(f.A).t, 0, st>>>(mv<V>(f.A), (const S*)f.d,
                   (const S*)ca, (S*)cb, (S*)xf, s->z, s->r, (const S*)f.dinv, f.dm, f.skip_post, s->sc);
               else
-                km_post2<V, S, R, true, false, G><<<ga<V>(f.A), MNT, 0, st>>>(mv<V>(f.A), (const S*)f.d,
+                km_post2<V, S, R, true, false, G><<<ga<V>(f.A).g, ga<V>(f.A).t, 0, st>>>(mv<V>(f.A), (const S*)f.d,
                   (const S*)ca, (S*)cb, (S*)xf, nullptr, nullptr, (const S*)f.dinv, f.dm, f.skip_post, s->sc);
             });
           ++launches;
@@ -1087,18 +1241,18 @@ namespace mr
       if(!dry)
         km_open<<<1, 32, 0, st>>>(s->sc, K);
       if(!dry)
-        by_form(A64(), [&](auto gc) {
-          km_pcg_init<S, R, decltype(gc)::value><<<ga<double>(A64()), MNT, 0, st>>>(mv<double>(A64()), s->rhs,
+        by_form<double>(A64(), [&](auto gc) {
+          km_pcg_init<S, R, decltype(gc)::value><<<ga<double>(A64()).g, ga<double>(A64()).t, 0, st>>>(mv<double>(A64()), s->rhs,
             s->x, s->r, t.dm, f64 ? (S*)t.x : (S*)nullptr, (const S*)t.dinv, t.skip_pre, s->sc);
         });
       if(!dry)
         km_count_progress<<<1, 64, 0, st>>>(s->sc, K, 0);
       launches += 3;
-      bytes += mbytes(A64(), 8.0) + double(t.n) * K * 8.0 * 3;
+      bytes += mbytes<double>(A64()) + double(t.n) * K * 8.0 * 3;
       if(!f64)
       {
         if(!dry)
-          km_prep<S, R><<<g(t.n), MNT, 0, st>>>(s->r, (S*)t.b, (S*)t.x, (const S*)t.dinv, t.dm, t.skip_pre, t.n, s->sc);
+          km_prep<S, R><<<flat(t.n).g, flat(t.n).t, 0, st>>>(s->r, (S*)t.b, (S*)t.x, (const S*)t.dinv, t.dm, t.skip_pre, t.n, s->sc);
         ++launches;
         bytes += double(t.n) * K * (8.0 + 2 * sizeof(S));
       }
@@ -1110,21 +1264,21 @@ namespace mr
       const bool f64 = s->cfg.precision == FB_PREC_F64;
       if(!dry)
       {
-        km_pcg_p<R><<<g(t.n), MNT, 0, st>>>(s->p, s->z, t.n, first ? 1 : 0, s->sc);
-        by_form(A64(), [&](auto gc) {
-          km_pcg_q<R, decltype(gc)::value><<<ga<double>(A64()), MNT, 0, st>>>(mv<double>(A64()), s->p, s->q, t.dm,
+        km_pcg_p<R><<<flat(t.n).g, flat(t.n).t, 0, st>>>(s->p, s->z, t.n, first ? 1 : 0, s->sc);
+        by_form<double>(A64(), [&](auto gc) {
+          km_pcg_q<R, decltype(gc)::value><<<ga<double>(A64()).g, ga<double>(A64()).t, 0, st>>>(mv<double>(A64()), s->p, s->q, t.dm,
             s->sc);
         });
         if(f64)
-          km_pcg_x<S, R, false><<<g(t.n), MNT, 0, st>>>(s->x, s->r, s->p, s->q, t.dm, (S*)nullptr, (S*)t.x,
+          km_pcg_x<S, R, false><<<flat(t.n).g, flat(t.n).t, 0, st>>>(s->x, s->r, s->p, s->q, t.dm, (S*)nullptr, (S*)t.x,
             (const S*)t.dinv, t.skip_pre, s->hist, t.n, K, s->sc);
         else
-          km_pcg_x<S, R, true><<<g(t.n), MNT, 0, st>>>(s->x, s->r, s->p, s->q, t.dm, (S*)t.b, (S*)t.x,
+          km_pcg_x<S, R, true><<<flat(t.n).g, flat(t.n).t, 0, st>>>(s->x, s->r, s->p, s->q, t.dm, (S*)t.b, (S*)t.x,
             (const S*)t.dinv, t.skip_pre, s->hist, t.n, K, s->sc);
         km_count_progress<<<1, 64, 0, st>>>(s->sc, K, cond);
       }
       launches += 4;
-      bytes += double(t.n) * K * 8.0 * 3 + mbytes(A64(), 8.0) + double(t.n) * K * 8.0 * 3 +
+      bytes += double(t.n) * K * 8.0 * 3 + mbytes<double>(A64()) + double(t.n) * K * 8.0 * 3 +
                double(t.n) * K * (8.0 * 6 + 2 * sizeof(S));
     }
   };
@@ -1310,9 +1464,9 @@ fb_status fb_msolver_create(fb_msolver** out, fb_hierarchy* h, const fb_solver_c
     const std::vector<uint32_t> inv_f = pf.empty() ? std::vector<uint32_t>() : inverse_perm(pf);
     D.n = H.A.rows;
     HostCsr A = permute(H.A, pf, inv_f);
-    MR_TRY(mr::upload(s.get(), D.A, A, prec, &dms[size_t(l)], cfg.diagonal != 0));
+    MR_TRY(mr::upload(s.get(), D.A, A, prec, &dms[size_t(l)], true));
     if(l == 0 && prec != FB_PREC_F64)
-      MR_TRY(mr::upload(s.get(), D.A64, A, FB_PREC_F64, &dms[size_t(l)], cfg.diagonal != 0));
+      MR_TRY(mr::upload(s.get(), D.A64, A, FB_PREC_F64, &dms[size_t(l)], true));
     if(l + 1 < s->nlev)
     {
       const std::vector<uint32_t>& pc = perms[size_t(l + 1)];

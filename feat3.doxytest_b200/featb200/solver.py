@@ -483,10 +483,9 @@ class MultiRhsPCG:
         self.cfg.tol_rel, self.cfg.max_iter = float(tol_rel), int(max_iter)
         self.cfg.precision, self.cfg.ordering = _lib.PREC[precision], _lib.ORDER[ordering]
         self.cfg.use_graph = 1 if use_graph else 0
-        # stencil=True: system matrices with the Q1 stencil pattern in the device numbering run in the
-        # stencil form (strips of rows sharing their gathers; row sums bitwise those of the CSR form).
-        # Off by default: on one B200 it measured no faster than the CSR form (10.29 against 9.95 ms
-        # for 64 solves at 3D L6).
+        # System matrices with the Q1 stencil pattern in the device numbering run in the stencil form
+        # (strips of rows sharing their gathers; row sums bitwise those of the CSR form) where they have
+        # enough rows to fill the SMs; stencil=True: at every size.
         self.cfg.diagonal = 1 if stencil else 0
         if hierarchy._h is None:
             hierarchy.init()

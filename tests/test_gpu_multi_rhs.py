@@ -99,3 +99,32 @@ def test_multi_rhs_stencil_form(featlib, cuda, dim, level, precision):
     else:
         assert err <= 2e-7, err
         assert max(abs(a - b) for a, b in zip(out[True][1], out[False][1])) <= 1
+
+
+# the CSR and the stencil form of the system matrix: levels of 16,641 rows (too few strips to fill the
+# SMs) and of 66,049 and 35,937 (strips of four rows, the last one partial), FP64 with 64 right-hand
+# sides in two sweeps
+@pytest.mark.parametrize("dim,level,K,precision", [(2, 7, 32, "f64"), (2, 8, 64, "f64"), (2, 8, 32, "f32"), (3, 5, 64, "f32")])
+def test_forms_of_large_levels(featlib, cuda, dim, level, K, precision):
+    """Every right-hand side agrees with its own solve (kernel/solver/pcg.hpp:159-286); forced and chosen
+    forms take the same number of iterations."""
+    torch, fb = cuda, featlib
+    from featb200 import assembly as AS
+    levels, b = AS.poisson_hierarchy(level, dim, rhs="gauss", gauss=AS.gauss_params(7, dim))
+    scale = np.random.default_rng(K).uniform(0.5, 2.0, K)
+    rhs = torch.tensor(b[:, None] * scale, device="cuda")
+    one = fb.build_pcg_multigrid(levels, precision=precision)
+    h = fb.build_hierarchy(levels)
+    iters = []
+    for stencil in (False, True):
+        m = fb.MultiRhsPCG(h, K, precision=precision, stencil=stencil)
+        x = torch.zeros_like(rhs)
+        m.solve_device(x, rhs)
+        iters.append(m.iterations())
+        for j in (0, K // 2 - 1, K // 2, K - 1):
+            ref = torch.zeros(b.size, dtype=torch.float64, device="cuda")
+            assert one.correct_device(ref, rhs[:, j].contiguous()) == fb.Status.success == m.statuses()[j]
+            assert iters[-1][j] == one.get_num_iter()
+            # only the order of the PCG's sums differs
+            assert rel_err(x[:, j].cpu().numpy(), ref.cpu().numpy()) <= (1e-12 if precision == "f64" else 1e-9)
+    assert iters[0] == iters[1]
