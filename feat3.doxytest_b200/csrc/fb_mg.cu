@@ -1781,6 +1781,8 @@ struct fb_solver
   cudaGraph_t vgraph = nullptr;
   cudaGraphExec_t vexec = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaEvent_t ev_caller = nullptr;          // orders the solver's stream and the caller's
+  fb::Scalars* hsc = nullptr;               // pinned: the scalars (and the error word) after a solve
   std::vector<fb::DevSor> sor;              // per level (not the coarsest): SOR / SSOR sweep data
   std::vector<fb::CycEv> events;            // one multigrid cycle
   uint8_t* tail_prog = nullptr;             // tail kernel programs: events op << 4 | tail level
@@ -1795,6 +1797,7 @@ struct fb_solver
   double* cred = nullptr; // cluster tail: per-block partial sums (2 * MAX_TAIL * CT_CS)
   cudaError_t launch_err = cudaSuccess;
   int nsm = 148;          // streaming multiprocessors of the device
+  int device = 0;
   int* err = nullptr;     // device error word (bounded waits that expired)
   uint64_t launches_init = 0, launches_body = 0, launches_vcycle = 0;
   double bytes_init = 0, bytes_body = 0;
@@ -3515,6 +3518,8 @@ void fb_solver_destroy(fb_solver* s)
   if(s->graph) cudaGraphDestroy(s->graph);
   if(s->ev0) cudaEventDestroy(s->ev0);
   if(s->ev1) cudaEventDestroy(s->ev1);
+  if(s->ev_caller) cudaEventDestroy(s->ev_caller);
+  if(s->hsc) cudaFreeHost(s->hsc);
   if(s->stream) cudaStreamDestroy(s->stream);
   for(void* p : s->allocs)
     cudaFree(p);
@@ -3667,12 +3672,16 @@ fb_status fb_solver_create(fb_solver** out, fb_hierarchy* h, const fb_solver_con
     FB_CUDA(cudaMemcpy(s->perm0, s->perms[0].data(), sizeof(uint32_t) * n0, cudaMemcpyHostToDevice));
   }
   FB_TRY(dalloc(s.get(), (void**)&s->hist, sizeof(double) * (size_t(cfg.max_iter) + 2)));
-  FB_TRY(dalloc(s.get(), (void**)&s->sc, sizeof(Scalars)));
-  FB_TRY(dalloc(s.get(), (void**)&s->err, sizeof(int)));
+  // the scalars and, behind them, the error word: one copy to the pinned host buffer after a solve
+  FB_TRY(dalloc(s.get(), (void**)&s->sc, sizeof(Scalars) + sizeof(int)));
+  s->err = reinterpret_cast<int*>(s->sc + 1);
+  FB_CUDA(cudaMallocHost((void**)&s->hsc, sizeof(Scalars) + sizeof(int)));
+  FB_CUDA(cudaEventCreateWithFlags(&s->ev_caller, cudaEventDisableTiming));
   {
     int dev = 0;
     FB_CUDA(cudaGetDevice(&dev));
     FB_CUDA(cudaDeviceGetAttribute(&s->nsm, cudaDevAttrMultiProcessorCount, dev));
+    s->device = dev;
   }
   // the fused passes' grids: ceil(W / 16)^2 (up, 16 x 16 fine tiles) and ceil(Wc / 8)^2 (down,
   // 8 x 8 coarse tiles) blocks, each with two partial sums
@@ -3883,18 +3892,19 @@ namespace fb
 
 extern "C" {
 
-static fb_status solve_common(fb_solver* s, fb_solve_info* info)
+// enqueues a solve from x (initial guess, result) and rhs in the device numbering, and the copy of
+// its scalars
+static fb_status solve_enqueue(fb_solver* s, double* x, const double* rhs)
 {
   cudaStream_t st = s->stream;
-  const uint32_t n0 = s->lv[0].n;
   FB_CUDA(cudaEventRecord(s->ev0, st));
   fb_status e = FB_OK;
   if(s->cfg.precision == FB_PREC_F64)
-    e = solve_dispatch<double, double>(s, s->x, s->rhs);
+    e = solve_dispatch<double, double>(s, x, rhs);
   else if(s->cfg.precision == FB_PREC_F32)
-    e = solve_dispatch<float, float>(s, s->x, s->rhs);
+    e = solve_dispatch<float, float>(s, x, rhs);
   else
-    e = solve_dispatch<bf16_t, float>(s, s->x, s->rhs);
+    e = solve_dispatch<bf16_t, float>(s, x, rhs);
   if(e != FB_OK)
     return e;
   if(s->launch_err != cudaSuccess)
@@ -3904,18 +3914,22 @@ static fb_status solve_common(fb_solver* s, fb_solve_info* info)
     return cuda_fail(le, "cluster tail launch");
   }
   FB_CUDA(cudaEventRecord(s->ev1, st));
-  Scalars h;
-  int err = 0;
-  FB_CUDA(cudaMemcpyAsync(&h, s->sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
-  FB_CUDA(cudaMemcpyAsync(&err, s->err, sizeof(int), cudaMemcpyDeviceToHost, st));
+  FB_CUDA(cudaMemcpyAsync(s->hsc, s->sc, sizeof(Scalars) + sizeof(int), cudaMemcpyDeviceToHost, st));
+  return FB_OK;
+}
+
+// waits for the solver's stream and reports the solve
+static fb_status solve_finish(fb_solver* s, fb_solve_info* info)
+{
+  cudaStream_t st = s->stream;
   FB_CUDA(cudaStreamSynchronize(st));
-  if(err)
+  const Scalars& h = *s->hsc;
+  if(*reinterpret_cast<const int*>(s->hsc + 1))
   {
     FB_CUDA(cudaMemsetAsync(s->err, 0, sizeof(int), st));
     set_error("solve: a bounded wait for staged matrix data expired (results invalid)");
     return FB_ERR_CUDA;
   }
-  (void)n0;
   count_launches(s->launches_init + (h.iter > 1 ? uint64_t(h.iter - 1) : 0) * s->launches_body);
   if(info)
   {
@@ -3972,11 +3986,24 @@ fb_status fb_solver_solve(fb_solver* s, double* sol, const double* rhs, fb_solve
   FB_TRY(to_device_order(s, s->rhs, s->tmp_in));
   FB_CUDA(cudaMemcpyAsync(s->tmp_in, sol, 8 * size_t(n), cudaMemcpyHostToDevice, s->stream));
   FB_TRY(to_device_order(s, s->x, s->tmp_in));
-  FB_TRY(solve_common(s, info));
+  FB_TRY(solve_enqueue(s, s->x, s->rhs));
+  FB_TRY(solve_finish(s, info));
   FB_TRY(from_device_order(s, s->tmp_out, s->x));
   FB_CUDA(cudaMemcpyAsync(sol, s->tmp_out, 8 * size_t(n), cudaMemcpyDeviceToHost, s->stream));
   FB_CUDA(cudaStreamSynchronize(s->stream));
   return FB_OK;
+}
+
+// whether a kernel on the solver's device may work on a caller's vector in place
+static bool on_device(const fb_solver* s, const void* p)
+{
+  cudaPointerAttributes a;
+  if((reinterpret_cast<uintptr_t>(p) & 7u) != 0 || cudaPointerGetAttributes(&a, p) != cudaSuccess)
+  {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == s->device;
 }
 
 fb_status fb_solver_solve_device(fb_solver* s, double* sol, const double* rhs, void* stream, fb_solve_info* info)
@@ -3988,20 +4015,35 @@ fb_status fb_solver_solve_device(fb_solver* s, double* sol, const double* rhs, v
   }
   cudaStream_t cs = as_stream(stream);
   // order the solver's private stream after the caller's stream, and the caller's after the solve
-  cudaEvent_t ev;
-  FB_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-  FB_CUDA(cudaEventRecord(ev, cs));
-  FB_CUDA(cudaStreamWaitEvent(s->stream, ev, 0));
-  FB_TRY(to_device_order(s, s->rhs, rhs));
-  FB_TRY(to_device_order(s, s->x, sol));
-  fb_status e = solve_common(s, info);
-  if(e == FB_OK)
-    e = from_device_order(s, sol, s->x);
-  FB_CUDA(cudaEventRecord(ev, s->stream));
-  FB_CUDA(cudaStreamWaitEvent(cs, ev, 0));
-  FB_CUDA(cudaStreamSynchronize(s->stream));
-  cudaEventDestroy(ev);
-  return e;
+  FB_CUDA(cudaEventRecord(s->ev_caller, cs));
+  FB_CUDA(cudaStreamWaitEvent(s->stream, s->ev_caller, 0));
+  // a whole-solve kernel reads rhs and works on x row by row: without a permutation it takes the
+  // caller's buffers, where they are this device's memory and apart from each other (the copies take
+  // any memory and give each its own)
+  const size_t n = s->lv[0].n;
+  const bool direct = s->cl_full.first >= 0 && !s->perm0 && (sol + n <= rhs || rhs + n <= sol) && on_device(s, sol) &&
+                      on_device(s, rhs);
+  fb_status e = FB_OK;
+  if(direct)
+    e = solve_enqueue(s, sol, rhs);
+  else
+  {
+    e = to_device_order(s, s->rhs, rhs);
+    if(e == FB_OK)
+      e = to_device_order(s, s->x, sol);
+    if(e == FB_OK)
+      e = solve_enqueue(s, s->x, s->rhs);
+    if(e == FB_OK)
+      e = from_device_order(s, sol, s->x);
+  }
+  FB_CUDA(cudaEventRecord(s->ev_caller, s->stream));
+  FB_CUDA(cudaStreamWaitEvent(cs, s->ev_caller, 0));
+  if(e != FB_OK)
+  {
+    (void)cudaStreamSynchronize(s->stream);
+    return e;
+  }
+  return solve_finish(s, info);
 }
 
 fb_status fb_solver_vcycle(fb_solver* s, double* cor, const double* def)
