@@ -33,6 +33,7 @@ namespace fb
 namespace bt
 {
   constexpr int BNT = 256;       // block size of the PCG-space kernels (4 resident per SM: at most 64 registers)
+  constexpr int PCGP_ROWS = 4;   // rows per thread of p = z + beta p
   constexpr int BNT_MAX = 512;   // largest block size the autotuner may pick for the V-cycle passes
   constexpr int BW = BNT / 32;
   constexpr int MAXG = 16;
@@ -363,6 +364,9 @@ namespace bt
     finalize_all(sc, fin);
   }
 
+  // The operations' own loads (pre) do not wait for the row's instance and its status: a branch on
+  // them would hold back the gathers behind two more dependent loads (64 instances of 2D levels 5 to 9 on
+  // the level of 1.37 M rows: restriction 60 -> 41 us, last post-smoothing step on 5.46 M rows 71 -> 60).
   // x' = x + F(D F(b - A x)) (smooth_row); skipped -> 0
   template<typename V, typename S>
   struct BOpSmooth
@@ -374,17 +378,14 @@ namespace bt
     __device__ bool closed() const { return bt::closed(sc); }
     __device__ Pre pre(uint32_t i) const
     {
-      Pre p{};
+      Pre p;
       const int j = __ldg(sinst + (i >> 5));
+      p.d = __ldg(dm + i) != 0;
+      p.b = Ac(b[i]);
+      p.x = Ac(x[i]);
+      p.di = Ac(__ldg(dinv + i));
       p.on = active(sc, j);
-      if(p.on)
-      {
-        p.skip = skip[j] != 0;
-        p.d = __ldg(dm + i) != 0;
-        p.b = Ac(b[i]);
-        p.x = Ac(x[i]);
-        p.di = Ac(__ldg(dinv + i));
-      }
+      p.skip = skip[j] != 0;
       return p;
     }
     __device__ double operator()(uint32_t i, Ac sum, const Pre& p) const
@@ -416,13 +417,11 @@ namespace bt
     __device__ bool closed() const { return bt::closed(sc); }
     __device__ Pre pre(uint32_t i) const
     {
-      Pre p{};
-      p.on = active(sc, __ldg(sinst + (i >> 5)));
-      if(p.on)
-      {
-        p.d = __ldg(dm + i) != 0;
-        p.b = Ac(b[i]);
-      }
+      Pre p;
+      const int j = __ldg(sinst + (i >> 5));
+      p.d = __ldg(dm + i) != 0;
+      p.b = Ac(b[i]);
+      p.on = active(sc, j);
       return p;
     }
     __device__ double operator()(uint32_t i, Ac sum, const Pre& p) const
@@ -445,13 +444,11 @@ namespace bt
     __device__ bool closed() const { return bt::closed(sc); }
     __device__ Pre pre(uint32_t i) const
     {
-      Pre p{};
-      p.on = active(sc, __ldg(sinst + (i >> 5)));
-      if(p.on)
-      {
-        p.d = __ldg(dm + i) != 0;
-        p.x = Ac(x[i]);
-      }
+      Pre p;
+      const int j = __ldg(sinst + (i >> 5));
+      p.d = __ldg(dm + i) != 0;
+      p.x = Ac(x[i]);
+      p.on = active(sc, j);
       return p;
     }
     __device__ double operator()(uint32_t i, Ac sum, const Pre& p) const
@@ -478,15 +475,12 @@ namespace bt
     __device__ bool closed() const { return bt::closed(sc); }
     __device__ Pre pre(uint32_t i) const
     {
-      Pre p{};
+      Pre p;
       const int j = __ldg(sinst + (i >> 5));
+      p.d = __ldg(dm + i) != 0;
+      p.b = Ac(b[i]);
+      p.di = Ac(__ldg(dinv + i));
       p.j = active(sc, j) ? j : -1;
-      if(p.j >= 0)
-      {
-        p.d = __ldg(dm + i) != 0;
-        p.b = Ac(b[i]);
-        p.di = Ac(__ldg(dinv + i));
-      }
       return p;
     }
     __device__ void operator()(uint32_t i, Ac sum, const Pre& p, InstSum& acc) const
@@ -527,24 +521,22 @@ namespace bt
     {
       Pre p{};
       const int j = __ldg(sinst + (i >> 5));
+      p.dd = __ldg(dm + i) != 0;
+      p.d = Ac(d[i]);
+      p.c = Ac(c[i]);
+      p.di = Ac(__ldg(dinv + i));
+      if(LAST)
+        p.x = Ac(x[i]);
       p.j = active(sc, j) ? j : -1;
-      if(p.j >= 0)
+      p.skip = skip[j] != 0;
+      if(LAST)
       {
-        p.skip = skip[j] != 0;
-        p.dd = __ldg(dm + i) != 0;
-        p.d = Ac(d[i]);
-        p.c = Ac(c[i]);
-        p.di = Ac(__ldg(dinv + i));
-        if(LAST)
+        p.top = sc.top[j] == g;
+        if(p.top)
         {
-          p.x = Ac(x[i]);
-          p.top = sc.top[j] == g;
-          if(p.top)
-          {
-            p.pr = uint32_t(__ldg(pcg_base + (i >> 5))) + (i & 31u);
-            p.r = r[p.pr];
-            p.inv = sc.inv_scale[j];
-          }
+          p.pr = uint32_t(__ldg(pcg_base + (i >> 5))) + (i & 31u);
+          p.r = r[p.pr];
+          p.inv = sc.inv_scale[j];
         }
       }
       return p;
@@ -615,13 +607,10 @@ namespace bt
     {
       Pre p{};
       const int j = __ldg(sinstc + (i >> 5));
+      p.dc = __ldg(dmc + i) != 0;
+      if(xc)
+        p.di = Ac(__ldg(dinvc + i));
       p.j = (active(sc, j) && sc.top[j] != gc) ? j : -1;
-      if(p.j >= 0)
-      {
-        p.dc = __ldg(dmc + i) != 0;
-        if(xc)
-          p.di = Ac(__ldg(dinvc + i));
-      }
       return p;
     }
     __device__ void operator()(uint32_t i, Ac sum, const Pre& p, InstSum& acc) const
@@ -668,14 +657,11 @@ namespace bt
     __device__ bool closed() const { return bt::closed(sc); }
     __device__ Pre pre(uint32_t i) const
     {
-      Pre r{};
+      Pre r;
       const int j = __ldg(sinst + (i >> 5));
+      r.d = __ldg(dm + i) != 0;
+      r.p = p[i];
       r.j = active(sc, j) ? j : -1;
-      if(r.j >= 0)
-      {
-        r.d = dm[i] != 0;
-        r.p = p[i];
-      }
       return r;
     }
     __device__ void operator()(uint32_t i, double sum, const Pre& pr, InstSum& acc) const
@@ -754,7 +740,47 @@ namespace bt
     }
   };
 
-  // r = F(rhs - A x), ||r|| -> def_init, status
+  // an instance's start from ||r||^2
+  __device__ __forceinline__ void open_instance(const BScal& sc, int j, double tot)
+  {
+    const double d0 = sqrt(tot);
+    sc.def_init[j] = d0;
+    sc.def_cur[j] = d0;
+    sc.iter[j] = 0;
+    sc.gamma[j] = 0.0;
+    int st = FB_SOLVER_PROGRESS;
+    if(!isfinite(d0))
+      st = FB_SOLVER_ABORTED;
+    else if(d0 <= EPS64 * EPS64)
+      st = FB_SOLVER_SUCCESS;
+    sc.status[j] = st;
+  }
+
+  // r = F(rhs - A x), ||r|| -> def_init, status: the staged pass (5.46 M rows: 106 us against 204
+  // of the row kernel below, which serves what the staged pass does not)
+  struct BOpPcgInit
+  {
+    struct Pre { double b; bool d; int j; };
+    typedef InstSum Acc;
+    static constexpr bool REDUCES = false;
+    const double* rhs; double* r; const uint8_t* dm; const int* sinst; BScal sc;
+    __device__ bool closed() const { return false; }
+    __device__ Pre pre(uint32_t i) const { return Pre{rhs[i], __ldg(dm + i) != 0, __ldg(sinst + (i >> 5))}; }
+    __device__ void operator()(uint32_t i, double sum, const Pre& p, InstSum& acc) const
+    {
+      const double rv = p.d ? 0.0 : sub(p.b, sum);
+      r[i] = rv;
+      acc.add(mul(rv, rv), p.j, sc);
+    }
+    __device__ void finish(double) const {}
+    __device__ void block_done(InstSum& acc) const
+    {
+      acc.flush(sc);
+      const BScal& s = sc;
+      blocks_done(sc, [&](int j, double tot) { open_instance(s, j, tot); });
+    }
+  };
+
   __global__ void __launch_bounds__(BNT, 3) kb_pcg_init(DCsr<double> A, const double* __restrict__ rhs,
     const double* __restrict__ x, double* __restrict__ r, const uint8_t* __restrict__ dm, const int* __restrict__ sinst,
     BScal sc)
@@ -780,20 +806,7 @@ namespace bt
       acc.add(sq, inst, sc);
     }
     acc.flush(sc);
-    blocks_done(sc, [&](int j, double tot)
-      {
-        const double d0 = sqrt(tot);
-        sc.def_init[j] = d0;
-        sc.def_cur[j] = d0;
-        sc.iter[j] = 0;
-        sc.gamma[j] = 0.0;
-        int st = FB_SOLVER_PROGRESS;
-        if(!isfinite(d0))
-          st = FB_SOLVER_ABORTED;
-        else if(d0 <= EPS64 * EPS64)
-          st = FB_SOLVER_SUCCESS;
-        sc.status[j] = st;
-      });
+    blocks_done(sc, [&](int j, double tot) { open_instance(sc, j, tot); });
   }
 
   // the V-cycle input of every instance at its top level: b = S(r * scale_j), sol1 = F(D .* b);
@@ -840,18 +853,38 @@ namespace bt
       });
   }
 
+  // p = z + beta p.  Bound by memory; one row per thread left too few loads in flight behind the
+  // instance's and its status' (5.46 M rows: 31 us against 23 with four)
   __global__ void __launch_bounds__(BNT, 4) kb_pcg_p(double* __restrict__ p, const double* __restrict__ z,
     const int* __restrict__ sinst, uint32_t n, int first, BScal sc)
   {
     if(closed(sc))
       return;
-    const uint32_t i = blockIdx.x * BNT + threadIdx.x;
-    if(i >= n)
-      return;
-    const int j = __ldg(sinst + (i >> 5));
-    if(!active(sc, j))
-      return;
-    p[i] = first ? z[i] : add(mul(p[i], sc.beta[j]), z[i]);
+    constexpr int U = PCGP_ROWS;
+    const uint32_t i0 = blockIdx.x * (BNT * U) + threadIdx.x;
+    double zv[U], pv[U];
+    int jv[U];
+    #pragma unroll
+    for(int u = 0; u < U; ++u)
+    {
+      const uint32_t i = i0 + uint32_t(u) * BNT;
+      jv[u] = i < n ? __ldg(sinst + (i >> 5)) : -1;
+    }
+    #pragma unroll
+    for(int u = 0; u < U; ++u)
+      if(jv[u] >= 0 && !active(sc, jv[u]))
+        jv[u] = -1;
+    #pragma unroll
+    for(int u = 0; u < U; ++u)
+      if(jv[u] >= 0)
+      {
+        zv[u] = z[i0 + uint32_t(u) * BNT];
+        pv[u] = first ? 0.0 : p[i0 + uint32_t(u) * BNT];
+      }
+    #pragma unroll
+    for(int u = 0; u < U; ++u)
+      if(jv[u] >= 0)
+        p[i0 + uint32_t(u) * BNT] = first ? zv[u] : add(mul(pv[u], sc.beta[jv[u]]), zv[u]);
   }
 
   __global__ void __launch_bounds__(BNT, 4) kb_pcg_q(DCsr<double> A, const double* __restrict__ p, double* __restrict__ q,
@@ -887,10 +920,12 @@ namespace bt
       });
   }
 
-  // x += alpha p, r -= alpha q, ||r||, stopping test, next V-cycle input at the top level; four
-  // rows per thread in flight
+  // x += alpha p, r -= alpha q, ||r||, stopping test, next V-cycle input at the top level.  Bound by
+  // memory: four rows per thread in flight with all they read, and an instance's scalars and pointers
+  // fetched where the instance changes, not per row (5.46 M rows: 86 us with the inverse diagonal and
+  // the scalars read row by row, 75 us now)
   template<typename S>
-  __global__ void __launch_bounds__(BNT, 4) kb_pcg_x(double* __restrict__ x, double* __restrict__ r,
+  __global__ void __launch_bounds__(BNT, 3) kb_pcg_x(double* __restrict__ x, double* __restrict__ r,
     const double* __restrict__ p, const double* __restrict__ q, const uint8_t* __restrict__ dm, TopPtrs<S> tp,
     const int* __restrict__ mg_base, const int* __restrict__ sinst, uint32_t n, int scale_mode, BScal sc)
   {
@@ -899,10 +934,16 @@ namespace bt
     constexpr int U = 4;
     InstSum acc;
     const Chunks ch(n);
+    int jc = -1;             // the instance of the scalars and pointers held
+    double alpha = 0.0, s = 1.0;
+    S *tb = nullptr, *tx = nullptr;
     for(uint32_t c0 = ch.first; c0 < ch.end; c0 += U)
     {
       double xv[U], rv[U], pv[U], qv[U];
+      S di[U];
+      uint32_t mr[U];
       int jv[U];
+      uint8_t dv[U];
       #pragma unroll
       for(int u = 0; u < U; ++u)
       {
@@ -912,12 +953,15 @@ namespace bt
         {
           const int j = __ldg(sinst + (i >> 5));
           jv[u] = active(sc, j) ? j : -1;
+          mr[u] = uint32_t(__ldg(mg_base + (i >> 5))) + (i & 31u);
           if(jv[u] >= 0)
           {
+            di[u] = __ldg(tp.dinv[sc.top[j]] + mr[u]);
             xv[u] = x[i];
             rv[u] = r[i];
             pv[u] = p[i];
             qv[u] = q[i];
+            dv[u] = __ldg(dm + i);
           }
         }
       }
@@ -926,20 +970,25 @@ namespace bt
       {
         const uint32_t i = (c0 + uint32_t(u)) * BNT + threadIdx.x;
         const int j = __shfl_sync(0xffffffffu, jv[u], 0);   // the warp's instance (a last partial warp's too)
+        if(j >= 0 && j != jc)
+        {
+          jc = j;
+          alpha = sc.alpha[j];
+          s = scale_mode ? pow2_inv(sc.def_cur[j]) : 1.0;
+          const int g = sc.top[j];
+          tb = tp.b[g];
+          tx = tp.x[g];
+        }
         double sq = 0.0;
         if(jv[u] >= 0)
         {
-          const double alpha = sc.alpha[j];
-          const double s = scale_mode ? pow2_inv(sc.def_cur[j]) : 1.0;
           x[i] = add(xv[u], mul(alpha, pv[u]));
           const double rn = add(rv[u], mul(-alpha, qv[u]));
           r[i] = rn;
-          const int g = sc.top[j];
-          const uint32_t mr = uint32_t(__ldg(mg_base + (i >> 5))) + (i & 31u);
           const S b = S(mul(rn, s));
-          tp.b[g][mr] = b;
-          const S cv = dm[i] ? S(0) : mul(tp.dinv[g][mr], b);
-          tp.x[g][mr] = add(S(0), cv);
+          tb[mr[u]] = b;
+          const S cv = dv[u] ? S(0) : mul(di[u], b);
+          tx[mr[u]] = add(S(0), cv);
           sq = mul(rn, rn);
         }
         acc.add(sq, j, sc);
@@ -1279,6 +1328,7 @@ namespace bt
       if(BLaunch<double, double>::use_tma(s->Atop))
       {
         BLaunch<double, double> d64{s, st, false};
+        d64.template tma<double, double>(s->Atop, nullptr, BOpPcgInit{}, true);
         d64.template tma<double, double>(s->Atop, nullptr, BOpPcgQ{}, true);
       }
     }
@@ -1396,7 +1446,14 @@ namespace bt
       if(!dry)
       {
         kb_open<<<4, 256, 0, st>>>(sc);
-        kb_pcg_init<<<one_wave(s->np, 3), BNT, 0, st>>>(bview<double>(s->Atop), s->rhs, s->x, s->r, s->dm_top, s->sinst_top, sc);
+        if(BLaunch<double, double>::use_tma(s->Atop))
+        {
+          BLaunch<double, double> d64{s, st, false};
+          d64.template tma<double, double>(s->Atop, s->x, BOpPcgInit{s->rhs, s->r, s->dm_top, s->sinst_top, sc});
+        }
+        else
+          kb_pcg_init<<<one_wave(s->np, 3), BNT, 0, st>>>(bview<double>(s->Atop), s->rhs, s->x, s->r, s->dm_top,
+            s->sinst_top, sc);
         kb_count<<<1, 256, 0, st>>>(sc, 0);
         kb_prep<S><<<one_wave(s->np), BNT, 0, st>>>(s->r, tops(), s->mg_base_top, s->dm_top, s->sinst_top, s->np,
           f64 ? 0 : 1, sc);
@@ -1411,7 +1468,7 @@ namespace bt
       const bool f64 = s->cfg.precision == FB_PREC_F64;
       if(!dry)
       {
-        kb_pcg_p<<<nblk(s->np), BNT, 0, st>>>(s->p, s->z, s->sinst_top, s->np, first ? 1 : 0, sc);
+        kb_pcg_p<<<nblk(s->np, BNT * PCGP_ROWS), BNT, 0, st>>>(s->p, s->z, s->sinst_top, s->np, first ? 1 : 0, sc);
         if(BLaunch<double, double>::use_tma(s->Atop))
         {
           BLaunch<double, double> d64{s, st, false};
@@ -1419,7 +1476,7 @@ namespace bt
         }
         else
           kb_pcg_q<<<nblk(s->np), BNT, 0, st>>>(bview<double>(s->Atop), s->p, s->q, s->dm_top, s->sinst_top, sc);
-        kb_pcg_x<S><<<one_wave(s->np), BNT, 0, st>>>(s->x, s->r, s->p, s->q, s->dm_top, tops(), s->mg_base_top,
+        kb_pcg_x<S><<<one_wave(s->np, 3), BNT, 0, st>>>(s->x, s->r, s->p, s->q, s->dm_top, tops(), s->mg_base_top,
           s->sinst_top, s->np, f64 ? 0 : 1, sc);
         kb_count<<<1, 256, 0, st>>>(sc, cond);
       }
