@@ -300,8 +300,19 @@ namespace un
     return conv_wbytes<C, BN, NST>() + halo_bytes(C, DIL);
   }
 
+  // Resident blocks per SM: by shared memory, and with registers for the accumulators (BN columns) and
+  // the fragments in flight.  The kernels are compiled for it: left alone the unrolled taps take 120 to
+  // 170 registers, so that three or four blocks were resident of a grid of eight per SM (the 48 -> 16 layer, batch 32 at 129 points: 81 -> 68 us).
+  template<int C, int BN, int DIL, int IN, int NST>
+  __host__ __device__ constexpr int conv_blocks()
+  {
+    constexpr int by_smem = 227 * 1024 / (conv_smem<C, BN, DIL, NST>() + 1024);
+    constexpr int by_regs = BN > 32 || IN == IN_CAT ? 4 : BN > 16 ? 5 : 6;
+    return by_smem < by_regs ? by_smem : by_regs;
+  }
+
   template<int C, int BN, int DIL, int IN, int OUT, int NST>
-  __global__ void __launch_bounds__(CNT) k_conv(const ConvArgs a)
+  __global__ void __launch_bounds__(CNT, conv_blocks<C, BN, DIL, IN, NST>()) k_conv(const ConvArgs a)
   {
     constexpr int HD = halo_dim(DIL), PXC = px_chunks(C), NT8 = BN / 8, BST = BN + 8;
     constexpr int WROWS = C == 8 ? 80 : C;         // weight rows of one stage
@@ -334,6 +345,14 @@ namespace un
     const uint32_t brow = smem_addr(sw) + uint32_t((lane & 15) * BST + (lane >> 4) * 8) * 2;
     const int half = lane >> 4;
 
+    // the weights that stay are fetched before the wait for the kernel ahead: no kernel that is followed
+    // by a convolution directly writes them
+    if constexpr(C == 8)
+      load_w(0, 0);
+    else if constexpr(NST == 9)
+      for(int s = 0; s < 9; ++s)
+        load_w(s, s);
+    pdl_wait();
     bool first = true;
     for(int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x)
     {
@@ -342,14 +361,8 @@ namespace un
       if(!first)
         __syncthreads();                            // the previous tile's reads are done
       load_halo<C, DIL, IN, CNT>(a.in, a.t, b, y0, x0, sx);
-      if(NST == 9 ? first : true)
-      {
-        if constexpr(C == 8)
-          load_w(0, 0);
-        else
-          for(int s = 0; s < (NST == 9 ? 9 : 1); ++s)
-            load_w(s, s);
-      }
+      if constexpr(C != 8 && NST != 9)
+        load_w(0, 0);
       cp_commit();
       float acc[2][NT8][4];
       #pragma unroll
@@ -520,10 +533,12 @@ namespace un
   };
 
   template<int C, int M, int DIL>
-  __host__ __device__ constexpr int wgrad_smem()
+  __host__ __device__ constexpr int wgrad_stage()
   {
     return halo_bytes(C, DIL) + 128 * px_chunks(M) * 16;
   }
+  template<int C, int M, int DIL>
+  __host__ __device__ constexpr int wgrad_smem() { return 2 * wgrad_stage<C, M, DIL>(); }
 
   template<int C, int M, int DIL, int IN, bool SCALAR, int NW>
   __global__ void __launch_bounds__(NW * 32) k_wgrad(const WgradArgs a)
@@ -535,6 +550,7 @@ namespace un
     extern __shared__ __align__(16) unsigned char smem[];
     bf* sx = reinterpret_cast<bf*>(smem);
     bf* sd = reinterpret_cast<bf*>(smem + halo_bytes(C, DIL));
+    constexpr int STAGE = wgrad_stage<C, M, DIL>();
     __shared__ int pxo[128];                        // halo offset (bytes) of each pixel slot
     Input in = a.in;
     in.c0 += int(blockIdx.y) * C;
@@ -568,19 +584,19 @@ namespace un
       for(int e = 0; e < 4; ++e)
         accb[i][e] = 0.f;
     }
-    for(int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x)
+    // a tile's input and output gradient into buffer `buf`
+    auto load = [&](int tile, int buf)
     {
       const int b = tile / (nt * nt), r = tile - b * (nt * nt);
       const int y0 = r / nt * T, x0 = (r - r / nt * nt) * T;
-      __syncthreads();                              // pxo written; the previous tile's reads are done
-      load_halo<C, DIL, IN, NT>(in, a.t, b, y0, x0, sx);
+      load_halo<C, DIL, IN, NT>(in, a.t, b, y0, x0, sx + buf * (STAGE / 2));
       for(int e = tid; e < 128 * (M / 8); e += NT)
       {
         const int ch = e % (M / 8), m = e / (M / 8);
         const int ty = m / T, y = y0 + ty, x = x0 + m - ty * T;
         const bool ok = m < TT && y < G && x < G;
         const size_t p = (size_t(b) * G + y) * G + x;
-        bf* dst = sd + (m * PXD + ch) * 8;
+        bf* dst = sd + buf * (STAGE / 2) + (m * PXD + ch) * 8;
         if constexpr(SCALAR)
         {
           const uint32_t w = ok && ch == 0 ? uint32_t(f2bf(__ldg(static_cast<const float*>(a.dy) + p))) : 0u;
@@ -593,12 +609,28 @@ namespace un
         }
       }
       cp_commit();
-      cp_wait<0>();
-      __syncthreads();
+    };
+    int buf = 0;
+    pdl_wait();
+    if(int(blockIdx.x) < a.ntiles)
+      load(int(blockIdx.x), 0);
+    for(int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x, buf ^= 1)
+    {
+      // the next tile's copies run under this tile's products (its buffer's reads ended with the last
+      // round's barrier)
+      if(tile + int(gridDim.x) < a.ntiles)
+      {
+        load(tile + int(gridDim.x), buf ^ 1);
+        cp_wait<1>();
+      }
+      else
+        cp_wait<0>();
+      __syncthreads();                              // (pxo written, the first time)
+      const uint32_t so = uint32_t(buf * STAGE);
       #pragma unroll 2
       for(int k = 0; k < 8; ++k)
       {
-        const uint32_t px = uint32_t(pxo[k * 16 + (lane & 15)]);
+        const uint32_t px = uint32_t(pxo[k * 16 + (lane & 15)]) + so;
         uint32_t bfr[GPW][4];
         #pragma unroll
         for(int j = 0; j < GPW; ++j)
@@ -607,7 +639,7 @@ namespace un
         for(int mt = 0; mt < MT; ++mt)
         {
           uint32_t af[4];
-          ldm_x4a_t(af, drow + uint32_t(k * 16 * PXD * 16 + mt * 32));
+          ldm_x4a_t(af, drow + so + uint32_t(k * 16 * PXD * 16 + mt * 32));
           #pragma unroll
           for(int j = 0; j < GPW; ++j)
           {
@@ -618,6 +650,7 @@ namespace un
             mma16816(accb[mt], af, 0x3F803F80u, 0x3F803F80u);   // times ones: the bias gradient
         }
       }
+      __syncthreads();                              // this buffer's reads are done
     }
     const int g = lane >> 2, tg = lane & 3;
     const int n9 = 9 * in.ct;
@@ -676,6 +709,7 @@ namespace un
   __global__ void __launch_bounds__(GR_E * GR_G) k_grad_reduce(const __grid_constant__ NetMap net,
     float* __restrict__ grad, int accumulate)
   {
+    pdl_wait();
     __shared__ float sh[GR_G][GR_E];
     const int x = threadIdx.x % GR_E, grp = threadIdx.x / GR_E;
     const int e = blockIdx.x * GR_E + x;
@@ -722,6 +756,7 @@ namespace un
   }
   __global__ void __launch_bounds__(256) k_prep_weights(const __grid_constant__ NetMap net, const float* __restrict__ p)
   {
+    pdl_wait();
     const int e = blockIdx.x * 256 + threadIdx.x;
     if(e >= net.n)
       return;
@@ -735,6 +770,7 @@ namespace un
     const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v, float lr, float b1, float b2, float eps,
     float c1, float c2)
   {
+    pdl_wait();
     const int i = blockIdx.x * 256 + threadIdx.x;
     if(i >= net.n)
       return;
@@ -754,6 +790,7 @@ namespace un
   // NCHW FP32 input (2 channels) -> BF16 pairs per pixel (kept for the first layer's weight gradient)
   __global__ void k_pack_input(const float* __restrict__ in, int B, int G, uint32_t* __restrict__ x)
   {
+    pdl_wait();
     const size_t n = size_t(G) * G;
     for(size_t p = blockIdx.x * size_t(blockDim.x) + threadIdx.x; p < n * B; p += size_t(gridDim.x) * blockDim.x)
     {
@@ -784,6 +821,7 @@ namespace un
   __global__ void __launch_bounds__(256) k_upsample_bwd_mask(const float* __restrict__ gf, int C, int B, int Gf,
     const bf* __restrict__ post, bf* __restrict__ dpre)
   {
+    pdl_wait();
     const int Gc = (Gf + 1) / 2, C8 = C / 8;
     const size_t n = size_t(B) * Gc * Gc * C8;
     for(size_t e = blockIdx.x * size_t(256) + threadIdx.x; e < n; e += size_t(gridDim.x) * 256)
@@ -817,6 +855,7 @@ namespace un
   __global__ void __launch_bounds__(256) k_grad_mask(const bf* __restrict__ post, int C, int B, int G,
     const float* __restrict__ g1, const float* __restrict__ g2, bf* __restrict__ dpre)
   {
+    pdl_wait();
     const int Gc = (G + 1) / 2, C8 = C / 8;
     const size_t n = size_t(B) * G * G * C8;
     for(size_t e = blockIdx.x * size_t(256) + threadIdx.x; e < n; e += size_t(gridDim.x) * 256)
@@ -845,6 +884,7 @@ namespace un
   __global__ void __launch_bounds__(MSE_NT) k_mse(const float* __restrict__ y, const float* __restrict__ t, size_t n,
     float* __restrict__ grad, RedSlot slot, double* __restrict__ loss)
   {
+    pdl_wait();
     __shared__ double sh[32];
     double s = 0.0;
     const float inv = 1.f / float(n);
@@ -951,17 +991,35 @@ namespace
     return m;
   }
 
+  // A launch with programmatic stream serialisation: scheduled while the kernel ahead finishes, every
+  // kernel waits for it in pdl_wait.  Ten layers forward and forty kernels of a training step spent 2 us
+  // each between one's end and the next one's first load (a prediction of batch 1: 83 -> 52 us).
+  template<typename... KA, typename... A>
+  cudaError_t launch(void (*k)(KA...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, A&&... args)
+  {
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = grid;
+    lc.blockDim = dim3(block);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = &at;
+    lc.numAttrs = 1;
+    return cudaLaunchKernelEx(&lc, k, KA(args)...);
+  }
+
   template<int C, int BN, int DIL, int IN, int OUT, int NST>
   fb_status launch_conv(const ConvArgs& a, cudaStream_t st)
   {
     constexpr int smem = conv_smem<C, BN, DIL, NST>();
     if(smem > 48 * 1024)
       FB_CUDA(cudaFuncSetAttribute(k_conv<C, BN, DIL, IN, OUT, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    // resident blocks per SM by shared memory, at most 8 (32 warps)
-    constexpr int occ = std::min(8, 227 * 1024 / (smem + 1024));
+    constexpr int occ = conv_blocks<C, BN, DIL, IN, NST>();
     const int ny = a.n / BN;
     dim3 grid(unsigned(std::min(a.ntiles, std::max(1, SMS * occ / ny))), unsigned(ny));
-    k_conv<C, BN, DIL, IN, OUT, NST><<<grid, CNT, smem, st>>>(a);
+    FB_CUDA(launch(k_conv<C, BN, DIL, IN, OUT, NST>, dim3(grid), CNT, smem, st, a));
     FB_LAUNCHED(1);
     return FB_OK;
   }
@@ -1024,14 +1082,14 @@ namespace
     a.m_real = LAYERS[l].cout;
     a.ntiles = tiles(a.t, B);
     const dim3 grid(unsigned(wgrad_blocks(u, l, B)), unsigned(u->cin_pad[l] / C));
-    k_wgrad<C, M, DIL, IN, SCALAR, NW><<<grid, NW * 32, smem, st>>>(a);
+    FB_CUDA(launch(k_wgrad<C, M, DIL, IN, SCALAR, NW>, dim3(grid), NW * 32, smem, st, a));
     FB_LAUNCHED(1);
     return FB_OK;
   }
 
   fb_status prep_weights(fb_unet* u, cudaStream_t st)
   {
-    k_prep_weights<<<unsigned((u->nparam + 255) / 256), 256, 0, st>>>(net_map(u, 0), u->param);
+    FB_CUDA(launch(k_prep_weights, dim3(unsigned((u->nparam + 255) / 256)), 256, 0, st, net_map(u, 0), u->param));
     FB_LAUNCHED(1);
     u->weights_ready = true;
     return FB_OK;
@@ -1200,7 +1258,7 @@ fb_status fb_unet_forward(fb_unet* u, const float* in, float* out, int batch, vo
   }
   cudaStream_t st = as_stream(stream);
   const int B = batch;
-  k_pack_input<<<grid_for(size_t(B) * u->G[0] * u->G[0]), 256, 0, st>>>(in, B, u->G[0], u->xp);
+  FB_CUDA(launch(k_pack_input, dim3(grid_for(size_t(B) * u->G[0] * u->G[0])), 256, 0, st, in, B, u->G[0], u->xp));
   FB_LAUNCHED(1);
   UN_TRY((conv_fwd<8, 16, 1, IN_PAIR, OUT_RELU, 9>(u, 0, Input{u->xp, nullptr, 0, 8, 0}, B, u->e[0], st)));
   UN_TRY((conv_fwd<16, 32, 1, IN_SUB, OUT_RELU, 9>(u, 1, plain(u->e[0], 16), B, u->e[1], st)));
@@ -1234,14 +1292,14 @@ fb_status fb_unet_backward(fb_unet* u, const float* dout, int batch, int accumul
   // dpre = mask(post) * U^T(du) at level lv + 1 (C channels)
   auto up_bwd = [&](int lv, int C, const bf* post, bf* dpre)
   {
-    k_upsample_bwd_mask<<<grid_for(n8(lv + 1, C)), 256, 0, st>>>(u->du[lv], C, B, G[lv], post, dpre);
+    FB_CUDA(launch(k_upsample_bwd_mask, dim3(grid_for(n8(lv + 1, C))), 256, 0, st, u->du[lv], C, B, G[lv], post, dpre));
     FB_LAUNCHED(1);
     return fb_status(FB_OK);
   };
   // dpre = mask(e[lv]) * (skip gradient + S^T(gs))
   auto skip_bwd = [&](int lv, int C, bf* dpre)
   {
-    k_grad_mask<<<grid_for(n8(lv, C)), 256, 0, st>>>(u->e[lv], C, B, G[lv], u->dk[lv], u->gs, dpre);
+    FB_CUDA(launch(k_grad_mask, dim3(grid_for(n8(lv, C))), 256, 0, st, u->e[lv], C, B, G[lv], u->dk[lv], u->gs, dpre));
     FB_LAUNCHED(1);
     return fb_status(FB_OK);
   };
@@ -1279,7 +1337,7 @@ fb_status fb_unet_backward(fb_unet* u, const float* dout, int batch, int accumul
   // L1 (input f, log kappa)
   UN_TRY(skip_bwd(0, 16, p0));
   UN_TRY((wgrad<8, 16, 1, IN_PAIR, false, 5>(u, 0, p0, Input{u->xp, nullptr, 0, 8, 0}, B, st)));
-  k_grad_reduce<<<unsigned((u->nparam + GR_E - 1) / GR_E), GR_E * GR_G, 0, st>>>(net_map(u, B), u->grad, accumulate ? 1 : 0);
+  FB_CUDA(launch(k_grad_reduce, dim3(unsigned((u->nparam + GR_E - 1) / GR_E)), GR_E * GR_G, 0, st, net_map(u, B), u->grad, accumulate ? 1 : 0));
   FB_LAUNCHED(1);
   return FB_OK;
 }
@@ -1295,8 +1353,8 @@ fb_status fb_unet_adam(fb_unet* u, float lr, float beta1, float beta2, float eps
   }
   cudaStream_t st = as_stream(stream);
   const float c1 = 1.f - std::pow(beta1, float(t)), c2 = 1.f - std::pow(beta2, float(t));
-  k_adam<<<unsigned((u->nparam + 255) / 256), 256, 0, st>>>(net_map(u, 0), u->param, u->grad, u->adam_m, u->adam_v, lr,
-    beta1, beta2, eps, c1, c2);
+  FB_CUDA(launch(k_adam, dim3(unsigned((u->nparam + 255) / 256)), 256, 0, st, net_map(u, 0), u->param, u->grad, u->adam_m, u->adam_v, lr,
+    beta1, beta2, eps, c1, c2));
   FB_LAUNCHED(1);
   u->weights_ready = true;
   return FB_OK;
@@ -1313,7 +1371,7 @@ fb_status fb_unet_mse(fb_unet* u, const float* y, const float* t, uint64_t n, fl
   }
   cudaStream_t st = as_stream(stream);
   const int nb = int(std::min<uint64_t>(1024, (n + MSE_NT - 1) / MSE_NT));
-  k_mse<<<nb, MSE_NT, 0, st>>>(y, t, size_t(n), grad, RedSlot{u->mse_part, u->mse_counter}, loss);
+  FB_CUDA(launch(k_mse, dim3(nb), MSE_NT, 0, st, y, t, size_t(n), grad, RedSlot{u->mse_part, u->mse_counter}, loss));
   FB_LAUNCHED(1);
   return FB_OK;
 }
