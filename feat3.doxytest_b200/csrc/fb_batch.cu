@@ -208,6 +208,135 @@ namespace bt
     coarse_block<S, BNT>(b + r0, x + r0, n, free_dofs + f0, inv + inv_off[j], m);
   }
 
+  // The levels 0 .. count-1 of every instance's V-cycle in one kernel, one block per instance: levels of
+  // at most BOT_NT rows per instance, below every instance's top.  A launched pass over such levels takes
+  // 3 us, 6 us with a norm, whatever it computes, and they are 6 per level; here a pass is a row per
+  // thread and a block barrier, matrices and vectors in the SM's L1 after the first pass.  The rows are
+  // the launched passes' (fb_rows.cuh); vectors are read by plain loads, the block writes them itself.
+  // 64 instances of 2D levels 5 to 9 (three levels and the coarse solve): 31 us for 78 us of launched
+  // passes, 6,986 -> 6,612 us a batch of eight iterations.
+  constexpr int BOT_NT = 320;
+  constexpr int BOT_MAX = 6;
+  template<typename V, typename S>
+  struct BotLevel
+  {
+    DCsr<V> A, P, R;             // P: this level <- the next coarser, R: the next coarser <- this level
+    S *b, *x, *x2, *d, *c, *c2;
+    const S* dinv;
+    const uint8_t* dm;
+    const uint32_t* off;         // per instance: first row, rows
+  };
+  template<typename V, typename S>
+  struct BotParams
+  {
+    BotLevel<V, S> lv[BOT_MAX];  // level 0 = the coarsest
+    int count, steps;
+    const int* skip_pre;         // the finest of these levels' flags, from the restriction ahead
+    const uint32_t* free_off;
+    const uint32_t* free_dofs;
+    const uint64_t* inv_off;
+    const double* inv;
+  };
+
+  template<typename V, typename S>
+  __global__ void __launch_bounds__(BOT_NT) kb_bottom(const __grid_constant__ BotParams<V, S> p, BScal sc)
+  {
+    if(closed(sc))
+      return;
+    const int j = blockIdx.x;
+    if(!active(sc, j))
+      return;
+    __shared__ double red[BOT_NT / 32];
+    __shared__ int skips[BOT_MAX];
+    // the block's sum of v, the same in every thread
+    auto total = [&](double v)
+    {
+      #pragma unroll
+      for(int o = 16; o > 0; o >>= 1)
+        v += __shfl_xor_sync(0xffffffffu, v, o);
+      if((threadIdx.x & 31u) == 0)
+        red[threadIdx.x >> 5] = v;
+      __syncthreads();
+      double t = 0.0;
+      for(int w = 0; w < BOT_NT / 32; ++w)
+        t += red[w];
+      __syncthreads();
+      return t;
+    };
+    const int steps = p.steps;
+    if(threadIdx.x == 0)
+      skips[p.count - 1] = p.skip_pre[j];
+    __syncthreads();
+    for(int t = p.count - 1; t >= 1; --t)
+    {
+      const BotLevel<V, S>& f = p.lv[t];
+      const BotLevel<V, S>& c = p.lv[t - 1];
+      const uint32_t i = f.off[2 * j] + threadIdx.x, ic = c.off[2 * j] + threadIdx.x;
+      const bool on = threadIdx.x < f.off[2 * j + 1], onc = threadIdx.x < c.off[2 * j + 1];
+      const bool skip = skips[t] != 0;
+      S *xa = f.x, *xb = f.x2;
+      for(int k = 1; k < steps; ++k)
+      {
+        if(on)
+          xb[i] = smooth_row<V, S, false>(f.A, f.b, xa, f.dinv, f.dm, skip, i);
+        __syncthreads();
+        S* y = xa;
+        xa = xb;
+        xb = y;
+      }
+      if(on)
+        f.d[i] = defect_row<V, S, false>(f.A, f.b, xa, f.dm, i);
+      __syncthreads();
+      double sq = 0.0;
+      if(onc)
+        sq = restrict_row<V, S, false>(f.R, f.d, c.b, t > 1 ? c.x : static_cast<S*>(nullptr), c.dinv, c.dm, ic);
+      const double nrm = total(sq);
+      if(threadIdx.x == 0)
+        skips[t - 1] = skip_from_norm<S>(sqrt(nrm));
+      __syncthreads();
+    }
+    {
+      const BotLevel<V, S>& c = p.lv[0];
+      const uint32_t r0 = c.off[2 * j], f0 = p.free_off[j];
+      coarse_block<S, BOT_NT>(c.b + r0, c.x + r0, c.off[2 * j + 1], p.free_dofs + f0, p.inv + p.inv_off[j],
+        p.free_off[j + 1] - f0);
+      __syncthreads();
+    }
+    for(int t = 1; t < p.count; ++t)
+    {
+      const BotLevel<V, S>& f = p.lv[t];
+      const uint32_t i = f.off[2 * j] + threadIdx.x;
+      const bool on = threadIdx.x < f.off[2 * j + 1];
+      // the buffers the pre-smoothing steps left the iterates in
+      const bool odd = (steps - 1) % 2 != 0;
+      S* xf = odd ? f.x2 : f.x;
+      const S* xc = t > 1 && odd ? p.lv[t - 1].x2 : p.lv[t - 1].x;
+      if(on)
+        xf[i] = prolong_row<V, S, false>(f.P, xc, xf, f.dm, i);
+      __syncthreads();
+      double sq = 0.0;
+      if(on)
+        sq = post1_row<V, S, false>(f.A, f.b, xf, f.d, f.c, f.dinv, f.dm, i);
+      const bool skip = skip_from_norm<S>(sqrt(total(sq))) != 0;
+      S *ca = f.c, *cb = f.c2;
+      for(int k = 2; k <= steps; ++k)
+      {
+        if(on)
+        {
+          const auto cn = post2_row<V, S, false>(f.A, f.d, ca, f.dinv, f.dm, skip, i);
+          if(k == steps)
+            xf[i] = S(add(typename ValueTraits<V>::acc(xf[i]), cn));
+          else
+            cb[i] = S(cn);
+        }
+        __syncthreads();
+        S* y = ca;
+        ca = cb;
+        cb = y;
+      }
+    }
+  }
+
   template<typename V, typename S>
   __global__ void __launch_bounds__(BNT_MAX) kb_prolong(DCsr<V> P, const S* __restrict__ xc, S* __restrict__ x,
     const uint8_t* __restrict__ dm, const int* __restrict__ sinst, BScal sc)
@@ -1063,10 +1192,12 @@ struct fb_batch
     int* sinst = nullptr;
     int* pcg_base = nullptr;
     std::vector<uint32_t> off;   // per instance row offset (UINT32_MAX: absent)
+    uint32_t* span = nullptr;    // levels of the bottom kernel: per instance first row and rows
     int bs = 256;                // rows per block of this level's V-cycle passes (autotuned)
   };
   fb_solver_config cfg;
   int J = 0, NG = 0;
+  int bottom = 0;                // levels 0 .. bottom run in kb_bottom (0: the coarse solve alone)
   std::vector<int> top;
   std::vector<GLevel> g;
   std::vector<void*> allocs;
@@ -1333,13 +1464,33 @@ namespace bt
       }
     }
 
+    void launch_bottom()
+    {
+      BotParams<V, S> p;
+      std::memset(&p, 0, sizeof(p));
+      p.count = s->bottom + 1;
+      p.steps = s->cfg.smooth_steps;
+      for(int G = 0; G < p.count; ++G)
+      {
+        const fb_batch::GLevel& f = s->g[size_t(G)];
+        p.lv[G] = BotLevel<V, S>{bview<V>(f.A), bview<V>(f.P), bview<V>(f.R), (S*)f.b, (S*)f.x, (S*)f.x2, (S*)f.d,
+                                 (S*)f.c, (S*)f.c2, (const S*)f.dinv, f.dm, f.span};
+      }
+      p.skip_pre = s->sc.skip_pre + size_t(s->bottom) * s->sc.J;
+      p.free_off = s->c_free_off;
+      p.free_dofs = s->c_free;
+      p.inv_off = s->c_inv_off;
+      p.inv = s->c_inv;
+      kb_bottom<V, S><<<s->J, BOT_NT, 0, st>>>(p, s->sc);
+    }
+
     void vcycle()
     {
       const int NG = s->NG;
       const int steps = s->cfg.smooth_steps;
       BScal sc = s->sc;
       std::vector<void*> xcur(static_cast<size_t>(NG));
-      for(int G = NG - 1; G >= 1; --G)
+      for(int G = NG - 1; G >= 1 && G > s->bottom; --G)
       {
         fb_batch::GLevel& f = s->g[size_t(G)];
         fb_batch::GLevel& c = s->g[size_t(G - 1)];
@@ -1381,6 +1532,18 @@ namespace bt
         launches += 2;
         bytes += cb(f.A, 1, 1) + cb(f.R, 0, 3);
       }
+      if(s->bottom > 0)
+      {
+        if(!dry)
+          launch_bottom();
+        ++launches;
+        for(int G = 1; G <= s->bottom; ++G)
+          bytes += cb(s->g[size_t(G)].A, 6 + 4 * (steps - 1), 3 + 2 * (steps - 1)) + cb(s->g[size_t(G)].R, 0, 3) +
+                   cb(s->g[size_t(G)].P, 1, 1);
+        fb_batch::GLevel& c = s->g[size_t(s->bottom)];
+        xcur[size_t(s->bottom)] = (steps - 1) % 2 ? c.x2 : c.x;
+      }
+      else
       {
         fb_batch::GLevel& c = s->g[0];
         if(!dry)
@@ -1390,7 +1553,7 @@ namespace bt
         bytes += double(c.n) * 2 * sizeof(S);
         xcur[0] = c.x;
       }
-      for(int G = 1; G < NG; ++G)
+      for(int G = s->bottom + 1; G < NG; ++G)
       {
         fb_batch::GLevel& f = s->g[size_t(G)];
         void* xf = xcur[size_t(G)];
@@ -2025,6 +2188,23 @@ fb_status fb_batch_create(fb_batch** out, int num, fb_hierarchy* const* hs, cons
     BT_TRY(bt::upload_vec(s.get(), &s->c_free, fr_all));
     BT_TRY(bt::upload_vec(s.get(), &s->c_inv_off, inv_off));
     BT_TRY(bt::upload_vec(s.get(), &s->c_inv, inv_all));
+  }
+  // the levels of the bottom kernel: below every instance's top, a row per thread of one block
+  const int low = *std::min_element(s->top.begin(), s->top.end());
+  for(int G = 0; G < low && G < bt::BOT_MAX; ++G)
+  {
+    std::vector<uint32_t> span(size_t(J) * 2);
+    uint32_t rows = 0;
+    for(int j = 0; j < J; ++j)
+    {
+      span[size_t(j) * 2] = s->g[size_t(G)].off[size_t(j)];
+      span[size_t(j) * 2 + 1] = hs[j]->levels[size_t(own(j, G))].A.rows;
+      rows = std::max(rows, span[size_t(j) * 2 + 1]);
+    }
+    if(rows > uint32_t(bt::BOT_NT))
+      break;
+    BT_TRY(bt::upload_vec(s.get(), &s->g[size_t(G)].span, span));
+    s->bottom = G;
   }
   // per instance scalars
   {

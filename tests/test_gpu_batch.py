@@ -126,3 +126,31 @@ def test_batch_many_instances_per_block(featlib, cuda, precision):
         assert len(set(bat.iterations()[k::3])) == 1
         for j in (k, 150 + k, 297 + k):
             assert rel_err(X[j], x.elements) <= (1e-12 if precision == "f64" else 1e-7)
+
+
+# the bottom kernel's range: no level of its own (a top on level 2), one, four (289 rows) and the most
+# with a level of 1,089 rows left to launched passes; one instance and more than one block per SM holds;
+# three smoothing steps (the correction's buffers change places)
+@pytest.mark.parametrize("levels,ordering,precision,steps", [
+    ([2, 3], "native", "f64", 2), ([3], "rcm", "f64", 3), ([5, 6, 5], "native", "f64", 2), ([6, 7], "rcm", "f32_bf16", 2),
+    ([5, 6], "native", "f32", 3), ([5] * 200 + [6], "native", "f32", 2)])
+def test_batch_bottom_kernel(featlib, cuda, levels, ordering, precision, steps):
+    """Instances agree with their single solves at every depth of the levels below the lowest top."""
+    fb = featlib
+    inst = _family(sorted(set(levels)))
+    by = dict(zip(sorted(set(levels)), inst))
+    single = {}
+    for L, (lv, b) in by.items():
+        s = fb.build_pcg_multigrid(lv, ordering=ordering, precision=precision, steps=steps)
+        x = fb.DenseVector(b.size)
+        assert fb.solve(s, x, fb.DenseVector(b)) == fb.Status.success
+        single[L] = (x.elements.copy(), s.get_num_iter())
+    hs = {L: fb.build_hierarchy(lv, steps=steps) for L, (lv, _) in by.items()}
+    bat = fb.BatchPCG([hs[L] for L in levels], ordering=ordering, precision=precision)
+    rhs = np.concatenate([by[L][1] for L in levels])
+    X = bat.split(bat.solve(np.zeros_like(rhs), rhs))
+    for k, L in enumerate(levels):
+        assert bat.statuses()[k] == fb.Status.success
+        assert bat.iterations()[k] == single[L][1]
+        # the order of the PCG's sums differs
+        assert rel_err(X[k], single[L][0]) <= (1e-12 if precision == "f64" else 1e-9)
