@@ -167,7 +167,7 @@ namespace un
     const int cy0 = (y0 - DIL) >> 1, cx0 = (x0 - DIL) >> 1;
     const unsigned ncx = unsigned(((x0 + t.T + DIL - 1) >> 1) - cx0 + 1), ncy = unsigned(((y0 + t.T + DIL - 1) >> 1) - cy0 + 1);
     const bf* cb = static_cast<const bf*>(in.x) + size_t(b) * Gc * Gc * in.cu + in.c0;
-    #pragma unroll 2
+    #pragma unroll 1
     for(unsigned e = threadIdx.x; e < ncy * ncx * nu; e += NT)
     {
       const unsigned q = e / nu, ch = e - q * nu, iy = q / ncx;
@@ -307,7 +307,7 @@ namespace un
   __host__ __device__ constexpr int conv_blocks()
   {
     constexpr int by_smem = 227 * 1024 / (conv_smem<C, BN, DIL, NST>() + 1024);
-    constexpr int by_regs = BN > 32 || IN == IN_CAT ? 4 : BN > 16 ? 5 : 6;
+    constexpr int by_regs = BN > 32 ? 4 : BN > 16 || IN == IN_CAT ? 5 : 6;
     return by_smem < by_regs ? by_smem : by_regs;
   }
 
@@ -540,8 +540,14 @@ namespace un
   template<int C, int M, int DIL>
   __host__ __device__ constexpr int wgrad_smem() { return 2 * wgrad_stage<C, M, DIL>(); }
 
+  // Resident blocks per SM by the accumulators' registers: layers of few weights take three or four
+  // (batch 32 at 129 points: 48 -> 16 62 -> 57 us, 2 -> 16 31 -> 19, 16 -> 1 32 -> 26); 96 -> 32 takes one of
+  // 18 warps, three column groups each, where nine warps with six held 14% of the SM's warps (58 -> 47 us)
+  template<int C, int M>
+  __host__ __device__ constexpr int wgrad_resident() { return C * M <= 256 ? 4 : C * M <= 768 ? 3 : 1; }
+
   template<int C, int M, int DIL, int IN, bool SCALAR, int NW>
-  __global__ void __launch_bounds__(NW * 32) k_wgrad(const WgradArgs a)
+  __global__ void __launch_bounds__(NW * 32, wgrad_resident<C, M>()) k_wgrad(const WgradArgs a)
   {
     constexpr int NT = NW * 32, HD = halo_dim(DIL), PXC = px_chunks(C), PXD = px_chunks(M);
     constexpr int MT = M / 16, CH = C / 8;
@@ -965,7 +971,8 @@ namespace
   {
     const int nt = tiles(tiling(u->G[LAYERS[l].level]), B);
     const int big = LAYERS[l].cin * LAYERS[l].cout >= 64 * 64;
-    const int cap = l == 6 ? SMS / 2 : big ? SMS : 2 * SMS;
+    const int w = u->cin_pad[l] * pad8(LAYERS[l].cout);
+    const int cap = l == 6 ? SMS / 2 : w <= 256 ? 4 * SMS : w <= 768 ? 3 * SMS : SMS;
     return std::max(1, std::min(big ? (nt + 1) / 2 : nt, cap));
   }
 
@@ -1312,7 +1319,7 @@ fb_status fb_unet_backward(fb_unet* u, const float* dout, int batch, int accumul
   UN_TRY((conv_bwd<16, 48, 1, IN_PLAIN, OUT_F32, 9>(u, 8, plain(p0, 16), B, u->du[0], u->dk[0], 32, nullptr, st)));
   UN_TRY(up_bwd(0, 32, u->d[1], p1));
   // L6 (input [U(d3), e2])
-  UN_TRY((wgrad<96, 32, 1, IN_CAT, false, 9>(u, 7, p1, concat(u->d[2], 64, u->e[1], 32), B, st)));
+  UN_TRY((wgrad<96, 32, 1, IN_CAT, false, 18>(u, 7, p1, concat(u->d[2], 64, u->e[1], 32), B, st)));
   UN_TRY((conv_bwd<32, 48, 1, IN_PLAIN, OUT_F32, 9>(u, 7, plain(p1, 32), B, u->du[1], u->dk[1], 64, nullptr, st)));
   UN_TRY(up_bwd(1, 64, u->d[2], p0));
   // L5 (input [U(e4), e3])
