@@ -41,12 +41,12 @@ namespace fb
   }
 
   // Row sum of row `row` in stored entry order; every product and sum rounded separately.  NC:
-  // gather the vector through the read-only path (vectors not written by the same kernel).
-  template<typename V, typename S, bool NC = true>
+  // gather the vector through the read-only path (vectors not written by the same kernel).  U: entries
+  // whose loads go out together.
+  template<typename V, typename S, bool NC = true, uint32_t U = 9>
   __device__ __forceinline__ typename ValueTraits<V>::acc row_sum(const DCsr<V>& M, uint32_t row, const S* x)
   {
     typedef typename ValueTraits<V>::acc A;
-    constexpr uint32_t U = 9;
     const uint32_t sl = row >> 5;
     if(M.kw == U && (M.dcol || M.doff))
     {
@@ -167,14 +167,14 @@ namespace fb
   // b_c = F_c(R d) and (with_x) sol1_c = F_c(D_c .* b_c), without stores
   template<typename Ac>
   struct RestrictOut { Ac v, x; };
-  template<typename V, typename S, bool NC>
+  template<typename V, typename S, bool NC, uint32_t U = 9>
   __device__ __forceinline__ RestrictOut<typename ValueTraits<V>::acc> restrict_calc(const DCsr<V>& R, const S* d,
     bool with_x, const S* dinvc, const uint8_t* dmc, uint32_t j)
   {
     typedef typename ValueTraits<V>::acc Ac;
     const bool dc = __ldg(dmc + j) != 0;
     const Ac di = with_x ? Ac(__ldg(dinvc + j)) : Ac(0);
-    const Ac sum = row_sum<V, S, NC>(R, j, d);
+    const Ac sum = row_sum<V, S, NC, U>(R, j, d);
     const Ac v = dc ? Ac(0) : add(sum, Ac(0));
     Ac x = Ac(0);
     if(with_x)
@@ -186,11 +186,11 @@ namespace fb
   }
 
   // b_c = F_c(R d) and (xc != null) sol1_c = F_c(D_c .* b_c); returns b_c^2
-  template<typename V, typename S, bool NC>
+  template<typename V, typename S, bool NC, uint32_t U = 9>
   __device__ __forceinline__ double restrict_row(const DCsr<V>& R, const S* d, S* bc, S* xc, const S* dinvc,
     const uint8_t* dmc, uint32_t j)
   {
-    const auto o = restrict_calc<V, S, NC>(R, d, xc != nullptr, dinvc, dmc, j);
+    const auto o = restrict_calc<V, S, NC, U>(R, d, xc != nullptr, dinvc, dmc, j);
     bc[j] = S(o.v);
     if(xc)
       xc[j] = S(o.x);
