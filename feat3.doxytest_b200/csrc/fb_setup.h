@@ -75,7 +75,7 @@ namespace fb
   // DIAG_MAX diagonals and every row's columns are strictly increasing, the matrix is stored as
   // plain ELL whose entry k of every row is the diagonal doff[k] (column = row + doff[k]), without
   // column indices: a row's entries keep their stored order, the diagonals it lacks hold value 0
-  // (at most 12.5% padding, except for matrices of at most DIAG_SMALL_ROWS rows).
+  // (at most 25% padding, except for matrices of at most DIAG_SMALL_ROWS rows).
   constexpr uint32_t DIAG_MAX = 27;
   constexpr uint32_t DIAG_SMALL_ROWS = 4096;   // up to this many rows: no padding limit
   struct HostSell

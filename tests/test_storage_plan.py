@@ -3,6 +3,7 @@ structured grids numbered lexicographically, sliced / uniform ELL with int16 col
 otherwise, absolute columns for the rectangular transfer matrices; the layout the solver actually
 uploads is the same function of the same inputs."""
 import numpy as np
+import pytest
 
 from featb200 import assembly as AS
 from featb200.lafem import SparseMatrixCSR
@@ -58,3 +59,13 @@ def test_unsorted_row_keeps_the_stored_order(featlib):
     M = SparseMatrixCSR(rp, ci, v, A.shape)
     assert fb.storage_plan(M)["kind"] != "diagonal"
     assert fb.storage_plan(_csr(A))["kind"] == "diagonal"
+
+
+@pytest.mark.parametrize("level,kind", [(4, "ell"), (5, "diagonal")])
+def test_padding_limit(featlib, level, kind):
+    """27 / (interior share) per row: 45% padding at 4,913 rows, 20.6% at 35,937 (the limit is 25%)."""
+    A = AS.stiffness(level, 3)
+    p = featlib.storage_plan(_csr(A), AS.boundary_dofs(level, 3))
+    assert (p["kind"] == "diagonal") == (kind == "diagonal")
+    n, inner = 2 ** level + 1, 2 ** level - 1
+    assert (n ** 3 <= 1.25 * inner ** 3) == (kind == "diagonal")
