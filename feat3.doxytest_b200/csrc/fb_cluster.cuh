@@ -9,8 +9,8 @@
 // entries of other blocks through distributed shared memory, and passes are separated by a barrier
 // in the blocks' shared memory (ClBar).  What is left is latency: a pass is one or two rows' chain of
 // shared or distributed loads per thread and a barrier, 0.5 us to 2 us; a whole solve of 2D FP64 level
-// 5 (1,089 rows, 5 iterations) takes 232 us with host work and copies, 349 us as launched passes, and
-// level 7 (16,641 rows, 6 iterations) 502 us against 568 us.  One short loop runs a list of passes written by the host: the code
+// 5 (1,089 rows, 5 iterations) takes 205 us with host work, 370 us as launched passes, and level 7
+// (16,641 rows, 6 iterations) 416 us against 556 us.  One short loop runs a list of passes written by the host: the code
 // of a pass is fetched once per launch and reused, where the single-block tail's straight-line
 // sequence waits for instruction fetch.
 //
@@ -90,11 +90,18 @@ namespace fb
     ClPass pass[CL_PASSES];
   };
 
-  // the PCG's scalars between its phases (in registers they would be live across the V-cycle and
-  // leave its passes too few to keep a row's loads in flight: twice the time per pass)
+  // What the phases share through memory: the PCG's scalars, and what few instructions need.  In
+  // registers they would be live across the V-cycle and leave its passes too few: a row's loads no longer
+  // all in flight (twice the time per pass), or spills, whose stores every barrier's release then waits
+  // for (1,000 cycles more per barrier; level 7 FP64, one solve: 470 -> 416 us without).
   struct ClState
   {
     double d0, dc, scale, gamma, gamma_prev, alpha, beta;
+    const unsigned char* gimg;            // this block's image in global memory
+    int* err;
+    uint32_t staged, img;                 // bytes of it staged in shared memory, and where
+    double *x, *hist;                     // whole solves: the iterate, the defect history
+    const Scalars* sc;
     int it, status;
   };
 
@@ -141,11 +148,10 @@ namespace fb
   // and all blocks' are returned.
   struct ClBar
   {
-    uint32_t n = 0;       // barriers passed
-    bool lost = false;    // a wait expired: no further ones (the error word is set)
+    // barriers passed; the top bit: a wait expired, no further ones (the error word is set)
+    uint32_t n = 0;
     template<bool NORM>
-    __device__ __forceinline__ uint32_t sync(unsigned char* sm, uint32_t me, uint32_t cs, uint32_t f, uint32_t turn,
-      int* err)
+    __device__ __forceinline__ uint32_t sync(unsigned char* sm, uint32_t me, uint32_t cs, uint32_t f, uint32_t turn)
     {
       volatile uint32_t* word = reinterpret_cast<volatile uint32_t*>(sm + CL_FLAGS + turn * 4u);
       if(NORM)
@@ -167,10 +173,10 @@ namespace fb
                      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [r];\n\t}"
                      :: "r"(bar), "r"(threadIdx.x) : "memory");
       }
-      if(!lost && !cl_wait(bar, (n >> 1) & 1u))
+      if(!(n >> 31) && !cl_wait(bar, (n >> 1) & 1u))
       {
-        lost = true;
-        *err = 1;
+        n |= 1u << 31;
+        *reinterpret_cast<ClState*>(sm + CL_STATE)->err = 1;
       }
       ++n;
       if(!NORM)
@@ -312,8 +318,8 @@ namespace fb
   // or not).  Returns the norm flags of this thread's rows: 1 an entry above CL_BIG, 2 one above
   // CL_HUGE.
   template<typename V, typename S, int U, bool LOCAL>
-  __device__ __forceinline__ uint32_t cl_rows(const uint4& d0, const uint4& d1, unsigned char* sm,
-    const unsigned char* gimg, uint32_t img, uint32_t staged, uint32_t nl, uint32_t me, bool skip)
+  __device__ __forceinline__ uint32_t cl_rows(const uint4& d0, const uint4& d1, unsigned char* sm, uint32_t img,
+    uint32_t nl, uint32_t me, bool skip)
   {
     const uint32_t fl = d0.x & 0xffffu, K = d0.x >> 16, ns = d0.z & 0xffffu;
     const S* dinv = reinterpret_cast<const S*>(sm + img + (d0.z >> 16) * 16u);
@@ -329,15 +335,31 @@ namespace fb
     uint32_t f = 0;
     for(uint32_t i = threadIdx.x; i < nl; i += CL_NT)
     {
-      const bool d = dm[i] != 0;
-      const S di = dinv[i], bi = vb[i], c1 = v1[i], c2 = v2[i];
+      // (the row's own entries: ahead of the sum in FP32, behind it in FP64, whose sum takes the registers)
+      bool d;
+      S di, bi, c1, c2;
+      auto own_entries = [&]()
+      {
+        d = dm[i] != 0;
+        di = dinv[i];
+        bi = vb[i];
+        c1 = v1[i];
+        c2 = v2[i];
+      };
+      if(sizeof(S) == 4)
+        own_entries();
       S s;
       if constexpr(U == 0)
-        s = cl_row<V, S>(reinterpret_cast<const V*>((vo_ < staged ? sm + img : gimg) + vo_) + i,
-                         reinterpret_cast<const uint16_t*>((co_ < staged ? sm + img : gimg) + co_) + i, ns, K, ga);
+      {
+        const ClState& st = *reinterpret_cast<const ClState*>(sm + CL_STATE);
+        s = cl_row<V, S>(reinterpret_cast<const V*>((vo_ < st.staged ? sm + img : st.gimg) + vo_) + i,
+                         reinterpret_cast<const uint16_t*>((co_ < st.staged ? sm + img : st.gimg) + co_) + i, ns, K, ga);
+      }
       else
         s = cl_rowu<V, S, U, LOCAL>(reinterpret_cast<const V*>(sm + img + vo_) + i,
                                     reinterpret_cast<const uint16_t*>(sm + img + co_) + i, ns, K, ga, gv, me << 12);
+      if(sizeof(S) == 8)
+        own_entries();
       const S u = d ? S(0) : ((fl & CLF_B) ? sub(bi, s) : add(s, S(0)));
       const S w = d ? S(0) : mul(di, u);
       S v = (fl & CLF_W) ? w : u;
@@ -366,15 +388,14 @@ namespace fb
   }
 
   // The passes of one V-cycle.  `ext`: the top level's skip flag.  Not inlined: inside the solve kernel
-  // its loop would share the registers of the PCG's state and run from spilled copies (twice the time).
+  // its loop would share registers with the calls around it and spill.
   template<typename V, typename S>
-  __device__ __noinline__ ClBar cl_vcycle(const unsigned char* gimg, uint32_t img, uint32_t staged, uint32_t me, bool ext,
-    ClBar bar, int* err)
+  __device__ __noinline__ ClBar cl_vcycle(bool ext, ClBar bar)
   {
     extern __shared__ __align__(128) unsigned char cl_sm[];
     unsigned char* const sm = cl_sm;
     const ClParams& cp = *reinterpret_cast<const ClParams*>(cl_sm);
-    const uint32_t cs = uint32_t(cp.cs);
+    const uint32_t cs = uint32_t(cp.cs), me = cl_rank(), img = reinterpret_cast<const ClState*>(sm + CL_STATE)->img;
     const bool last = me == cs - 1u;
     double* part = reinterpret_cast<double*>(sm + CL_PART);
     const uint32_t base = cl_smem(sm);
@@ -398,7 +419,7 @@ namespace fb
         pc = cp.small_end;
         if(pc + 1 < np)
           d0 = dp[2 * (pc + 1)];
-        bar.sync<false>(sm, me, cs, 0u, 0u, err);
+        bar.sync<false>(sm, me, cs, 0u, 0u);
         continue;
       }
       const uint32_t r0 = small ? 0u : me * rpc;
@@ -427,13 +448,13 @@ namespace fb
         vout = (d1.z >> 16) * 16u;
         const bool sk = (fl & CLF_SKIP_EXT) ? ext : ((fl & CLF_SKIP) ? skip : false);
         if(fl & CLF_U9)
-          f = (fl & CLF_LOCAL) ? cl_rows<V, S, 9, true>(d, d1, sm, gimg, img, staged, nl, me, sk)
-                               : cl_rows<V, S, 9, false>(d, d1, sm, gimg, img, staged, nl, me, sk);
+          f = (fl & CLF_LOCAL) ? cl_rows<V, S, 9, true>(d, d1, sm, img, nl, me, sk)
+                               : cl_rows<V, S, 9, false>(d, d1, sm, img, nl, me, sk);
         else if(fl & CLF_U4)
-          f = (fl & CLF_LOCAL) ? cl_rows<V, S, 4, true>(d, d1, sm, gimg, img, staged, nl, me, sk)
-                               : cl_rows<V, S, 4, false>(d, d1, sm, gimg, img, staged, nl, me, sk);
+          f = (fl & CLF_LOCAL) ? cl_rows<V, S, 4, true>(d, d1, sm, img, nl, me, sk)
+                               : cl_rows<V, S, 4, false>(d, d1, sm, img, nl, me, sk);
         else
-          f = cl_rows<V, S, 0, false>(d, d1, sm, gimg, img, staged, nl, me, sk);
+          f = cl_rows<V, S, 0, false>(d, d1, sm, img, nl, me, sk);
       }
       // the next pass's word: its latency runs beside the barrier's
       if(pc + 1 < np)
@@ -443,11 +464,11 @@ namespace fb
         if(small && !(fl & CLF_CLUSTER))
           cl_small_sync();
         else
-          bar.sync<false>(sm, me, cs, 0u, 0u, err);
+          bar.sync<false>(sm, me, cs, 0u, 0u);
       }
       else if(!small)
       {
-        const uint32_t all = bar.sync<true>(sm, me, cs, f, turn, err);
+        const uint32_t all = bar.sync<true>(sm, me, cs, f, turn);
         turn ^= 1u;
         const bool big = (all & 1u) != 0u, huge = (all & 2u) != 0u;
         skip = false;
@@ -460,9 +481,9 @@ namespace fb
           for(uint32_t i = threadIdx.x; i < nl; i += CL_NT)
             sq += double(u[i]) * double(u[i]);
           cl_put(base + CL_PART, sq, me, cs);
-          bar.sync<false>(sm, me, cs, 0u, 0u, err);
+          bar.sync<false>(sm, me, cs, 0u, 0u);
           skip = skip_from_norm<S>(sqrt(cl_total(part, 0u, cs * CL_NW))) != 0;
-          bar.sync<false>(sm, me, cs, 0u, 0u, err);
+          bar.sync<false>(sm, me, cs, 0u, 0u);
         }
       }
       else
@@ -485,7 +506,7 @@ namespace fb
           cl_small_sync();
         }
         if(fl & CLF_CLUSTER)
-          bar.sync<false>(sm, me, cs, 0u, 0u, err);
+          bar.sync<false>(sm, me, cs, 0u, 0u);
       }
     }
     return bar;
@@ -518,7 +539,14 @@ namespace fb
         reinterpret_cast<uint32_t*>(sm)[k] = __ldg(reinterpret_cast<const uint32_t*>(gp) + k);
     }
     if(threadIdx.x == 0)
+    {
       *reinterpret_cast<volatile int*>(sm + CL_HUGE) = 0;
+      ClState& st = *reinterpret_cast<ClState*>(sm + CL_STATE);
+      st.gimg = gimg;
+      st.staged = staged;
+      st.img = img_off;
+      st.err = err;
+    }
     __syncthreads();
     pdl_wait();
     if(!after_wait())
@@ -595,7 +623,7 @@ namespace fb
          return true;
        }))
       return;
-    cl_vcycle<V, S>(gimg, img_off, staged, me, ext, ClBar(), err);
+    cl_vcycle<V, S>(ext, ClBar());
     const S* o = reinterpret_cast<const S*>(cl_sm + cp.vout);
     for(uint32_t i = threadIdx.x; i < nl; i += CL_NT)
       gout[r0 + i] = o[i];
@@ -620,9 +648,9 @@ namespace fb
     const double *a64, *part;
     const uint16_t* acode;
 
-    __device__ __forceinline__ ClPcg(unsigned char* s, const unsigned char* gimg, uint32_t im, uint32_t staged, uint32_t m)
-      : sm(s), cp(*reinterpret_cast<const ClParams*>(s)), st(*reinterpret_cast<volatile ClState*>(s + CL_STATE)), me(m),
-        cs(uint32_t(cp.cs)), img(im)
+    __device__ __forceinline__ explicit ClPcg(unsigned char* s)
+      : sm(s), cp(*reinterpret_cast<const ClParams*>(s)), st(*reinterpret_cast<volatile ClState*>(s + CL_STATE)), me(cl_rank()),
+        cs(uint32_t(cp.cs)), img(st.img)
     {
       const bool last = me == cs - 1u;
       plo = cp.top_small ? (cs - 1u) * CL_NW : 0u;
@@ -639,7 +667,7 @@ namespace fb
       vr = reinterpret_cast<double*>(s + cp.vr);
       dinv = reinterpret_cast<const S*>(s + img + cp.dinv);
       dm = s + img + cp.dm;
-      a64 = reinterpret_cast<const double*>((cp.a64 < staged ? s + img : gimg) + cp.a64);
+      a64 = reinterpret_cast<const double*>((cp.a64 < st.staged ? s + img : st.gimg) + cp.a64);
       acode = reinterpret_cast<const uint16_t*>(s + img + cp.acode);
       part = reinterpret_cast<const double*>(s + CL_PART);
     }
@@ -665,14 +693,15 @@ namespace fb
 
   // r = F(rhs - A x), ||r||, the first V-cycle's input (iterative.hpp:748-771)
   template<typename V, typename S>
-  __device__ __noinline__ ClBar cl_pcg_init(const unsigned char* gimg, uint32_t img, uint32_t staged, uint32_t me,
-    const double* gx, const double* rhs, double* __restrict__ hist, ClBar bar, int* err)
+  __device__ __noinline__ ClBar cl_pcg_init(const double* rhs, ClBar bar)
   {
     extern __shared__ __align__(128) unsigned char cl_sm[];
-    const ClPcg<V, S> w(cl_sm, gimg, img, staged, me);
+    const ClPcg<V, S> w(cl_sm);
+    const uint32_t me = w.me;
+    const double* gx = w.st.x;
     for(uint32_t i = threadIdx.x; i < w.nl; i += CL_NT)
       w.vp[i] = gx[w.r0 + i];
-    bar.sync<false>(cl_sm, me, w.cs, 0u, 0u, err);
+    bar.sync<false>(cl_sm, me, w.cs, 0u, 0u);
     double sq = 0.0;
     for(uint32_t i = threadIdx.x; i < w.nl; i += CL_NT)
     {
@@ -687,7 +716,7 @@ namespace fb
     }
     if(w.mine)
       cl_put(w.base + CL_PART, sq, me, w.cs);
-    bar.sync<false>(cl_sm, me, w.cs, 0u, 0u, err);
+    bar.sync<false>(cl_sm, me, w.cs, 0u, 0u);
     const double d0 = sqrt(cl_total(w.part, w.plo, w.pcnt));
     int status = FB_SOLVER_PROGRESS;
     if(!isfinite(d0))
@@ -713,20 +742,21 @@ namespace fb
       w.st.it = 0;
       w.st.status = status;
       if(me == 0u)
-        hist[0] = d0;
+        w.st.hist[0] = d0;
     }
     // every block has read the partial sums and p before the next pass writes them
-    bar.sync<false>(cl_sm, me, w.cs, 0u, 0u, err);
+    bar.sync<false>(cl_sm, me, w.cs, 0u, 0u);
     return bar;
   }
 
   // The PCG iteration after the V-cycle, up to the next V-cycle's input
   template<typename V, typename S>
-  __device__ __noinline__ ClBar cl_pcg_step(const unsigned char* gimg, uint32_t img, uint32_t staged, uint32_t me,
-    double* gx, double* __restrict__ hist, const Scalars* __restrict__ sc, ClBar bar, int* err)
+  __device__ __noinline__ ClBar cl_pcg_step(ClBar bar)
   {
     extern __shared__ __align__(128) unsigned char cl_sm[];
-    const ClPcg<V, S> w(cl_sm, gimg, img, staged, me);
+    const ClPcg<V, S> w(cl_sm);
+    const uint32_t me = w.me;
+    double* gx = w.st.x;
     // z = x_top / scale (FP64), r.z -> beta; p = z + beta p
     const int it = w.st.it;
     const double dc0 = w.st.dc, gamma_prev = w.st.gamma, inv_scale = 1.0 / w.st.scale;
@@ -735,7 +765,7 @@ namespace fb
       rz += mul(w.vr[i], mul(double(w.vz[i]), inv_scale));
     if(w.mine)
       cl_put(w.base + CL_PART, rz, me, w.cs);
-    bar.sync<false>(cl_sm, me, w.cs, 0u, 0u, err);
+    bar.sync<false>(cl_sm, me, w.cs, 0u, 0u);
     const double gamma = cl_total(w.part, w.plo, w.pcnt);
     const double beta = gamma / gamma_prev;
     for(uint32_t i = threadIdx.x; i < w.nl; i += CL_NT)
@@ -743,7 +773,7 @@ namespace fb
       const double z = mul(double(w.vz[i]), inv_scale);
       w.vp[i] = it == 0 ? z : add(mul(w.vp[i], beta), z);
     }
-    bar.sync<false>(cl_sm, me, w.cs, 0u, 0u, err);
+    bar.sync<false>(cl_sm, me, w.cs, 0u, 0u);
     // q = F(A p), q.p -> alpha
     double qp = 0.0;
     for(uint32_t i = threadIdx.x; i < w.nl; i += CL_NT)
@@ -755,7 +785,7 @@ namespace fb
     }
     if(w.mine)
       cl_put(w.base + CL_PART + CL_PARTS, qp, me, w.cs);
-    bar.sync<false>(cl_sm, me, w.cs, 0u, 0u, err);
+    bar.sync<false>(cl_sm, me, w.cs, 0u, 0u);
     const double alpha = gamma / cl_total(w.part + CL_PARTS / 8u, w.plo, w.pcnt);
     // x += alpha p; r -= alpha q; ||r||; the next V-cycle's input
     const double nscale = w.F64 ? 1.0 : pow2_near_inverse(dc0);
@@ -770,11 +800,12 @@ namespace fb
     }
     if(w.mine)
       cl_put(w.base + CL_PART, rr, me, w.cs);   // (every block has read r.z: barriers lie between)
-    bar.sync<false>(cl_sm, me, w.cs, 0u, 0u, err);
+    bar.sync<false>(cl_sm, me, w.cs, 0u, 0u);
     const double dc = sqrt(cl_total(w.part, w.plo, w.pcnt));
     if(threadIdx.x == 0)
     {
       const double d0 = w.st.d0;
+      const Scalars* sc = w.st.sc;
       int status = FB_SOLVER_PROGRESS;
       if(!isfinite(dc))
         status = FB_SOLVER_ABORTED;
@@ -795,7 +826,7 @@ namespace fb
       w.st.it = it + 1;
       w.st.status = status;
       if(me == 0u)
-        hist[it + 1] = dc;
+        w.st.hist[it + 1] = dc;
     }
     __syncthreads();
     return bar;
@@ -817,11 +848,18 @@ namespace fb
     if(!cl_start(gp, cl_sm, me, cs, img, staged, gimg, err, [] { return true; }))
       return;
     volatile ClState& st = *reinterpret_cast<volatile ClState*>(cl_sm + CL_STATE);
-    ClBar bar = cl_pcg_init<V, S>(gimg, img, staged, me, gx, rhs, hist, ClBar(), err);
+    if(threadIdx.x == 0)
+    {
+      st.x = gx;
+      st.hist = hist;
+      st.sc = sc;
+    }
+    __syncthreads();
+    ClBar bar = cl_pcg_init<V, S>(rhs, ClBar());
     while(st.status == FB_SOLVER_PROGRESS)
     {
-      bar = cl_vcycle<V, S>(gimg, img, staged, me, skip_from_norm<S>(st.dc * st.scale) != 0, bar, err);
-      bar = cl_pcg_step<V, S>(gimg, img, staged, me, gx, hist, sc, bar, err);
+      bar = cl_vcycle<V, S>(skip_from_norm<S>(st.dc * st.scale) != 0, bar);
+      bar = cl_pcg_step<V, S>(bar);
     }
     cl_sync();   // no block leaves while another may still arrive at its barriers; all have read *sc
     if(threadIdx.x == 0 && me == 0u)
