@@ -26,6 +26,7 @@
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <tuple>
 #include <vector>
 
 namespace fb
@@ -1319,48 +1320,32 @@ namespace bt
 
   constexpr uint32_t STAGED_ROWS = 1000;   // matrices of at least this many rows take the staged passes
 
-  // resident blocks per SM of a staged-pass kernel with `smem` bytes of dynamic shared memory
-  static uint32_t staged_resident(const void* kern, size_t smem)
+  // Resident blocks per SM of a staged-pass kernel with `smem` bytes of dynamic shared memory.  The one
+  // way to its grid, so it also raises the kernel's 48 KB limit on this device.
+  static cudaError_t staged_resident(const void* kern, size_t smem, uint32_t& blocks)
   {
     static std::mutex mu;
-    static std::map<std::pair<const void*, size_t>, uint32_t> cache;
+    static std::map<std::tuple<int, const void*, size_t>, uint32_t> cache;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if(e != cudaSuccess)
+      return e;
     std::lock_guard<std::mutex> g(mu);
-    const auto key = std::make_pair(kern, smem);
+    const auto key = std::make_tuple(dev, kern, smem);
     const auto it = cache.find(key);
     if(it != cache.end())
-      return it->second;
-    int nb = 0;
-    if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, TMA_NT, smem) != cudaSuccess || nb < 1)
     {
-      (void)cudaGetLastError();
-      nb = 1;
+      blocks = it->second;
+      return cudaSuccess;
     }
-    cache[key] = uint32_t(nb);
-    return uint32_t(nb);
-  }
-
-  // dynamic shared memory above 48 KB for every staged-pass instance the batch may launch
-  template<typename V, typename S, class Op>
-  static fb_status staged_attr()
-  {
-    const int mx = int(TMA_SMEM_MAX) + 8 * 1024;
-    FB_CUDA(cudaFuncSetAttribute(k_tma_pass<V, S, Op, 9, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    FB_CUDA(cudaFuncSetAttribute(k_tma_pass<V, S, Op, 9>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    FB_CUDA(cudaFuncSetAttribute(k_tma_pass<V, S, Op, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    return FB_OK;
-  }
-  template<typename V, typename S>
-  static fb_status staged_attrs()
-  {
-    BT_TRY((staged_attr<V, S, BOpSmooth<V, S>>()));
-    BT_TRY((staged_attr<V, S, BOpDefect<V, S>>()));
-    BT_TRY((staged_attr<V, S, BOpProlong<V, S>>()));
-    BT_TRY((staged_attr<V, S, BOpPost1<V, S>>()));
-    BT_TRY((staged_attr<V, S, BOpPost2<V, S, true>>()));
-    BT_TRY((staged_attr<V, S, BOpPost2<V, S, false>>()));
-    BT_TRY((staged_attr<V, S, BOpRestrict<V, S>>()));
-    BT_TRY((staged_attr<double, double, BOpPcgQ>()));
-    return FB_OK;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TMA_SMEM_MAX) + 8 * 1024);
+    int nb = 0;
+    if(e == cudaSuccess)
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, TMA_NT, smem);
+    if(e != cudaSuccess)
+      return e;
+    blocks = cache[key] = uint32_t(std::max(nb, 1));
+    return cudaSuccess;
   }
 
   template<typename V> DCsr<V> bview(const fb_batch::Mat& m)
@@ -1379,6 +1364,7 @@ namespace bt
     bool dry;
     uint64_t launches = 0;
     double bytes = 0;
+    cudaError_t err = cudaSuccess;   // the first staged pass that cannot be launched
 
     // the PCG-space kernels' grid: one wave of their resident blocks per SM (launch bounds)
     unsigned int one_wave(uint32_t n, unsigned bps = 4) const
@@ -1423,9 +1409,13 @@ namespace bt
       const uint32_t nch = (m.rows + TMA_NT - 1) / TMA_NT;
       auto launch = [&](auto kern, size_t sm)
       {
-        const uint32_t grid = std::max(1u, std::min(nch, uint32_t(s->nsm) * staged_resident((const void*)kern, sm)));
-        if(query_only)
+        uint32_t resident = 0;
+        const cudaError_t e = staged_resident((const void*)kern, sm, resident);
+        if(e != cudaSuccess && err == cudaSuccess)
+          err = e;
+        if(e != cudaSuccess || query_only)
           return;
+        const uint32_t grid = std::max(1u, std::min(nch, uint32_t(s->nsm) * resident));
         kern<<<grid, TMA_NT, sm, st>>>(bview<VV>(m), static_cast<const XS*>(x), m.rows, m.kmax, nullptr, 0u, 0u, 0,
           op, RedSlot{nullptr, nullptr}, s->err);
       };
@@ -1461,6 +1451,8 @@ namespace bt
         BLaunch<double, double> d64{s, st, false};
         d64.template tma<double, double>(s->Atop, nullptr, BOpPcgInit{}, true);
         d64.template tma<double, double>(s->Atop, nullptr, BOpPcgQ{}, true);
+        if(err == cudaSuccess)
+          err = d64.err;
       }
     }
 
@@ -1702,7 +1694,6 @@ namespace bt
   static fb_status build(fb_batch* s)
   {
     cudaStream_t st = s->stream;
-    BT_TRY((staged_attrs<V, S>()));
     if(s->cfg.rows_per_block > 0)
       for(auto& g : s->g)
         g.bs = std::max(32, std::min(BNT_MAX, (s->cfg.rows_per_block + 31) / 32 * 32));
@@ -1715,6 +1706,7 @@ namespace bt
     {
       BLaunch<V, S> a{s, st, true};
       a.prime();
+      FB_CUDA(a.err);
       a.init();
       a.vcycle();
       a.tail(true, 0);
@@ -1731,12 +1723,15 @@ namespace bt
     FB_CUDA(cudaGraphCreate(&s->graph, 0));
     cudaGraphConditionalHandle cond;
     FB_CUDA(cudaGraphConditionalHandleCreate(&cond, s->graph, 0u, cudaGraphCondAssignDefault));
+    (void)cudaGetLastError();   // what callers left; a launch that capture refuses is this build's error
+    cudaError_t launched = cudaSuccess;
     FB_CUDA(cudaStreamBeginCaptureToGraph(st, s->graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     {
       BLaunch<V, S> a{s, st, false};
       a.init();
       a.vcycle();
       a.tail(true, cond);
+      launched = cudaGetLastError();
     }
     cudaStreamCaptureStatus cst;
     const cudaGraphNode_t* deps = nullptr;
@@ -1753,15 +1748,18 @@ namespace bt
     FB_CUDA(cudaStreamUpdateCaptureDependencies(st, &cnode, 1, cudaStreamSetCaptureDependencies));
     cudaGraph_t g_out = nullptr;
     FB_CUDA(cudaStreamEndCapture(st, &g_out));
+    FB_CUDA(launched);
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     FB_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     {
       BLaunch<V, S> b{s, st, false};
       b.vcycle();
       b.tail(false, cond);
+      launched = cudaGetLastError();
     }
     cudaGraph_t b_out = nullptr;
     FB_CUDA(cudaStreamEndCapture(st, &b_out));
+    FB_CUDA(launched);
     FB_CUDA(cudaGraphInstantiate(&s->gexec, s->graph, 0));
     return FB_OK;
   }

@@ -154,3 +154,72 @@ def test_batch_bottom_kernel(featlib, cuda, levels, ordering, precision, steps):
         assert bat.iterations()[k] == single[L][1]
         # the order of the PCG's sums differs
         assert rel_err(X[k], single[L][0]) <= (1e-12 if precision == "f64" else 1e-9)
+
+def _coarse_first(levels, dim=2):
+    """The hierarchy with every mesh's vertices numbered coarse vertices first: no level is lexicographic, and
+    from 2D level 8 on column offsets leave the 16-bit range."""
+    import featb200 as fb
+
+    def order(level):
+        idx = np.indices((2 ** level + 1,) * dim).reshape(dim, -1)
+        age = np.zeros(idx.shape[1], dtype=np.int64)
+        for lv in range(level):
+            age += np.any(idx % (1 << (level - lv)) != 0, axis=0)
+        return np.argsort(age, kind="stable")
+
+    def permuted(m, rows, cols):
+        return fb.SparseMatrixCSR.from_scipy(m.to_scipy()[rows][:, cols])
+
+    out = []
+    for d in levels:
+        o = order(d["level"])
+        place = np.argsort(o).astype(np.uint64)
+        e = {"matrix": permuted(d["matrix"], o, o), "level": d["level"],
+             "filter": fb.UnitFilter(np.sort(place[d["filter"].indices.astype(np.int64)]))}
+        if "transfer" in d:
+            c = order(d["level"] - 1)
+            e["transfer"] = fb.Transfer(permuted(d["transfer"].get_mat_prol(), o, c),
+                                        permuted(d["transfer"].get_mat_rest(), c, o))
+        out.append(e)
+    return out, order(levels[0]["level"])
+
+
+def _widened(levels, c=0.05):
+    """A + c A A on every level (boundary rows and columns of the product zero): 25 entries per interior row."""
+    import scipy.sparse as sp
+    import featb200 as fb
+    out = []
+    for d in levels:
+        A = d["matrix"].to_scipy().tocsr()
+        inner = np.ones(A.shape[0])
+        inner[d["filter"].indices.astype(np.int64)] = 0.0
+        A0 = sp.diags(inner) @ A @ sp.diags(inner)
+        W = (A + c * (A0 @ A0)).tocsr()
+        W.sort_indices()
+        out.append(dict(d, matrix=fb.SparseMatrixCSR.from_scipy(W)))
+    return out
+
+
+# top matrices whose staged start needs more than 48 KB of shared memory: nine entries with 32-bit columns
+# (55,296 bytes), and rows of up to 25 entries with 16-bit ones
+@pytest.mark.parametrize("level,wide", [(8, False), (6, True)])
+@pytest.mark.parametrize("use_graph", [True, False])
+def test_batch_large_staged_start(featlib, cuda, level, wide, use_graph):
+    """Instances numbered coarse vertices first match their single solves."""
+    from featb200 import assembly as AS
+    fb = featlib
+    lex, b = AS.poisson_hierarchy(level, 2, rhs="gauss", gauss=AS.gauss_params(level, 2))
+    levels, o = _coarse_first(_widened(lex) if wide else lex)
+    b = b[o]
+    plan = fb.storage_plan(levels[0]["matrix"], levels[0]["filter"].indices)
+    assert plan["kind"] != "diagonal" and plan["narrow"] == wide and plan["width"] == (25 if wide else 9), plan
+    s = fb.build_pcg_multigrid(levels)
+    x = fb.DenseVector(b.size)
+    assert fb.solve(s, x, fb.DenseVector(b)) == fb.Status.success
+    h = fb.build_hierarchy(levels)
+    bat = fb.BatchPCG([h, h], use_graph=use_graph)
+    X = bat.split(bat.solve(np.zeros(2 * b.size), np.concatenate([b, b])))
+    for k in range(2):
+        assert bat.statuses()[k] == fb.Status.success
+        assert bat.iterations()[k] == s.get_num_iter()
+        assert rel_err(X[k], x.elements) <= 1e-12
