@@ -344,6 +344,11 @@ namespace un
     }
     const uint32_t brow = smem_addr(sw) + uint32_t((lane & 15) * BST + (lane >> 4) * 8) * 2;
     const int half = lane >> 4;
+    // what the missing tenth tap of eight channels reads: zeros, since its zero weights would turn an
+    // infinite pixel into NaN
+    __shared__ __align__(16) uint4 zeros;
+    if(C == 8 && tid == 0)
+      zeros = make_uint4(0u, 0u, 0u, 0u);
 
     // the weights that stay are fetched before the wait for the kernel ahead: no kernel that is followed
     // by a convolution directly writes them
@@ -372,13 +377,13 @@ namespace un
           #pragma unroll
           for(int e = 0; e < 4; ++e)
             acc[i][j][e] = 0.f;
-      // one 16-deep step: A chunks at aoff (bytes), B rows at boff (bytes)
-      auto step = [&](uint32_t aoff, uint32_t boff)
+      // one 16-deep step: A chunks at aoff (bytes), B rows at boff (bytes); zero: this lane's are zeros
+      auto step = [&](uint32_t aoff, uint32_t boff, bool zero = false)
       {
         uint32_t af[2][4];
         #pragma unroll
         for(int mt = 0; mt < 2; ++mt)
-          ldm_x4a(af[mt], arow[mt] + aoff);
+          ldm_x4a(af[mt], zero ? smem_addr(&zeros) : arow[mt] + aoff);
         #pragma unroll
         for(int j = 0; j < NT8; j += 2)
         {
@@ -413,7 +418,7 @@ namespace un
         {
           const int q0 = 2 * s, q1 = 2 * s + 1 < 9 ? 2 * s + 1 : 0;
           const int o0 = (q0 / 3 * HD + q0 % 3) * DIL * PXC * 16, o1 = (q1 / 3 * HD + q1 % 3) * DIL * PXC * 16;
-          step(uint32_t(half ? o1 : o0), uint32_t(s * 16 * BST * 2));
+          step(uint32_t(half ? o1 : o0), uint32_t(s * 16 * BST * 2), s == 4 && half);
         }
       }
       else if constexpr(NST == 9)

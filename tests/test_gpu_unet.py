@@ -150,3 +150,28 @@ def test_rejects_bad_arguments(featlib, cuda):
     x = cuda.zeros((3, 2, 17, 17), dtype=cuda.float32, device="cuda")
     with pytest.raises(fb.FeatB200Error):
         net.forward(x)
+
+
+def _pass_through():
+    """Parameters that carry input channel 0 through tap (-1, -1) of the first layer, the skip connection and
+    the last two layers; every other weight is zero."""
+    W = [np.zeros((co, 9, ci), np.float32) for ci, co, *_ in UO.LAYERS]
+    W[0][0, 0, 0] = 1.0
+    W[8][0, 4, 32] = 1.0
+    W[9][0, 4, 0] = 1.0
+    return np.concatenate([np.concatenate([w.ravel(), np.zeros(w.shape[0], np.float32)]) for w in W])
+
+
+@pytest.mark.parametrize("G,y,x", [(17, 3, 4), (17, 8, 8), (33, 10, 21), (33, 31, 0)])
+def test_infinite_input_stays_infinite(featlib, cuda, G, y, x):
+    """An infinite pixel reaches its output pixel as infinity (no product with padding turns it into NaN, which
+    ReLU would turn into 0); its products with the last layer's zero weights are NaN, everything else 0."""
+    from featb200.unet import UNet
+    torch = cuda
+    inp = np.zeros((1, 2, G, G), np.float32)
+    inp[0, 0, y, x] = np.inf
+    out = UNet(G, 1, params=_pass_through()).forward(torch.tensor(inp, device="cuda")).cpu().numpy()[0]
+    want = np.zeros((G, G), np.float32)
+    want[y:y + 3, x:x + 3] = np.nan
+    want[y + 1, x + 1] = np.inf
+    assert np.array_equal(out, want, equal_nan=True)
