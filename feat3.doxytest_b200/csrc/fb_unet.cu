@@ -526,6 +526,8 @@ namespace un
   // read transposed by ldmatrix.trans from the staged tiles; warp w takes GPW groups of 16 columns
   // and all M rows, so a warp issues MT + GPW ldmatrix.x4 for 2 MT GPW MMAs.  Blocks are
   // persistent over tiles and write one partial each (FP32), which k_grad_reduce sums in block order.
+  // A slot outside the tile or the grid reads zeros for x too: its zero in dy would turn an infinite
+  // activation into NaN.
   struct WgradArgs
   {
     Input in;
@@ -562,13 +564,14 @@ namespace un
     bf* sx = reinterpret_cast<bf*>(smem);
     bf* sd = reinterpret_cast<bf*>(smem + halo_bytes(C, DIL));
     constexpr int STAGE = wgrad_stage<C, M, DIL>();
-    __shared__ int pxo[128];                        // halo offset (bytes) of each pixel slot
+    __shared__ int pxo[2][128];                     // halo offset (bytes) of each pixel slot, -1: none
+    __shared__ __align__(16) uint4 zeros;
     Input in = a.in;
     in.c0 += int(blockIdx.y) * C;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int T = a.t.T, G = a.t.G, nt = a.t.nt, TT = T * T;
-    for(int m = tid; m < 128; m += NT)
-      pxo[m] = m < TT ? (m / T * HD + m % T) * PXC * 16 : 0;
+    if(tid == 0)
+      zeros = make_uint4(0u, 0u, 0u, 0u);
     // byte offset of this lane's chunk of each column group (chunks past the end read chunk 0)
     uint32_t goff[GPW];
     #pragma unroll
@@ -601,6 +604,11 @@ namespace un
       const int b = tile / (nt * nt), r = tile - b * (nt * nt);
       const int y0 = r / nt * T, x0 = (r - r / nt * nt) * T;
       load_halo<C, DIL, IN, NT>(in, a.t, b, y0, x0, sx + buf * (STAGE / 2));
+      for(int m = tid; m < 128; m += NT)
+      {
+        const int ty = m / T, tx = m - ty * T;
+        pxo[buf][m] = m < TT && y0 + ty < G && x0 + tx < G ? (ty * HD + tx) * PXC * 16 + buf * STAGE : -1;
+      }
       for(int e = tid; e < 128 * (M / 8); e += NT)
       {
         const int ch = e % (M / 8), m = e / (M / 8);
@@ -636,16 +644,16 @@ namespace un
       }
       else
         cp_wait<0>();
-      __syncthreads();                              // (pxo written, the first time)
+      __syncthreads();
       const uint32_t so = uint32_t(buf * STAGE);
       #pragma unroll 2
       for(int k = 0; k < 8; ++k)
       {
-        const uint32_t px = uint32_t(pxo[k * 16 + (lane & 15)]) + so;
+        const int px = pxo[buf][k * 16 + (lane & 15)];
         uint32_t bfr[GPW][4];
         #pragma unroll
         for(int j = 0; j < GPW; ++j)
-          ldm_x4a_t(bfr[j], goff[j] + px);
+          ldm_x4a_t(bfr[j], px < 0 ? smem_addr(&zeros) : goff[j] + uint32_t(px));
         #pragma unroll
         for(int mt = 0; mt < MT; ++mt)
         {
@@ -1083,7 +1091,7 @@ namespace
   fb_status wgrad(fb_unet* u, int l, const void* dy, const Input& in, int B, cudaStream_t st)
   {
     constexpr int smem = wgrad_smem<C, M, DIL>();
-    if(smem > 48 * 1024 - 1024)
+    if(smem > 48 * 1024 - 2048)
       FB_CUDA(cudaFuncSetAttribute(k_wgrad<C, M, DIL, IN, SCALAR, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     WgradArgs a{};
     a.in = in;

@@ -175,3 +175,20 @@ def test_infinite_input_stays_infinite(featlib, cuda, G, y, x):
     want[y:y + 3, x:x + 3] = np.nan
     want[y + 1, x + 1] = np.inf
     assert np.array_equal(out, want, equal_nan=True)
+
+
+@pytest.mark.parametrize("G,y,x", [(9, 8, 3), (17, 16, 8), (17, 8, 16), (33, 0, 0), (33, 32, 32)])
+def test_infinite_input_reaches_its_own_weight_gradients(featlib, cuda, G, y, x):
+    """In the first layer only the taps that read the infinite pixel from a grid point get a gradient that is not
+    finite: pixel slots beside the grid, in the last tiles of a row, take no part."""
+    torch = cuda
+    net, theta, inp, tgt, _, tgt_d = _setup(torch, G, 1, seed=G)
+    inp[0, 0, y, x] = np.inf
+    net.forward(torch.tensor(inp, device="cuda"))
+    net.backward(tgt_d)
+    g = net.get_grads()[:16 * 9 * 2].reshape(16, 9, 2)
+    finite = np.ones((16, 9, 2), bool)
+    for tap in range(9):
+        py, px = y - (tap // 3 - 1), x - (tap % 3 - 1)
+        finite[:, tap, 0] = not (0 <= py < G and 0 <= px < G)
+    assert np.array_equal(np.isfinite(g), finite)
