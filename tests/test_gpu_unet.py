@@ -192,3 +192,28 @@ def test_infinite_input_reaches_its_own_weight_gradients(featlib, cuda, G, y, x)
         py, px = y - (tap // 3 - 1), x - (tap % 3 - 1)
         finite[:, tap, 0] = not (0 <= py < G and 0 <= px < G)
     assert np.array_equal(np.isfinite(g), finite)
+
+
+@pytest.mark.parametrize("G,B", [(129, 1), (33, 8)])
+def test_weight_gradient_sums(featlib, cuda, G, B):
+    """With unit weights on single taps every activation and masked gradient is exact, so a weight gradient's error
+    is that of its FP32 sum: one tile's eight 16-deep steps, then blocks in four groups.  For the 64 x 64 layers
+    that is less than one rounding, 2^-24 (sixteen steps in a row gave 1.2 to 1.6 times that)."""
+    from featb200.unet import UNet
+    torch = cuda
+    W = [np.zeros((co, 9, ci)) for ci, co, *_ in UO.LAYERS]
+    for w in W:
+        w[np.arange(w.shape[0]), 4, np.arange(w.shape[0]) % w.shape[2]] = 1.0
+    theta = np.concatenate([np.concatenate([w.ravel(), np.zeros(w.shape[0])]) for w in W])
+    rng = np.random.default_rng(G * 100 + B)
+    inp = rng.uniform(0.1, 2.0, (B, 2, G, G)).astype(np.float32)
+    dout = (rng.standard_normal((B, G, G)) + 0.3).astype(np.float32)
+    net = UNet(G, B, params=theta.astype(np.float32))
+    y = net.forward(torch.tensor(inp, device="cuda"))
+    net.backward(torch.tensor(dout, device="cuda"))
+    yo, cache = UO.forward(theta, inp, exact=False)
+    assert np.array_equal(y.cpu().numpy(), yo.astype(np.float32))
+    go = UO.backward(cache, dout.astype(np.float64), exact=False)
+    g = net.get_grads()
+    for sl in _layer_slices()[6:12:2]:
+        assert _rel(g[sl], go[sl]) <= 2.0 ** -24
