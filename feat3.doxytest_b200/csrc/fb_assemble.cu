@@ -14,6 +14,7 @@
 // needed and the result is deterministic.
 #include "fb_common.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <mutex>
 #include <vector>
@@ -600,7 +601,7 @@ fb_status fb_q1_assemble_2d(int level, int kmodes, const double* xi, const doubl
   const int N = 1 << level;
   const double h = 1.0 / N;
   cudaStream_t st = as_stream(stream);
-  const int K = values ? kmodes : 0, ng = rhs ? ngauss : 0;
+  const int K = values ? kmodes : 0, ng = rhs ? std::max(ngauss, 0) : 0;   // no sources for a count below 1
   // the tables: ex, hy [3N][K] complex, gx, gy [3N][ng]
   const size_t nt = 3 * size_t(N), bytes = nt * (size_t(K) * 2 * sizeof(double2) + size_t(ng) * 2 * sizeof(double));
   void* ws = nullptr;

@@ -456,7 +456,7 @@ fb_status fb_q1_pattern_2d(int level, uint64_t* nnz, uint64_t* row_ptr, uint64_t
  * kappa = exp(g), g(x,y) = s sum_{i,j<K} (xi[i*K+j] cos t + eta[i*K+j] sin t) / (kx_i^2 + ky_j^2),
  * t = 2 pi (kx_i x + ky_j y), kx_i = i - K/2, ky_j = j - K/2, the (0,0) mode left out; kmodes = 0
  * gives kappa = 1 (xi, eta unused).  f = sum_g a_g exp(-|x - c_g|^2 / (2 w_g^2)) with
- * gauss[4g..4g+3] = (c_x, c_y, w, a) (DEVICE array).  row_ptr: DEVICE copy of the pattern's row
+ * gauss[4g..4g+3] = (c_x, c_y, w, a) (DEVICE array; ngauss < 1: f = 0).  row_ptr: DEVICE copy of the pattern's row
  * pointer (needed with values).  values or rhs may be NULL. */
 fb_status fb_q1_assemble_2d(int level, int kmodes, const double* xi, const double* eta, double s, int ngauss,
                             const double* gauss, const uint64_t* row_ptr, double* values, double* rhs,

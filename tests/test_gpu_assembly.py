@@ -74,6 +74,32 @@ def test_assembly_modes_and_sources(featlib, cuda, level, modes, sources):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("modes", [0, 64])
+def test_assembly_without_sources(featlib, cuda, modes):
+    """A source count below 1 means none (fb_q1_assemble_2d): a zero load vector beside the usual values."""
+    import ctypes as C
+    torch = cuda
+    from featb200 import _lib
+    from featb200.assembly_gpu import Q1Assembler2D
+    asm = Q1Assembler2D(4)
+    fp = AS.field_params(5, modes) if modes else None
+    ref, _ = asm.assemble(fp, rhs=False)
+    xi, eta = ((torch.tensor(np.ascontiguousarray(f), device="cuda") for f in fp[2:4]) if modes else (None, None))
+    some = torch.ones(4, dtype=torch.float64, device="cuda")
+
+    def ptr(t):
+        return C.c_void_p(t.data_ptr()) if t is not None else None
+
+    for count in (0, -1, -(2 ** 31)):
+        vals = torch.full((asm.nnz,), 7.0, dtype=torch.float64, device="cuda")
+        b = torch.full((asm.n,), 7.0, dtype=torch.float64, device="cuda")
+        _lib.check(_lib.lib().fb_q1_assemble_2d(4, modes, ptr(xi), ptr(eta), float(fp[4]) if modes else 0.0, count,
+                                                ptr(some), ptr(asm.row_ptr_d), ptr(vals), ptr(b),
+                                                C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        assert torch.equal(vals, ref) and not b.any()
+
+
+@pytest.mark.gpu
 def test_assembly_values_only_and_rhs_only(featlib, cuda):
     torch = cuda
     from featb200.assembly_gpu import Q1Assembler2D
