@@ -118,8 +118,10 @@ namespace as
   // kappa-weighted 4x4 element matrix and the 4 load contributions, in shared memory), then one
   // thread per vertex (its stiffness row, sorted neighbours, and its load entry, cells in ascending
   // order).  The cells on a tile's rim are computed by up to four blocks (1.14 cells per vertex); in
-  // exchange the element matrices (33 MB at level 9) never leave the SM.
+  // exchange the element matrices (33 MB at level 9) never leave the SM.  TAB: gx, gy are the tables;
+  // otherwise gx is the list of Gaussians itself, evaluated per point.
   constexpr int AT = 15, AC = AT + 1;
+  template<bool TAB>
   __global__ void __launch_bounds__(AC * AC) k_assemble(int N, double h, int K, const double2* __restrict__ ex,
     const double2* __restrict__ hy, double s, int ng, const double* __restrict__ gx, const double* __restrict__ gy,
     const uint64_t* __restrict__ rp, double* __restrict__ vals, double* __restrict__ rhs)
@@ -174,20 +176,37 @@ namespace as
         if(rhs)
         {
           double fq[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-          const double* xr = gx + size_t(cx) * 3 * ng;
-          const double* yr = gy + size_t(cy) * 3 * ng;
-          for(int g = 0; g < ng; ++g)
+          if constexpr(TAB)
           {
-            double a[3], b[3];
-            #pragma unroll
-            for(int q = 0; q < 3; ++q)
+            const double* xr = gx + size_t(cx) * 3 * ng;
+            const double* yr = gy + size_t(cy) * 3 * ng;
+            for(int g = 0; g < ng; ++g)
             {
-              a[q] = __ldg(xr + q * ng + g);
-              b[q] = __ldg(yr + q * ng + g);
+              double a[3], b[3];
+              #pragma unroll
+              for(int q = 0; q < 3; ++q)
+              {
+                a[q] = __ldg(xr + q * ng + g);
+                b[q] = __ldg(yr + q * ng + g);
+              }
+              #pragma unroll
+              for(int q = 0; q < 9; ++q)
+                fq[q] += a[q / 3] * b[q % 3];
             }
-            #pragma unroll
-            for(int q = 0; q < 9; ++q)
-              fq[q] += a[q / 3] * b[q % 3];
+          }
+          else
+          {
+            for(int g = 0; g < ng; ++g)
+            {
+              const double w = gx[4 * g + 2];
+              #pragma unroll
+              for(int q = 0; q < 9; ++q)
+              {
+                const double dx = (double(cx) + (1.0 + c_ref.xq[q / 3]) / 2.0) * h - gx[4 * g + 0];
+                const double dy = (double(cy) + (1.0 + c_ref.xq[q % 3]) / 2.0) * h - gx[4 * g + 1];
+                fq[q] += gx[4 * g + 3] * exp(-(dx * dx + dy * dy) / (2.0 * w * w));
+              }
+            }
           }
           #pragma unroll
           for(int a = 0; a < 4; ++a)
@@ -602,8 +621,11 @@ fb_status fb_q1_assemble_2d(int level, int kmodes, const double* xi, const doubl
   const double h = 1.0 / N;
   cudaStream_t st = as_stream(stream);
   const int K = values ? kmodes : 0, ng = rhs ? std::max(ngauss, 0) : 0;   // no sources for a count below 1
-  // the tables: ex, hy [3N][K] complex, gx, gy [3N][ng]
-  const size_t nt = 3 * size_t(N), bytes = nt * (size_t(K) * 2 * sizeof(double2) + size_t(ng) * 2 * sizeof(double));
+  // the tables: ex, hy [3N][K] complex, and gx, gy [3N][ng] up to the workspace that is kept (level 9: 2,730
+  // Gaussians); more Gaussians are evaluated point by point, so that their number is not bound by memory
+  const size_t nt = 3 * size_t(N), gbytes = nt * size_t(ng) * 2 * sizeof(double);
+  const bool tab = gbytes <= as::POOL_KEEP;
+  const size_t bytes = nt * size_t(K) * 2 * sizeof(double2) + (tab ? gbytes : 0);
   void* ws = nullptr;
   double2 *ex = nullptr, *hy = nullptr;
   double *gx = nullptr, *gy = nullptr;
@@ -616,11 +638,17 @@ fb_status fb_q1_assemble_2d(int level, int kmodes, const double* xi, const doubl
     hy = ex + nt * size_t(K);
     gx = reinterpret_cast<double*>(hy + nt * size_t(K));
     gy = gx + nt * size_t(ng);
-    as::k_tables<<<unsigned((nt + as::FT_T - 1) / as::FT_T), 128, 0, st>>>(N, h, K, xi, eta, ex, hy, ng, gauss, gx, gy);
+    as::k_tables<<<unsigned((nt + as::FT_T - 1) / as::FT_T), 128, 0, st>>>(N, h, K, xi, eta, ex, hy, tab ? ng : 0, gauss,
+      gx, gy);
     FB_LAUNCHED(1);
   }
   const unsigned tiles = unsigned((N + as::AT) / as::AT);   // (N + 1) vertices per side
-  as::k_assemble<<<dim3(tiles, tiles), as::AC * as::AC, 0, st>>>(N, h, K, ex, hy, s, ng, gx, gy, row_ptr, values, rhs);
+  if(tab)
+    as::k_assemble<true><<<dim3(tiles, tiles), as::AC * as::AC, 0, st>>>(N, h, K, ex, hy, s, ng, gx, gy, row_ptr, values,
+      rhs);
+  else
+    as::k_assemble<false><<<dim3(tiles, tiles), as::AC * as::AC, 0, st>>>(N, h, K, ex, hy, s, ng, gauss, nullptr, row_ptr,
+      values, rhs);
   FB_LAUNCHED(1);
   if(ws)
     FB_CUDA(cudaFreeAsync(ws, st));

@@ -100,6 +100,22 @@ def test_assembly_without_sources(featlib, cuda, modes):
 
 
 @pytest.mark.gpu
+def test_assembly_of_very_many_sources(featlib, cuda):
+    """More Gaussians than tables are kept for (43,690 at level 5) are evaluated point by point: the sum of two
+    halves that are tabulated, to the rounding of sums of 44,000 terms."""
+    torch = cuda
+    from featb200.assembly_gpu import Q1Assembler2D
+    asm = Q1Assembler2D(5)
+    gp = AS.gauss_params(9, 2, 44000)
+    vals, b = asm.assemble(None, gp)
+    ref, b0 = asm.assemble(None, gp[:22000])
+    _, b1 = asm.assemble(None, gp[22000:], values=False)
+    mag = asm.assemble(None, np.column_stack([gp[:, :3], np.abs(gp[:, 3])])[:43000], values=False)[1]
+    assert torch.equal(vals, ref)
+    assert ((b - b0 - b1).abs() <= 1e-13 * mag).all()
+
+
+@pytest.mark.gpu
 def test_assembly_values_only_and_rhs_only(featlib, cuda):
     torch = cuda
     from featb200.assembly_gpu import Q1Assembler2D
