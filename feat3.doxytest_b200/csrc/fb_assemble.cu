@@ -432,13 +432,13 @@ namespace as
   // Stream-ordered workspace from a pool of the library's own per device.  The device's default pool
   // gives its memory back at every synchronisation, and assembly calls end with one: each call then
   // mapped and unmapped its workspace anew (5 ms of the 9 ms that assembling, updating and solving a
-  // level-9 instance took).  The pool keeps at most POOL_KEEP bytes; what a call needs beyond that is
-  // given back at its synchronisation.
+  // level-9 instance took).  The pool keeps at most POOL_KEEP bytes until fb_q1_trim; what a call needs
+  // beyond that is given back at its synchronisation.
   constexpr uint64_t POOL_KEEP = uint64_t(64) << 20;
+  static std::mutex pool_mu;
+  static cudaMemPool_t pools[64] = {};
   static fb_status workspace(void** p, size_t bytes, cudaStream_t st)
   {
-    static std::mutex mu;
-    static cudaMemPool_t pools[64] = {};
     int dev = 0;
     FB_CUDA(cudaGetDevice(&dev));
     if(dev < 0 || dev >= 64)
@@ -448,7 +448,7 @@ namespace as
     }
     cudaMemPool_t pool;
     {
-      std::lock_guard<std::mutex> lock(mu);
+      std::lock_guard<std::mutex> lock(pool_mu);
       if(!pools[dev])
       {
         cudaMemPoolProps props = {};
@@ -653,6 +653,15 @@ fb_status fb_q1_assemble_2d(int level, int kmodes, const double* xi, const doubl
   if(ws)
     FB_CUDA(cudaFreeAsync(ws, st));
   FB_CUDA(cudaStreamSynchronize(st));
+  return FB_OK;
+}
+
+fb_status fb_q1_trim(void)
+{
+  std::lock_guard<std::mutex> lock(as::pool_mu);
+  for(cudaMemPool_t p : as::pools)
+    if(p)
+      FB_CUDA(cudaMemPoolTrimTo(p, 0));
   return FB_OK;
 }
 

@@ -111,6 +111,7 @@ _PROTOS = {
     "fb_solver_set_tolerances": (I, [P, D, D]),
     "fb_q1_pattern_2d": (I, [I, P, P, P]),
     "fb_q1_assemble_2d": (I, [I, I, P, P, D, I, P, P, P, P, P]),
+    "fb_q1_trim": (I, []),
     "fb_q1_sample_2d": (I, [I, I, P, P, D, I, P, P, P, P]),
     "fb_q1_prolongation_2d": (I, [I, C.POINTER(C.c_uint64), P, P, P, P]),
     "fb_unet_create": (I, [C.POINTER(P), I, I]),

@@ -41,6 +41,12 @@ class Q1Assembler2D:
         self.device = device
         self.row_ptr_d = torch.tensor(self.row_ptr.astype(np.int64), device=device)
 
+    def __del__(self):
+        try:
+            _lib.lib().fb_q1_trim()   # the workspace kept between calls
+        except Exception:
+            pass
+
     def assemble(self, field=None, gauss=None, values=True, rhs=True, stream=None, out_values=None, out_rhs=None):
         """field: None (kappa = 1) or featb200.assembly.field_params(...) (kx, ky, xi, eta, s) or the
         same with xi, eta as CUDA tensors; gauss: [g, 4] rows (c_x, c_y, w, a) or None (f = 0)."""
@@ -169,6 +175,12 @@ class Q1Assembler3D:
         self.nnz = self.col_ind.size
         self.device = device
         self.row_ptr_d = torch.tensor(self.row_ptr.astype(np.int64), device=device)
+
+    def __del__(self):
+        try:
+            _lib.lib().fb_q1_trim()   # the workspace kept between calls
+        except Exception:
+            pass
 
     def assemble(self, gauss=None, values=True, rhs=True, stream=None):
         import torch

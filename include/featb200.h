@@ -462,6 +462,10 @@ fb_status fb_q1_assemble_2d(int level, int kmodes, const double* xi, const doubl
                             const double* gauss, const uint64_t* row_ptr, double* values, double* rhs,
                             void* stream);
 
+/* Gives back the device memory (at most 64 MB per device) that the assembly calls keep between calls as
+ * workspace.  Calls in flight keep theirs. */
+fb_status fb_q1_trim(void);
+
 /* The Q1 prolongation from level-1 to `level` (1 <= level <= 13) on the lexicographic vertices
  * (weights 1, 1/2, 1/4; entries in ascending coarse index), written into DEVICE arrays (row_ptr
  * (2^level+1)^2+1, col_ind and values nnz entries); with all three NULL only nnz is returned.  The

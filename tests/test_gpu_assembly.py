@@ -116,6 +116,29 @@ def test_assembly_of_very_many_sources(featlib, cuda):
 
 
 @pytest.mark.gpu
+def test_workspace_is_given_back(featlib, cuda):
+    """What the calls keep between them (here tables of 49 MB) goes back to the device with the assembler."""
+    torch = cuda
+    from featb200.assembly_gpu import Q1Assembler2D
+    gp = AS.gauss_params(3, 2, 2000)
+    other = Q1Assembler2D(3)
+    other.assemble(None, gp)
+    asm = Q1Assembler2D(9)
+    b = torch.empty(asm.n, dtype=torch.float64, device="cuda")
+    other.assemble(None, gp)
+    del other
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    asm.assemble(None, gp, values=False, out_rhs=b)
+    kept = before - torch.cuda.mem_get_info()[0]
+    asm.assemble(None, gp, values=False, out_rhs=b)
+    assert 32 << 20 <= kept <= 80 << 20                # kept for the next call, which needs no more
+    assert before - torch.cuda.mem_get_info()[0] == kept
+    del asm
+    assert before - torch.cuda.mem_get_info()[0] <= 0
+
+
+@pytest.mark.gpu
 def test_assembly_values_only_and_rhs_only(featlib, cuda):
     torch = cuda
     from featb200.assembly_gpu import Q1Assembler2D
