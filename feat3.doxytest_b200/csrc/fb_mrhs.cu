@@ -8,8 +8,8 @@
 // (K/32 per lane): the row's entries are read once, coalesced, and broadcast by shuffles, and every
 // gather of x[col][0..K) is one coalesced K*sizeof(S) access -- the matrix traffic is shared by all
 // right-hand sides (the reference's multi-vector CSR kernel, apply.cu:109-135, covers K <= 3).
-// System matrices of lexicographically numbered Q1 grids with enough rows to fill the SMs (with the
-// configuration's `diagonal` set: of any size) run in a stencil form instead: values by diagonal, one
+// System matrices of lexicographically numbered Q1 grids run in a stencil form instead (the
+// configuration's `diagonal`: 0 none, 1 all, below 0 those with enough rows to fill the SMs): values by diagonal, one
 // warp per strip of consecutive rows, each x row gathered once for all the strip's rows it enters
 // (strip_rows).  Rows are summed in stored entry order without FMA, per right-hand side, as in the
 // single-RHS kernels, in both forms.  Dot products and norms are reduced per block and then with FP64
@@ -1032,11 +1032,11 @@ namespace mr
     const std::vector<uint32_t>& col, int prec)
   {
     d.nd = 0;
-    // whether a pass runs in this form: every SM has a block of strips to run (18,944 rows on 148 SMs),
-    // or the configuration asks.  Ten iterations, CSR against stencil form: 2D 16,641 rows, 64 right-hand
+    // whether a pass runs in this form, where the configuration leaves it open: every SM has a block of
+    // strips to run (18,944 rows on 148 SMs).  Ten iterations, CSR against stencil form: 2D 16,641 rows, 64 right-hand
     // sides FP64 2,547 against 2,906 us; 3D 4,913 rows, 64 FP32 1,223 against 1,353; above the line 2D
     // 66,049 rows, 64 FP32 4,377 against 3,832; 3D 35,937 rows, 64 FP64 4,305 against 3,899
-    if(!s->cfg.diagonal && d.rows < s->grid / 8u * uint32_t(MW_MAX * STRIP))
+    if(s->cfg.diagonal == 0 || (s->cfg.diagonal < 0 && d.rows < s->grid / 8u * uint32_t(MW_MAX * STRIP)))
       return FB_OK;
     std::vector<int64_t> off;
     for(uint32_t r = 0; r < d.rows; ++r)

@@ -474,7 +474,7 @@ class MultiRhsPCG:
     element layout of the reference's DenseVectorBlocked."""
 
     def __init__(self, hierarchy: MultiGridHierarchy, num_rhs, tol_rel=1e-8, max_iter=100, precision="f64",
-                 ordering="native", use_graph=True, stencil=False):
+                 ordering="native", use_graph=True, stencil=None):
         omega, steps = hierarchy.smoother_params()
         self.k = int(num_rhs)
         self.cfg = _lib.SolverConfig()
@@ -483,10 +483,10 @@ class MultiRhsPCG:
         self.cfg.tol_rel, self.cfg.max_iter = float(tol_rel), int(max_iter)
         self.cfg.precision, self.cfg.ordering = _lib.PREC[precision], _lib.ORDER[ordering]
         self.cfg.use_graph = 1 if use_graph else 0
-        # System matrices with the Q1 stencil pattern in the device numbering run in the stencil form
-        # (strips of rows sharing their gathers; row sums bitwise those of the CSR form) where they have
-        # enough rows to fill the SMs; stencil=True: at every size.
-        self.cfg.diagonal = 1 if stencil else 0
+        # System matrices with the Q1 stencil pattern in the device numbering have a stencil form (strips of
+        # rows sharing their gathers; row sums bitwise those of the CSR form).  stencil=False: always CSR,
+        # True: the stencil form at every size, None: where a level has enough rows to fill the SMs.
+        self.cfg.diagonal = -1 if stencil is None else (1 if stencil else 0)
         if hierarchy._h is None:
             hierarchy.init()
         self.hierarchy = hierarchy

@@ -246,8 +246,8 @@ typedef struct
                            missing diagonals hold zeros); 0 = always sliced ELL.  The multi-RHS
                            solver (fb_msolver_*) has a stencil form for system matrices whose stored
                            rows all have the same 9 or 27 column offsets in triplets (o-1, o, o+1):
-                           used for diagonal != 0, or where a level has enough rows to fill the SMs
-                           (the same results bit for bit) */
+                           never used for 0, at every size above 0, and below 0 where a level has
+                           enough rows to fill the SMs (the same row sums bit for bit) */
   int pdl;              /* 1 (default): the solve's kernels are launched with programmatic stream
                            serialisation, so each one's launch and its matrix prologue overlap the
                            end of its predecessor; 0 = plain stream order */

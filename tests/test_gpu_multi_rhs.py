@@ -106,8 +106,8 @@ def test_multi_rhs_stencil_form(featlib, cuda, dim, level, precision):
 # sides in two sweeps
 @pytest.mark.parametrize("dim,level,K,precision", [(2, 7, 32, "f64"), (2, 8, 64, "f64"), (2, 8, 32, "f32"), (3, 5, 64, "f32")])
 def test_forms_of_large_levels(featlib, cuda, dim, level, K, precision):
-    """Every right-hand side agrees with its own solve (kernel/solver/pcg.hpp:159-286); forced and chosen
-    forms take the same number of iterations."""
+    """Every right-hand side agrees with its own solve (kernel/solver/pcg.hpp:159-286); both forms and the
+    choice between them by level take the same number of iterations, and the bytes of a solve tell which ran."""
     torch, fb = cuda, featlib
     from featb200 import assembly as AS
     levels, b = AS.poisson_hierarchy(level, dim, rhs="gauss", gauss=AS.gauss_params(7, dim))
@@ -115,16 +115,22 @@ def test_forms_of_large_levels(featlib, cuda, dim, level, K, precision):
     rhs = torch.tensor(b[:, None] * scale, device="cuda")
     one = fb.build_pcg_multigrid(levels, precision=precision)
     h = fb.build_hierarchy(levels)
-    iters = []
-    for stencil in (False, True):
+    iters, moved = [], {}
+    for stencil in (False, True, None):
         m = fb.MultiRhsPCG(h, K, precision=precision, stencil=stencil)
         x = torch.zeros_like(rhs)
         m.solve_device(x, rhs)
         iters.append(m.iterations())
+        moved[stencil] = m.info[0].bytes_moved
         for j in (0, K // 2 - 1, K // 2, K - 1):
             ref = torch.zeros(b.size, dtype=torch.float64, device="cuda")
             assert one.correct_device(ref, rhs[:, j].contiguous()) == fb.Status.success == m.statuses()[j]
             assert iters[-1][j] == one.get_num_iter()
             # only the order of the PCG's sums differs
             assert rel_err(x[:, j].cpu().numpy(), ref.cpu().numpy()) <= (1e-12 if precision == "f64" else 1e-9)
-    assert iters[0] == iters[1]
+    assert iters[0] == iters[1] == iters[2]
+    assert moved[True] < moved[False]
+    if b.size < 18944:
+        assert moved[None] == moved[False]
+    else:
+        assert moved[True] < moved[None] < moved[False]
