@@ -10,7 +10,7 @@
 // in the blocks' shared memory (ClBar).  What is left is latency: a pass is one or two rows' chain of
 // shared or distributed loads per thread and a barrier, 0.5 us to 2 us; a whole solve of 2D FP64 level
 // 5 (1,089 rows, 5 iterations) takes 205 us with host work, 370 us as launched passes, and level 7
-// (16,641 rows, 6 iterations) 416 us against 556 us.  One short loop runs a list of passes written by the host: the code
+// (16,641 rows, 6 iterations) 390 us against 556 us.  One short loop runs a list of passes written by the host: the code
 // of a pass is fetched once per launch and reused, where the single-block tail's straight-line
 // sequence waits for instruction fetch.
 //
@@ -584,6 +584,73 @@ namespace fb
     if(!all && threadIdx.x == 0 && me == 0)
       *err = 1;
     return all != 0;
+  }
+
+  // ---------------------------------------------------------------- the image
+  // How a level's rows are dealt out: `last` = the block that holds them all, or CL_NONE
+  struct ClMap
+  {
+    uint32_t n, rpc, last;
+    __device__ __forceinline__ uint32_t owner(uint32_t i) const { return last == CL_NONE ? i / rpc : last; }
+    __device__ __forceinline__ uint32_t local(uint32_t i) const { return last == CL_NONE ? i % rpc : i; }
+  };
+  // A matrix as the launched passes store it and where its rows go in the image: K entries per row at
+  // stride ns, values at offset `val`, column codes at `code` (CL_NONE: values only)
+  template<typename V>
+  struct ClMat
+  {
+    DCsr<V> M;
+    const uint32_t* mask;    // diagonal storage of more than K diagonals: each row's own ones, as bits
+    ClMap rows, cols;
+    uint32_t K, ns, val, code;
+    unsigned char* img;
+    uint32_t stride;
+  };
+
+  // entry k of row i, in stored order; slots past a row's entries hold 0 at the row's own column where there is
+  // one, so that they do not make a warp's loads leave the block (at the level's first column: 2D level 7
+  // FP64, one solve 416 us, against 390)
+  template<typename V>
+  __device__ __forceinline__ void cl_copy_entry(const ClMat<V>& m, uint32_t i, uint32_t k)
+  {
+    const uint32_t sl = i >> 5;
+    unsigned char* base = m.img + size_t(m.rows.owner(i)) * m.stride;
+    const size_t o = size_t(k) * m.ns + m.rows.local(i);
+    const uint32_t b0 = m.M.kw ? sl * 32u * m.M.kw : m.M.soff[sl], w = m.M.kw ? m.M.kw : (m.M.soff[sl + 1] - b0) >> 5;
+    const uint32_t u = m.mask ? __fns(m.mask[i], 0u, int(k) + 1) : k;
+    V val{};
+    uint32_t col = m.cols.n;
+    if(u < w)
+    {
+      const uint32_t e = b0 + (i & 31u) + u * 32u;
+      val = m.M.val[e];
+      if(m.code != CL_NONE)
+        col = m.M.doff ? uint32_t(int32_t(i) + m.M.doff[u])
+                       : (m.M.dcol ? uint32_t(int32_t(i) + int32_t(m.M.dcol[e])) : m.M.col[e]);
+    }
+    reinterpret_cast<V*>(base + m.val)[o] = val;
+    if(m.code == CL_NONE)
+      return;
+    if(col >= m.cols.n)
+      col = i < m.cols.n ? i : 0u;
+    reinterpret_cast<uint16_t*>(base + m.code)[o] = uint16_t(m.cols.owner(col) << 12 | m.cols.local(col));
+  }
+
+  // A matrix's rows into the image, and (dinv given) the level's inverse diagonal and mask; blockIdx.y = the
+  // entry within the row
+  template<typename V, typename S>
+  __global__ void __launch_bounds__(256) k_cl_image(const ClMat<V> m, const S* __restrict__ dinv,
+    const uint8_t* __restrict__ dm, uint32_t odinv, uint32_t odm)
+  {
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    if(i >= m.rows.n)
+      return;
+    cl_copy_entry(m, i, blockIdx.y);
+    if(!dinv || blockIdx.y)
+      return;
+    unsigned char* base = m.img + size_t(m.rows.owner(i)) * m.stride;
+    reinterpret_cast<S*>(base + odinv)[m.rows.local(i)] = dinv[i];
+    base[odm + m.rows.local(i)] = dm[i];
   }
 
   // The V-cycle below the launched levels: b and sol1 of the cluster's top level come from the

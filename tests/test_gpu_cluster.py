@@ -59,3 +59,55 @@ def test_cluster_equals_launched_passes(featlib, cuda, oracle_lib, level, dim, o
     assert s.correct_device(zero, zero.clone()) == fb.Status.success and s.get_num_iter() == 0
     bad = torch.full((b.size,), float("nan"), dtype=torch.float64, device="cuda")
     assert s.correct_device(torch.zeros_like(bad), bad) == fb.Status.aborted
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32_bf16"])
+def test_update_follows_in_one_launch_per_array(featlib, cuda, precision):
+    """fb_solver_update_matrix launches what a solver without a cluster plan launches (values, in FP32 modes the
+    FP64 copy, diagonal): the plan's image is rewritten in the last of them."""
+    import torch
+    from featb200 import assembly as AS
+    fb = featlib
+    levels, _ = AS.poisson_hierarchy(6, 2, rhs="sine")
+    count = []
+    for kw in ({}, {"tail_rows": 301}):
+        s = fb.build_pcg_multigrid(levels, precision=precision, **kw)
+        c0 = fb.launch_count()
+        for l, L in enumerate(levels):
+            s.update_matrix(l, torch.tensor(L["matrix"].val, device="cuda"))
+        count.append(fb.launch_count() - c0)
+    assert count[0] == count[1]
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32_bf16"])
+def test_more_diagonals_than_entries_per_row(featlib, cuda, precision):
+    """Diagonal storage with diagonals that few rows have: the cluster's rows hold their own entries only, as
+    long as the longest of them; solves agree with the launched passes' before and after an update."""
+    import scipy.sparse as sp
+    import torch
+    from featb200 import assembly as AS
+    fb = featlib
+    levels, b = AS.poisson_hierarchy(5, 2, rhs="gauss", gauss=AS.gauss_params(5, 2))
+    for L in levels[:-2]:
+        A, n = L["matrix"].to_scipy().tocsr(), 2 ** L["level"] + 1
+        i = np.array([r * n + 1 + 2 * (r % 2) for r in range(1, n - 1)])   # couples (1 or 3, r) with 3 further on
+        E = sp.coo_matrix((np.full(i.size, -0.1), (i, i + 3)), shape=A.shape)
+        W = (A + E + E.T + sp.diags(np.asarray((-E - E.T).sum(axis=1)).ravel())).tocsr()
+        W.sort_indices()
+        L["matrix"] = fb.SparseMatrixCSR.from_scipy(W)
+        p = fb.storage_plan(L["matrix"], L["filter"].indices)
+        assert p["kind"] == "diagonal" and p["diagonals"] == 11 and np.diff(W.indptr).max() == 10
+    s, ref = (fb.build_pcg_multigrid(levels, precision=precision, **kw) for kw in ({}, {"tail_rows": 301}))
+    for scale in (1.0, 3.0):
+        if scale != 1.0:
+            for l, L in enumerate(levels):
+                v = torch.tensor(L["matrix"].val * scale, device="cuda")
+                s.update_matrix(l, v)
+                ref.update_matrix(l, v)
+        xs = []
+        for t in (s, ref):
+            x = torch.zeros(b.size, dtype=torch.float64, device="cuda")
+            assert t.correct_device(x, torch.tensor(b, device="cuda")) == fb.Status.success
+            xs.append(x.cpu().numpy())
+        assert s.get_num_iter() == ref.get_num_iter()
+        assert rel_err(xs[0], xs[1]) <= (1e-12 if precision == "f64" else 1e-9)
