@@ -1430,7 +1430,7 @@ namespace bt
     // every staged pass the solve launches, looked up once before its launches are captured
     void prime()
     {
-      for(int G = 1; G < s->NG; ++G)
+      for(int G = s->bottom + 1; G < s->NG; ++G)
       {
         const fb_batch::GLevel& f = s->g[size_t(G)];
         if(use_tma(f.A))
@@ -1644,7 +1644,8 @@ namespace bt
   // 2 .. 16 warps of 32 rows) that runs the level's defect pass fastest over all instances present
   // (median of 5 timed launches after 2 untimed ones; the pass writes only the level's defect
   // buffer, which the solve overwrites).  Small levels favour small blocks (more SMs busy), large
-  // levels larger ones.
+  // levels larger ones.  The levels of kb_bottom are left out, except its finest: the launched
+  // restriction into it takes that level's choice.
   template<typename V, typename S>
   static fb_status autotune(fb_batch* s)
   {
@@ -1653,7 +1654,7 @@ namespace bt
     kb_open<<<4, 256, 0, st>>>(sc);
     FB_LAUNCHED(1);
     const int cand[4] = {64, 128, 256, 512};
-    for(int G = 1; G < s->NG; ++G)
+    for(int G = std::max(1, s->bottom); G < s->NG; ++G)
     {
       fb_batch::GLevel& f = s->g[size_t(G)];
       float best = 1e30f;
@@ -1685,7 +1686,8 @@ namespace bt
       }
       f.bs = pick;
     }
-    s->g[0].bs = s->NG > 1 ? s->g[1].bs : 256;
+    if(s->bottom == 0)
+      s->g[0].bs = s->NG > 1 ? s->g[1].bs : 256;
     FB_CUDA(cudaStreamSynchronize(st));
     return FB_OK;
   }

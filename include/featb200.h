@@ -433,8 +433,8 @@ fb_status fb_batch_solve(fb_batch* b, double* sol, const double* rhs, fb_solve_i
 /* As fb_batch_solve with DEVICE packed arrays, ordered on `stream`. */
 fb_status fb_batch_solve_device(fb_batch* b, double* sol, const double* rhs, void* stream, fb_solve_info* info);
 /* Rows per block of the V-cycle passes per global level (finest first; rows_per_block may be NULL to
- * query num_levels): the autotuner's choice at creation, or cfg.rows_per_block.  No counterpart in
- * the reference. */
+ * query num_levels): the autotuner's choice at creation, or cfg.rows_per_block; 256 for the coarse levels
+ * that run in one kernel for all passes and are not tuned.  No counterpart in the reference. */
 fb_status fb_batch_rows_per_block(const fb_batch* b, int* rows_per_block, int* num_levels);
 
 /* ------------------------------------------------------------------------------------------ */

@@ -107,6 +107,19 @@ def test_batch_rows_per_block(featlib, cuda, rows_per_block):
         assert rel_err(X[k], x.elements) <= 1e-12
 
 
+def test_batch_tunes_launched_levels_only(featlib, cuda):
+    """Levels 1 to 3 of these instances run in the bottom kernel, with level 4 on top of it: 28 timed launches each
+    for levels 4, 5 and 6 (after one that opens the instances)."""
+    fb = featlib
+    hs = [fb.build_hierarchy(lv) for lv, _ in _family([5, 6])]
+    count = []
+    for rows_per_block in (0, 64):
+        c0 = fb.launch_count()
+        fb.BatchPCG(hs, rows_per_block=rows_per_block)
+        count.append(fb.launch_count() - c0)
+    assert count[0] - count[1] == 1 + 3 * 28
+
+
 @pytest.mark.parametrize("precision", ["f64", "f32"])
 def test_batch_many_instances_per_block(featlib, cuda, precision):
     """Enough small instances (300 of levels 3 to 5) that a block's range of rows holds several of
