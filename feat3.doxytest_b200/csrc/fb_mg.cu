@@ -2327,10 +2327,11 @@ namespace fb
   // The plan of a solver: whole solves when everything fits, otherwise the bottom of its V-cycle from
   // the finest level (below the top) that fits.  For the V-cycle with Jacobi smoothing and the
   // fixed coarse-grid correction; a configuration that chooses its passes itself (tail, fused,
-  // streamed, cluster or staged-pass options off their defaults) keeps them.  One cluster beats the
-  // launched passes wherever it fits (launched -> cluster, one solve): whole solves of 2D FP64 levels
-  // 5 and 7 349 -> 232 and 568 -> 502 us; bottoms below launched levels, 2D level 9 FP64 with RCM
-  // 1,193 -> 986 us, 2D level 10 FP32 1,534 -> 1,419 us, 3D level 6 FP32 1,425 -> 1,119 us.
+  // streamed or staged-pass options off their defaults, cluster_rows above 0) keeps them, and cluster_rows
+  // below 0 keeps clusters out.  One cluster beats the launched passes wherever it fits (launched ->
+  // cluster, one solve): whole solves of 2D FP64 levels 5 and 7 349 -> 205 and 557 -> 390 us; bottoms below
+  // launched levels, 2D level 9 FP64 with RCM 1,193 -> 942 us, 2D level 10 FP32 1,534 -> 1,392 us, 3D
+  // level 6 FP32 1,425 -> 988 us (with diagonal storage of level 5).
   template<typename V, typename S>
   static fb_status cl_build(fb_solver* s)
   {

@@ -272,7 +272,8 @@ class PCG:
 
     def set_cluster_rows(self, rows):
         """Levels with at most `rows` rows (below the finest) run in one kernel on a cluster of 8
-        thread blocks (0 = off; takes precedence over set_tail_rows)."""
+        thread blocks (takes precedence over set_tail_rows); 0 (default) = what fits the shared memory of
+        16 blocks runs in a cluster of 16, where the other options leave it open; below 0 = no clusters."""
         self.cfg.cluster_rows = int(rows)
 
     def set_diagonal(self, on):

@@ -221,18 +221,20 @@ typedef struct
   int tail_rows;        /* levels (below the finest) with at most this many rows, down to the
                            coarsest, run in one single-block kernel per visit of the cycle (a
                            V-cycle bottom, or an F/W sub-cycle with its peak smoothing); 0 = off.
-                           With tail_rows, cluster_rows, fused, streamed, tma_rows and tma_window at
-                           their defaults a V-cycle with Jacobi smoothing and the fixed coarse-grid
-                           correction takes neither: its levels from the finest that fits the shared
-                           memory of 16 SMs run in one kernel on a cluster of 16 thread blocks, and
-                           where all levels fit the whole solve does */
+                           Where cluster_rows leaves the choice open, a V-cycle runs its coarse
+                           levels on a cluster of thread blocks instead */
   int tma_rows;         /* levels with at least this many rows use the TMA-staged persistent
                            passes (bulk copies into shared memory); 0 = off */
   int cluster_rows;     /* levels (below the finest) with at most this many rows, down to the
                            coarsest, run in one kernel on a cluster of 8 thread blocks (8 SMs) per
                            V-cycle, passes separated by the cluster barrier; takes precedence over
-                           tail_rows; V-cycle only; 0 = off (default: measured slower than the
-                           single-block tail on B200 for every threshold) */
+                           tail_rows; V-cycle only (measured slower than the single-block tail on
+                           B200 for every threshold); below 0 = no clusters.  0 (default) = the
+                           levels from the finest that fits the shared memory of 16 SMs run in one
+                           kernel on a cluster of 16 thread blocks, and where all levels fit the
+                           whole solve does; for a V-cycle with Jacobi smoothing and the fixed
+                           coarse-grid correction, with tail_rows, fused, streamed, tma_rows and
+                           tma_window at their defaults, and as without clusters otherwise */
   int cycle;            /* FB_CYCLE_V (default), FB_CYCLE_F or FB_CYCLE_W: the multigrid cycle of
                            MultiGrid::_apply_cycle_v/_f/_w (kernel/solver/multigrid.hpp:1350-1440) */
   int tma_window;       /* the window of the gathered vector that a TMA-staged chunk reads:

@@ -111,3 +111,22 @@ def test_more_diagonals_than_entries_per_row(featlib, cuda, precision):
             xs.append(x.cpu().numpy())
         assert s.get_num_iter() == ref.get_num_iter()
         assert rel_err(xs[0], xs[1]) <= (1e-12 if precision == "f64" else 1e-9)
+
+
+def test_cluster_switch(featlib, cuda):
+    """cluster_rows below 0 keeps clusters out with every other option at its default: the launched passes and the
+    tail kernel, bit for bit those of a configuration that chooses its passes."""
+    import torch
+    from featb200 import assembly as AS
+    fb = featlib
+    levels, b = AS.poisson_hierarchy(5, 2, rhs="gauss", gauss=AS.gauss_params(5, 2))
+    xs, launches = [], []
+    for kw in ({}, {"cluster_rows": -1}, {"tail_rows": 301}):
+        s = fb.build_pcg_multigrid(levels, **kw)
+        x = torch.zeros(b.size, dtype=torch.float64, device="cuda")
+        c0 = fb.launch_count()
+        assert s.correct_device(x, torch.tensor(b, device="cuda")) == fb.Status.success
+        launches.append(fb.launch_count() - c0)
+        xs.append(x.cpu().numpy())
+    assert launches[0] == 1 and launches[1] == launches[2] > 1
+    assert np.array_equal(xs[1], xs[2]) and rel_err(xs[0], xs[1]) <= 1e-12
