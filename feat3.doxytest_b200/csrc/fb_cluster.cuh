@@ -100,7 +100,7 @@ namespace fb
     const unsigned char* gimg;            // this block's image in global memory
     int* err;
     uint32_t staged, img;                 // bytes of it staged in shared memory, and where
-    double *x, *hist;                     // whole solves: the iterate, the defect history
+    double* x;                            // whole solves: the iterate
     const Scalars* sc;
     int it, status;
   };
@@ -808,8 +808,6 @@ namespace fb
       w.st.beta = 0.0;
       w.st.it = 0;
       w.st.status = status;
-      if(me == 0u)
-        w.st.hist[0] = d0;
     }
     // every block has read the partial sums and p before the next pass writes them
     bar.sync<false>(cl_sm, me, w.cs, 0u, 0u);
@@ -892,18 +890,16 @@ namespace fb
       w.st.beta = beta;
       w.st.it = it + 1;
       w.st.status = status;
-      if(me == 0u)
-        w.st.hist[it + 1] = dc;
     }
     __syncthreads();
     return bar;
   }
 
   // A whole PCG solve (kernel/solver/pcg.hpp:159-286): x is the initial guess and the result; the
-  // scalars and the defect history go to *sc and hist as the launched passes leave them.
+  // scalars go to *sc as the launched passes leave them.
   template<typename V, typename S>
   __global__ void __launch_bounds__(CL_NT, 1) k_cl_solve(const ClParams* __restrict__ gp, double* gx,
-    const double* rhs, double* __restrict__ hist, Scalars* sc, int* err)
+    const double* rhs, Scalars* sc, int* err)
   {
     extern __shared__ __align__(128) unsigned char cl_sm[];
     const uint32_t me = cl_rank();
@@ -918,7 +914,6 @@ namespace fb
     if(threadIdx.x == 0)
     {
       st.x = gx;
-      st.hist = hist;
       st.sc = sc;
     }
     __syncthreads();

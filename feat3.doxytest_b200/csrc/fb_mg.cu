@@ -1265,7 +1265,7 @@ namespace fb
   template<typename S>
   __global__ void __launch_bounds__(NT) k_pcg_init(DCsr<double> A, const double* __restrict__ rhs,
     const double* __restrict__ x, double* __restrict__ r, const uint8_t* __restrict__ dm, S* __restrict__ x1,
-    const S* __restrict__ dinv, int* __restrict__ skip_top, double* __restrict__ hist, RedSlot slot,
+    const S* __restrict__ dinv, int* __restrict__ skip_top, RedSlot slot,
     Scalars* __restrict__ sc, cudaGraphConditionalHandle cond)
   {
     pdl_wait();
@@ -1292,7 +1292,6 @@ namespace fb
       sc->def_cur = d0;
       sc->iter = 0;
       sc->gamma = 0.0;
-      hist[0] = d0;
       int status = FB_SOLVER_PROGRESS;
       if(!isfinite(d0))
         status = FB_SOLVER_ABORTED;
@@ -1369,7 +1368,7 @@ namespace fb
   template<typename S, bool CONVERT>
   __global__ void __launch_bounds__(NT) k_pcg_x(double* __restrict__ x, double* __restrict__ r,
     const double* __restrict__ p, const double* __restrict__ q, const uint8_t* __restrict__ dm, S* __restrict__ bt,
-    S* __restrict__ x1, const S* __restrict__ dinv, int* __restrict__ skip_top, double* __restrict__ hist, uint32_t n,
+    S* __restrict__ x1, const S* __restrict__ dinv, int* __restrict__ skip_top, uint32_t n,
     RedSlot slot, Scalars* __restrict__ sc, cudaGraphConditionalHandle cond)
   {
     pdl_wait();
@@ -1424,7 +1423,6 @@ namespace fb
       const double dc = sqrt(total);
       sc->iter = it;
       sc->def_cur = dc;
-      hist[it] = dc;
       int status = FB_SOLVER_PROGRESS;
       if(!isfinite(dc))
         status = FB_SOLVER_ABORTED;
@@ -1772,7 +1770,6 @@ struct fb_solver
   double *tmp_in = nullptr, *tmp_out = nullptr;
   void* flush = nullptr;   // L2 flush buffer of fb_solver_time_kernel (allocated on first use)
   uint32_t* perm0 = nullptr;
-  double* hist = nullptr;
   // fb_solver_update_matrix: per level, the device slot of every caller CSR entry (UINT32_MAX =
   // not stored) and the caller entry of every device row's diagonal; built on first use
   std::vector<uint32_t*> upd_slot, upd_diag;
@@ -1792,7 +1789,7 @@ struct fb_solver
   uint8_t* tail_prog = nullptr;             // tail kernel programs: events op << 4 | tail level
   std::vector<uint32_t> seg_off, seg_len;   // program of each tail segment of `events`, in order
   double* cgc_omega = nullptr;   // step length of the adaptive coarse-grid correction
-  int max_iter_cap = 0;   // max_iter at creation: the defect history holds max_iter + 2 entries
+  int max_iter_cap = 0;   // max_iter at creation: the most that it may be set to
   void* vc_top = nullptr; // buffer that holds the finest level's result after a standalone V-cycle
   uint32_t slot_cap = 0;  // blocks whose (two) partial sums the reduction slot holds
   int fs_bps_down = 1, fs_bps_up = 1;   // resident blocks per SM of the streamed passes
@@ -3160,7 +3157,7 @@ namespace fb
       const bool f64 = s->cfg.precision == FB_PREC_F64;
       const DevMat& A = A64();
       if(!dry) go(k_pcg_init<S>, blocks(t.n), NT, A.smem, view<double>(A), s->rhs, s->x, s->r, t.dm,
-        f64 ? (S*)t.x : (S*)nullptr, (const S*)t.dinv, t.skip_pre, s->hist, s->slot, s->sc, 0);
+        f64 ? (S*)t.x : (S*)nullptr, (const S*)t.dinv, t.skip_pre, s->slot, s->sc, 0);
       ++launches;
       bytes += A.bytes + double(t.n) * 8 * 4 + t.n;
       if(!f64)
@@ -3188,10 +3185,10 @@ namespace fb
         ;
       else if(f64)
         go(k_pcg_x<S, false>, pcgx_grid(t.n), NT, 0, s->x, s->r, s->p, s->q, t.dm, (S*)nullptr, (S*)t.x,
-          (const S*)t.dinv, t.skip_pre, s->hist, t.n, s->slot, s->sc, cond);
+          (const S*)t.dinv, t.skip_pre, t.n, s->slot, s->sc, cond);
       else
         go(k_pcg_x<S, true>, pcgx_grid(t.n), NT, 0, s->x, s->r, s->p, s->q, t.dm, (S*)t.b, (S*)t.x,
-          (const S*)t.dinv, t.skip_pre, s->hist, t.n, s->slot, s->sc, cond);
+          (const S*)t.dinv, t.skip_pre, t.n, s->slot, s->sc, cond);
       launches += 3;
       bytes += double(t.n) * 8 * (first ? 2 : 3);                                    // P
       bytes += A.bytes + double(t.n) * 8 * 3 + t.n;                                   // Q
@@ -3338,7 +3335,7 @@ namespace fb
       cudaLaunchAttribute at[2];
       cl_config(s, s->cl_full, lc, at, st);
       FB_CUDA(cudaLaunchKernelEx(&lc, k_cl_solve<V, S>, (const ClParams*)s->cl_full.dpar, x, rhs,
-        s->hist, s->sc, s->err));
+        s->sc, s->err));
       return FB_OK;
     }
     if(s->cfg.use_graph)
@@ -3644,7 +3641,6 @@ fb_status fb_solver_create(fb_solver** out, fb_hierarchy* h, const fb_solver_con
     FB_TRY(dalloc(s.get(), (void**)&s->perm0, sizeof(uint32_t) * n0));
     FB_CUDA(cudaMemcpy(s->perm0, s->perms[0].data(), sizeof(uint32_t) * n0, cudaMemcpyHostToDevice));
   }
-  FB_TRY(dalloc(s.get(), (void**)&s->hist, sizeof(double) * (size_t(cfg.max_iter) + 2)));
   // the scalars and, behind them, the error word: one copy to the host after a solve
   FB_TRY(dalloc(s.get(), (void**)&s->sc, sizeof(Scalars) + sizeof(int)));
   s->err = reinterpret_cast<int*>(s->sc + 1);

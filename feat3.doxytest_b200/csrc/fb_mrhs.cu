@@ -787,8 +787,8 @@ namespace mr
   template<typename S, int R, bool CONVERT>
   __global__ void __launch_bounds__(MNT_BIG, 1) km_pcg_x(double* __restrict__ x, double* __restrict__ rr,
     const double* __restrict__ p, const double* __restrict__ q, const uint8_t* __restrict__ dm, S* __restrict__ bt,
-    S* __restrict__ x1, const S* __restrict__ dinv, int* __restrict__ skip_top, double* __restrict__ hist,
-    uint32_t n, int hist_stride, MScal* __restrict__ sc)
+    S* __restrict__ x1, const S* __restrict__ dinv, int* __restrict__ skip_top,
+    uint32_t n, MScal* __restrict__ sc)
   {
     constexpr int K = 32 * R;
     if(closed(sc))
@@ -842,7 +842,6 @@ namespace mr
       const double s = CONVERT ? pow2_inv(sc->def_cur[j]) : 1.0;
       sc->iter[j] = it;
       sc->def_cur[j] = dc;
-      hist[size_t(it) * hist_stride + j] = dc;
       int st = FB_SOLVER_PROGRESS;
       if(!isfinite(dc))
         st = FB_SOLVER_ABORTED;
@@ -950,7 +949,7 @@ struct fb_msolver
   double* cinv = nullptr;
   uint32_t nfree = 0;
   double *x = nullptr, *r = nullptr, *p = nullptr, *q = nullptr, *z = nullptr, *rhs = nullptr;
-  double *tin = nullptr, *tout = nullptr, *hist = nullptr;
+  double *tin = nullptr, *tout = nullptr;
   fb::mr::MScal* sc = nullptr;
   cudaStream_t stream = nullptr;
   cudaGraph_t graph = nullptr;
@@ -1271,10 +1270,10 @@ namespace mr
         });
         if(f64)
           km_pcg_x<S, R, false><<<flat(t.n).g, flat(t.n).t, 0, st>>>(s->x, s->r, s->p, s->q, t.dm, (S*)nullptr, (S*)t.x,
-            (const S*)t.dinv, t.skip_pre, s->hist, t.n, K, s->sc);
+            (const S*)t.dinv, t.skip_pre, t.n, s->sc);
         else
           km_pcg_x<S, R, true><<<flat(t.n).g, flat(t.n).t, 0, st>>>(s->x, s->r, s->p, s->q, t.dm, (S*)t.b, (S*)t.x,
-            (const S*)t.dinv, t.skip_pre, s->hist, t.n, K, s->sc);
+            (const S*)t.dinv, t.skip_pre, t.n, s->sc);
         km_count_progress<<<1, 64, 0, st>>>(s->sc, K, cond);
       }
       launches += 4;
@@ -1517,7 +1516,6 @@ fb_status fb_msolver_create(fb_msolver** out, fb_hierarchy* h, const fb_solver_c
     MR_TRY(mr::malloc0(s.get(), (void**)&s->perm0_d, 4 * n0));
     FB_CUDA(cudaMemcpy(s->perm0_d, s->perm0.data(), 4 * n0, cudaMemcpyHostToDevice));
   }
-  MR_TRY(mr::malloc0(s.get(), (void**)&s->hist, sizeof(double) * (size_t(cfg.max_iter) + 2) * K));
   MR_TRY(mr::malloc0(s.get(), (void**)&s->sc, sizeof(mr::MScal)));
   mr::MScal h0;
   std::memset(&h0, 0, sizeof(h0));

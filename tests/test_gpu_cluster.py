@@ -130,3 +130,17 @@ def test_cluster_switch(featlib, cuda):
         xs.append(x.cpu().numpy())
     assert launches[0] == 1 and launches[1] == launches[2] > 1
     assert np.array_equal(xs[1], xs[2]) and rel_err(xs[0], xs[1]) <= 1e-12
+
+
+@pytest.mark.parametrize("kw", [{}, {"cluster_rows": -1}])
+def test_min_iter_above_max_iter(featlib, cuda, kw):
+    """min_iter is tested before max_iter: a solve takes min_iter iterations."""
+    import torch
+    from featb200 import _lib, assembly as AS
+    fb = featlib
+    levels, b = AS.poisson_hierarchy(5, 2, rhs="gauss", gauss=AS.gauss_params(5, 2))
+    s = fb.build_pcg_multigrid(levels, max_iter=2, **kw)
+    _lib.check(_lib.lib().fb_solver_set_iteration_limits(s._s, 9, 2))
+    x = torch.zeros(b.size, dtype=torch.float64, device="cuda")
+    assert s.correct_device(x, torch.tensor(b, device="cuda")) == fb.Status.success
+    assert s.get_num_iter() == 9
