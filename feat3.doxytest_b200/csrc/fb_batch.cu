@@ -36,7 +36,6 @@ namespace bt
   constexpr int BNT = 256;       // block size of the PCG-space kernels (4 resident per SM: at most 64 registers)
   constexpr int PCGP_ROWS = 4;   // rows per thread of p = z + beta p
   constexpr int BNT_MAX = 512;   // largest block size the autotuner may pick for the V-cycle passes
-  constexpr int BW = BNT / 32;
   constexpr int MAXG = 16;
 
   struct BScal   // device-resident, per instance arrays of length J

@@ -3886,7 +3886,7 @@ static fb_status solve_enqueue(fb_solver* s, double* x, const double* rhs)
 
 // reads the scalars and the error word, which waits for everything enqueued before, and reports the
 // solve.  (To pageable memory: a pinned buffer of the solver's own made a 16,641-row solver's creation
-// 7 ms longer and a solve no faster.)
+// 10 ms longer and a solve no faster.)
 static fb_status solve_finish(fb_solver* s, fb_solve_info* info)
 {
   cudaStream_t st = s->stream;

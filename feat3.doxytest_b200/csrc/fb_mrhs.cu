@@ -536,7 +536,6 @@ namespace mr
     constexpr int K = 32 * R;
     if(closed(sc))
       return;
-    const int lane = threadIdx.x & 31;
     double part[R];
     #pragma unroll
     for(int r = 0; r < R; ++r)
@@ -573,7 +572,6 @@ namespace mr
     constexpr int K = 32 * R;
     if(closed(sc))
       return;
-    const int lane = threadIdx.x & 31;
     double part[R];
     #pragma unroll
     for(int r = 0; r < R; ++r)
@@ -644,7 +642,6 @@ namespace mr
     const S* __restrict__ dinv, int* __restrict__ skip_top, MScal* __restrict__ sc)
   {
     constexpr int K = 32 * R;
-    const int lane = threadIdx.x & 31;
     double part[R];
     #pragma unroll
     for(int r = 0; r < R; ++r)
@@ -759,7 +756,6 @@ namespace mr
     constexpr int K = 32 * R;
     if(closed(sc))
       return;
-    const int lane = threadIdx.x & 31;
     double part[R];
     #pragma unroll
     for(int r = 0; r < R; ++r)

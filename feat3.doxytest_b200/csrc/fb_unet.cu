@@ -44,11 +44,10 @@ namespace un
   }
 
   constexpr int NLAYER = 10;
-  struct LayerDef { int cin, cout, level; bool relu; int dil; };
-  // real channel counts; level = resolution index (0 = finest grid); dil = tap spacing
-  constexpr LayerDef LAYERS[NLAYER] = {
-    {2, 16, 0, true, 1}, {16, 32, 1, true, 1}, {32, 64, 2, true, 1}, {64, 64, 3, true, 1}, {64, 64, 3, true, 2},
-    {64, 64, 3, true, 4}, {128, 64, 2, true, 1}, {96, 32, 1, true, 1}, {48, 16, 0, true, 1}, {16, 1, 0, false, 1}};
+  struct LayerDef { int cin, cout, level; };
+  // real channel counts; level = resolution index (0 = finest grid)
+  constexpr LayerDef LAYERS[NLAYER] = {{2, 16, 0}, {16, 32, 1}, {32, 64, 2}, {64, 64, 3}, {64, 64, 3}, {64, 64, 3},
+                                       {128, 64, 2}, {96, 32, 1}, {48, 16, 0}, {16, 1, 0}};
 
   __host__ __device__ inline int pad8(int c) { return (c + 7) & ~7; }
 
