@@ -1760,6 +1760,9 @@ struct fb_solver
   int vsize = 8;   // bytes per MG vector entry
   std::vector<fb::DevLevel> lv;
   std::vector<void*> allocs;
+  // the block that small arrays are taken from: what is left of it, the next one's size
+  unsigned char* block = nullptr;
+  size_t block_left = 0, block_next = size_t(2) << 20;
   std::vector<std::vector<uint32_t>> perms;   // per level; empty = identity
   // coarse
   uint32_t* free_dofs = nullptr;
@@ -1808,18 +1811,41 @@ struct fb_solver
 
 namespace fb
 {
+  // Zeroed device memory of the solver's own, with 64 bytes behind it (16-byte copies may round up into
+  // them).  Arrays of at most BLOCK_MAX bytes share blocks of 2 to 32 MB: an allocation each made the
+  // driver map memory about ten times per solver, 0.4 ms each on an idle host and several on a busy one
+  // (creating a 2D level-7 solver 6.1 ms and up to 17, against 5.1).
+  constexpr size_t BLOCK_MAX = size_t(4) << 20;
   static fb_status dalloc(fb_solver* s, void** p, size_t bytes)
   {
-    cudaError_t e = cudaMalloc(p, bytes + 64);
-    if(e != cudaSuccess)
+    const size_t need = (bytes + 64 + 255) & ~size_t(255);
+    const bool own = need > BLOCK_MAX;
+    if(own || need > s->block_left)
     {
-      set_error(std::string("cudaMalloc: ") + cudaGetErrorString(e));
-      return FB_ERR_NOMEM;
+      const size_t size = own ? need : std::max(need, s->block_next);
+      void* q = nullptr;
+      cudaError_t e = cudaMalloc(&q, size);
+      if(e != cudaSuccess)
+      {
+        set_error(std::string("cudaMalloc: ") + cudaGetErrorString(e));
+        return FB_ERR_NOMEM;
+      }
+      s->allocs.push_back(q);
+      e = cudaMemset(q, 0, size);
+      if(e != cudaSuccess)
+        return cuda_fail(e, "cudaMemset");
+      if(own)
+      {
+        *p = q;
+        return FB_OK;
+      }
+      s->block = static_cast<unsigned char*>(q);
+      s->block_left = size;
+      s->block_next = std::min(size_t(32) << 20, 2 * s->block_next);
     }
-    s->allocs.push_back(*p);
-    e = cudaMemset(*p, 0, bytes + 64);
-    if(e != cudaSuccess)
-      return cuda_fail(e, "cudaMemset");
+    *p = s->block;
+    s->block += need;
+    s->block_left -= need;
     return FB_OK;
   }
 
