@@ -350,7 +350,8 @@ namespace un
       zeros = make_uint4(0u, 0u, 0u, 0u);
 
     // the weights that stay are fetched before the wait for the kernel ahead: no kernel that is followed
-    // by a convolution directly writes them
+    // by a convolution directly writes them, and none lets its dependents start before its own wait is over
+    // (dependents start when every block has exited), so the kernels before it have ended
     if constexpr(C == 8)
       load_w(0, 0);
     else if constexpr(NST == 9)
