@@ -1762,7 +1762,7 @@ struct fb_solver
   std::vector<void*> allocs;
   // the block that small arrays are taken from: what is left of it, the next one's size
   unsigned char* block = nullptr;
-  size_t block_left = 0, block_next = size_t(2) << 20;
+  size_t block_left = 0, block_next = size_t(1) << 20;
   std::vector<std::vector<uint32_t>> perms;   // per level; empty = identity
   // coarse
   uint32_t* free_dofs = nullptr;
@@ -1812,9 +1812,10 @@ struct fb_solver
 namespace fb
 {
   // Zeroed device memory of the solver's own, with 64 bytes behind it (16-byte copies may round up into
-  // them).  Arrays of at most BLOCK_MAX bytes share blocks of 2 to 32 MB: an allocation each made the
-  // driver map memory about ten times per solver, 0.4 ms each on an idle host and several on a busy one
-  // (creating a 2D level-7 solver 6.1 ms and up to 17, against 5.1).
+  // them).  Arrays of at most BLOCK_MAX bytes share blocks of 1 to 32 MB: an allocation and a memset each took
+  // 1 ms of the 6.1 that creating a 2D level-7 solver took (5.2 with blocks), 0.3 of the 0.9 for level 4 (0.6).
+  // The driver maps memory, 0.4 ms on an idle host and several on a busy one, no more often than it did; a
+  // first block of 2 MB would always make it, one of 0.5 MB more often at level 5.
   constexpr size_t BLOCK_MAX = size_t(4) << 20;
   static fb_status dalloc(fb_solver* s, void** p, size_t bytes)
   {
