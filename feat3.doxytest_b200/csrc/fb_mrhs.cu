@@ -987,6 +987,8 @@ namespace mr
   {
     std::vector<uint32_t> rp(size_t(M.rows) + 1, 0), col;
     std::vector<double> val;
+    col.reserve(M.col.size());
+    val.reserve(M.col.size());
     for(uint32_t r = 0; r < M.rows; ++r)
     {
       if(!(empty && (*empty)[r]))
