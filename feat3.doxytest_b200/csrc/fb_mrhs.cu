@@ -52,9 +52,11 @@ namespace mr
   __device__ __forceinline__ uint32_t warp_id() { return threadIdx.x >> 5; }
   __device__ __forceinline__ uint32_t warps() { return blockDim.x >> 5; }
 
-  // 64 right-hand sides in FP64: an x row is 512 bytes and the x rows around an SM's rows outgrow its
-  // L1, so the rows are swept twice, 32 right-hand sides each time
-  template<typename S, int R> struct Half { static constexpr bool value = sizeof(S) == 8 && R == 2; };
+  // 64 right-hand sides in FP64 in the stencil form: an x row is 512 bytes and the x rows around an SM's
+  // strips outgrow its L1, so the rows are swept twice, 32 right-hand sides each time.  (Not in CSR form, whose
+  // entries would be read and broadcast twice: ten iterations, 2D level 7 1,663 -> 1,442 us, 3D level 5 with
+  // coarse vertices first 2,287 -> 1,840.)
+  template<typename S, int R, int G> struct Half { static constexpr bool value = sizeof(S) == 8 && R == 2 && G > 0; };
 
   // A matrix in CSR form and, for a system matrix whose stored rows all share one pattern of 9 or
   // 27 column offsets made of triplets (o-1, o, o+1) -- the Q1 stencil of a lexicographically
@@ -324,7 +326,7 @@ namespace mr
   {
     typedef typename ValueTraits<V>::acc Ac;
     constexpr int K = 32 * R;
-    constexpr bool H = Half<S, R>::value;
+    constexpr bool H = Half<S, R, G>::value;
     constexpr int RR = H ? 1 : R;
     const int lane = threadIdx.x & 31;
     #pragma unroll 1
@@ -399,7 +401,7 @@ namespace mr
     constexpr int K = 32 * R;
     if(closed(sc))
       return;
-    constexpr int RR = Half<S, R>::value ? 1 : R;
+    constexpr int RR = Half<S, R, G>::value ? 1 : R;
     for_rows<V, S, R, G>(A, x, [&](uint32_t row, int j0, int, const Ac (&sum)[RR])
     {
       const bool d = __ldg(dm + row) != 0;
@@ -427,7 +429,7 @@ namespace mr
     constexpr int K = 32 * R;
     if(closed(sc))
       return;
-    constexpr int RR = Half<S, R>::value ? 1 : R;
+    constexpr int RR = Half<S, R, G>::value ? 1 : R;
     for_rows<V, S, R, G>(A, x, [&](uint32_t row, int j0, int, const Ac (&sum)[RR])
     {
       const bool d = __ldg(dm + row) != 0;
@@ -540,7 +542,7 @@ namespace mr
     #pragma unroll
     for(int r = 0; r < R; ++r)
       part[r] = 0.0;
-    constexpr int RR = Half<S, R>::value ? 1 : R;
+    constexpr int RR = Half<S, R, G>::value ? 1 : R;
     for_rows<V, S, R, G>(A, x, [&](uint32_t row, int j0, int q, const Ac (&sum)[RR])
     {
       const bool d = __ldg(dm + row) != 0;
@@ -560,7 +562,7 @@ namespace mr
       st_vec<S, RR>(dv + e, dvo);
       st_vec<S, RR>(cv + e, cvo);
     });
-    reduce_per_rhs<R, Half<S, R>::value>(part, sc, [&](int j, double tot) { skip[j] = skip_of<S>(sqrt(tot)); });
+    reduce_per_rhs<R, Half<S, R, G>::value>(part, sc, [&](int j, double tot) { skip[j] = skip_of<S>(sqrt(tot)); });
   }
 
   template<typename V, typename S, int R, bool LAST, bool TOP, int G>
@@ -576,7 +578,7 @@ namespace mr
     #pragma unroll
     for(int r = 0; r < R; ++r)
       part[r] = 0.0;
-    constexpr int RR = Half<S, R>::value ? 1 : R;
+    constexpr int RR = Half<S, R, G>::value ? 1 : R;
     for_rows<V, S, R, G>(A, cv, [&](uint32_t row, int j0, int q, const Ac (&sum)[RR])
     {
       const bool d = __ldg(dm + row) != 0;
@@ -618,7 +620,7 @@ namespace mr
     });
     if(!(LAST && TOP))
       return;
-    reduce_per_rhs<R, Half<S, R>::value>(part, sc, [&](int j, double tot)
+    reduce_per_rhs<R, Half<S, R, G>::value>(part, sc, [&](int j, double tot)
     {
       sc->gamma_prev[j] = sc->gamma[j];
       sc->gamma[j] = tot;
@@ -646,7 +648,7 @@ namespace mr
     #pragma unroll
     for(int r = 0; r < R; ++r)
       part[r] = 0.0;
-    constexpr int RR = Half<double, R>::value ? 1 : R;
+    constexpr int RR = Half<double, R, G>::value ? 1 : R;
     for_rows<double, double, R, G>(A, x, [&](uint32_t row, int j0, int q, const double (&sum)[RR])
     {
       const bool d = __ldg(dm + row) != 0;
@@ -667,7 +669,7 @@ namespace mr
       if(x1)
         st_vec<S, RR>(x1 + e, xo);
     });
-    reduce_per_rhs<R, Half<double, R>::value>(part, sc, [&](int j, double tot)
+    reduce_per_rhs<R, Half<double, R, G>::value>(part, sc, [&](int j, double tot)
     {
       const double d0 = sqrt(tot);
       sc->def_init[j] = d0;
@@ -760,7 +762,7 @@ namespace mr
     #pragma unroll
     for(int r = 0; r < R; ++r)
       part[r] = 0.0;
-    constexpr int RR = Half<double, R>::value ? 1 : R;
+    constexpr int RR = Half<double, R, G>::value ? 1 : R;
     for_rows<double, double, R, G>(A, p, [&](uint32_t row, int j0, int qi, const double (&sum)[RR])
     {
       const bool d = __ldg(dm + row) != 0;
@@ -775,7 +777,7 @@ namespace mr
       }
       st_vec<double, RR>(q + e, qo);
     });
-    reduce_per_rhs<R, Half<double, R>::value>(part, sc, [&](int j, double tot) { sc->alpha[j] = sc->gamma[j] / tot; });
+    reduce_per_rhs<R, Half<double, R, G>::value>(part, sc, [&](int j, double tot) { sc->alpha[j] = sc->gamma[j] / tot; });
   }
 
   // per right-hand side still in progress: x += alpha p, r -= alpha q; ||r||, stopping test; the
