@@ -52,12 +52,6 @@ namespace mr
   __device__ __forceinline__ uint32_t warp_id() { return threadIdx.x >> 5; }
   __device__ __forceinline__ uint32_t warps() { return blockDim.x >> 5; }
 
-  // 64 right-hand sides in FP64 in the stencil form: an x row is 512 bytes and the x rows around an SM's
-  // strips outgrow its L1, so the rows are swept twice, 32 right-hand sides each time.  (Not in CSR form, whose
-  // entries would be read and broadcast twice: ten iterations, 2D level 7 1,663 -> 1,442 us, 3D level 5 with
-  // coarse vertices first 2,287 -> 1,840.)
-  template<typename S, int R, int G> struct Half { static constexpr bool value = sizeof(S) == 8 && R == 2 && G > 0; };
-
   // A matrix in CSR form and, for a system matrix whose stored rows all share one pattern of 9 or
   // 27 column offsets made of triplets (o-1, o, o+1) -- the Q1 stencil of a lexicographically
   // numbered grid -- also in stencil form: dval[k * dn + row] is entry k of the row (zeros for rows
@@ -161,15 +155,6 @@ namespace mr
       *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
     else
       *p = v[0];
-  }
-
-  // part[k] += v with k known only by its range (a select each: the array stays in registers)
-  template<int R>
-  __device__ __forceinline__ void sum_to(double (&part)[R], int k, double v)
-  {
-    #pragma unroll
-    for(int r = 0; r < R; ++r)
-      part[r] += k == r ? v : 0.0;
   }
 
   template<typename S> __device__ __forceinline__ double epsq();
@@ -317,42 +302,34 @@ namespace mr
     }
   }
 
-  // epi(row, j0, q, sum) for every row of A, with sum[r] = (A x)[row][j0 + r] and q the first of the
-  // thread's partial sums they go to: in the stencil form with G = 9 or 3 triplets per row, in the CSR
-  // form for G = 0.  The form is a template parameter of every matrix pass, so the CSR instances keep
-  // the registers (and the resident warps) of the row kernel.
+  // epi(row, j0, sum) for every row of A, with sum[r] = (A x)[row][j0 + r]: in the stencil form with G = 9 or
+  // 3 triplets per row, in the CSR form for G = 0.  The form is a template parameter of every matrix pass, so
+  // the CSR instances keep the registers (and the resident warps) of the row kernel.
   template<typename V, typename S, int R, int G, class Epi>
   __device__ __forceinline__ void for_rows(const MCsr<V>& A, const S* __restrict__ x, Epi epi)
   {
     typedef typename ValueTraits<V>::acc Ac;
     constexpr int K = 32 * R;
-    constexpr bool H = Half<S, R, G>::value;
-    constexpr int RR = H ? 1 : R;
-    const int lane = threadIdx.x & 31;
-    #pragma unroll 1
-    for(int h = 0; h < (H ? 2 : 1); ++h)
+    const int j0 = (threadIdx.x & 31) * R;
+    auto one = [&](uint32_t row, const Ac (&sum)[R]) { epi(row, j0, sum); };
+    if constexpr(G > 0)
+      strip_rows<V, S, R, K, G>(A, x, j0, one);
+    else
     {
-      const int j0 = H ? 32 * h + lane : lane * R;
-      auto one = [&](uint32_t row, const Ac (&sum)[RR]) { epi(row, j0, h, sum); };
-      if constexpr(G > 0)
-        strip_rows<V, S, RR, K, G>(A, x, j0, one);
-      else
+      const Range rg(A.rows);
+      for(uint32_t row = rg.first + warp_id(); row < rg.end; row += warps())
       {
-        const Range rg(A.rows);
-        for(uint32_t row = rg.first + warp_id(); row < rg.end; row += warps())
-        {
-          Ac sum[RR];
-          mrow<V, S, RR, K>(A, row, x, j0, sum);
-          one(row, sum);
-        }
+        Ac sum[R];
+        mrow<V, S, R, K>(A, row, x, j0, sum);
+        one(row, sum);
       }
     }
   }
 
   // block partials per right-hand side (smem), atomically added to sc->acc; the last block calls
   // fin(j, total) for every j < K and clears the accumulators.  part[r] belongs to right-hand side
-  // lane R + r, or with H (Half) to 32 r + lane.
-  template<int R, bool H = false, class Fin>
+  // lane R + r.
+  template<int R, class Fin>
   __device__ __forceinline__ void reduce_per_rhs(const double (&part)[R], MScal* sc, Fin fin)
   {
     constexpr int K = 32 * R;
@@ -361,7 +338,7 @@ namespace mr
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     #pragma unroll
     for(int r = 0; r < R; ++r)
-      red[warp][H ? 32 * r + lane : lane * R + r] = part[r];
+      red[warp][lane * R + r] = part[r];
     __syncthreads();
     if(threadIdx.x < K)
     {
@@ -401,23 +378,22 @@ namespace mr
     constexpr int K = 32 * R;
     if(closed(sc))
       return;
-    constexpr int RR = Half<S, R, G>::value ? 1 : R;
-    for_rows<V, S, R, G>(A, x, [&](uint32_t row, int j0, int, const Ac (&sum)[RR])
+    for_rows<V, S, R, G>(A, x, [&](uint32_t row, int j0, const Ac (&sum)[R])
     {
       const bool d = __ldg(dm + row) != 0;
       const Ac di = Ac(__ldg(dinv + row));
       const size_t e = size_t(row) * K + j0;
-      S bv[RR], xv[RR], out[RR];
-      ld_vec<S, RR>(b + e, bv);
-      ldg_row<S, RR>(x + e, xv);
+      S bv[R], xv[R], out[R];
+      ld_vec<S, R>(b + e, bv);
+      ldg_row<S, R>(x + e, xv);
       #pragma unroll
-      for(int r = 0; r < RR; ++r)
+      for(int r = 0; r < R; ++r)
       {
         const Ac d1 = d ? Ac(0) : sub(Ac(bv[r]), sum[r]);
         const Ac c = d ? Ac(0) : mul(di, d1);
         out[r] = skip[j0 + r] ? S(0) : S(add(Ac(xv[r]), c));
       }
-      st_vec<S, RR>(xo + e, out);
+      st_vec<S, R>(xo + e, out);
     });
   }
 
@@ -429,17 +405,16 @@ namespace mr
     constexpr int K = 32 * R;
     if(closed(sc))
       return;
-    constexpr int RR = Half<S, R, G>::value ? 1 : R;
-    for_rows<V, S, R, G>(A, x, [&](uint32_t row, int j0, int, const Ac (&sum)[RR])
+    for_rows<V, S, R, G>(A, x, [&](uint32_t row, int j0, const Ac (&sum)[R])
     {
       const bool d = __ldg(dm + row) != 0;
       const size_t e = size_t(row) * K + j0;
-      S bv[RR], out[RR];
-      ld_vec<S, RR>(b + e, bv);
+      S bv[R], out[R];
+      ld_vec<S, R>(b + e, bv);
       #pragma unroll
-      for(int r = 0; r < RR; ++r)
+      for(int r = 0; r < R; ++r)
         out[r] = d ? S(0) : S(sub(Ac(bv[r]), sum[r]));
-      st_vec<S, RR>(dv + e, out);
+      st_vec<S, R>(dv + e, out);
     });
   }
 
@@ -542,27 +517,26 @@ namespace mr
     #pragma unroll
     for(int r = 0; r < R; ++r)
       part[r] = 0.0;
-    constexpr int RR = Half<S, R, G>::value ? 1 : R;
-    for_rows<V, S, R, G>(A, x, [&](uint32_t row, int j0, int q, const Ac (&sum)[RR])
+    for_rows<V, S, R, G>(A, x, [&](uint32_t row, int j0, const Ac (&sum)[R])
     {
       const bool d = __ldg(dm + row) != 0;
       const Ac di = Ac(__ldg(dinv + row));
       const size_t e = size_t(row) * K + j0;
-      S bv[RR], dvo[RR], cvo[RR];
-      ld_vec<S, RR>(b + e, bv);
+      S bv[R], dvo[R], cvo[R];
+      ld_vec<S, R>(b + e, bv);
       #pragma unroll
-      for(int r = 0; r < RR; ++r)
+      for(int r = 0; r < R; ++r)
       {
         const Ac dd = d ? Ac(0) : sub(Ac(bv[r]), sum[r]);
         dvo[r] = S(dd);
         const Ac c = d ? Ac(0) : mul(di, dd);
         cvo[r] = S(add(Ac(0), c));
-        sum_to(part, q + r, double(dd) * double(dd));
+        part[r] += double(dd) * double(dd);
       }
-      st_vec<S, RR>(dv + e, dvo);
-      st_vec<S, RR>(cv + e, cvo);
+      st_vec<S, R>(dv + e, dvo);
+      st_vec<S, R>(cv + e, cvo);
     });
-    reduce_per_rhs<R, Half<S, R, G>::value>(part, sc, [&](int j, double tot) { skip[j] = skip_of<S>(sqrt(tot)); });
+    reduce_per_rhs<R>(part, sc, [&](int j, double tot) { skip[j] = skip_of<S>(sqrt(tot)); });
   }
 
   template<typename V, typename S, int R, bool LAST, bool TOP, int G>
@@ -578,22 +552,21 @@ namespace mr
     #pragma unroll
     for(int r = 0; r < R; ++r)
       part[r] = 0.0;
-    constexpr int RR = Half<S, R, G>::value ? 1 : R;
-    for_rows<V, S, R, G>(A, cv, [&](uint32_t row, int j0, int q, const Ac (&sum)[RR])
+    for_rows<V, S, R, G>(A, cv, [&](uint32_t row, int j0, const Ac (&sum)[R])
     {
       const bool d = __ldg(dm + row) != 0;
       const Ac di = Ac(__ldg(dinv + row));
       const size_t e = size_t(row) * K + j0;
-      S dvv[RR], cvv[RR], out[RR];
-      double rv[RR], zo[RR];
-      ld_vec<S, RR>(dv + e, dvv);
-      ldg_row<S, RR>(cv + e, cvv);
+      S dvv[R], cvv[R], out[R];
+      double rv[R], zo[R];
+      ld_vec<S, R>(dv + e, dvv);
+      ldg_row<S, R>(cv + e, cvv);
       if constexpr(LAST)
-        ld_vec<S, RR>(x + e, out);
+        ld_vec<S, R>(x + e, out);
       if constexpr(LAST && TOP)
-        ld_vec<double, RR>(rr + e, rv);
+        ld_vec<double, R>(rr + e, rv);
       #pragma unroll
-      for(int r = 0; r < RR; ++r)
+      for(int r = 0; r < R; ++r)
       {
         const Ac dk = d ? Ac(0) : sub(Ac(dvv[r]), sum[r]);
         const Ac ck = d ? Ac(0) : mul(di, dk);
@@ -607,20 +580,20 @@ namespace mr
           if constexpr(TOP)
           {
             zo[r] = mul(double(xn), sc->inv_scale[j0 + r]);
-            sum_to(part, q + r, mul(rv[r], zo[r]));
+            part[r] += mul(rv[r], zo[r]);
           }
         }
       }
       if constexpr(!LAST)
-        st_vec<S, RR>(co + e, out);
+        st_vec<S, R>(co + e, out);
       else if constexpr(TOP)
-        st_vec<double, RR>(z + e, zo);
+        st_vec<double, R>(z + e, zo);
       else
-        st_vec<S, RR>(x + e, out);
+        st_vec<S, R>(x + e, out);
     });
     if(!(LAST && TOP))
       return;
-    reduce_per_rhs<R, Half<S, R, G>::value>(part, sc, [&](int j, double tot)
+    reduce_per_rhs<R>(part, sc, [&](int j, double tot)
     {
       sc->gamma_prev[j] = sc->gamma[j];
       sc->gamma[j] = tot;
@@ -648,28 +621,27 @@ namespace mr
     #pragma unroll
     for(int r = 0; r < R; ++r)
       part[r] = 0.0;
-    constexpr int RR = Half<double, R, G>::value ? 1 : R;
-    for_rows<double, double, R, G>(A, x, [&](uint32_t row, int j0, int q, const double (&sum)[RR])
+    for_rows<double, double, R, G>(A, x, [&](uint32_t row, int j0, const double (&sum)[R])
     {
       const bool d = __ldg(dm + row) != 0;
       const size_t e = size_t(row) * K + j0;
-      double bv[RR];
-      S xo[RR];
-      ld_vec<double, RR>(rhs + e, bv);
+      double bv[R];
+      S xo[R];
+      ld_vec<double, R>(rhs + e, bv);
       #pragma unroll
-      for(int r = 0; r < RR; ++r)
+      for(int r = 0; r < R; ++r)
       {
         const double rv = d ? 0.0 : sub(bv[r], sum[r]);
         bv[r] = rv;
         const S c = d || !x1 ? S(0) : mul(__ldg(dinv + row), S(rv));
         xo[r] = add(S(0), c);
-        sum_to(part, q + r, mul(rv, rv));
+        part[r] += mul(rv, rv);
       }
-      st_vec<double, RR>(rr + e, bv);
+      st_vec<double, R>(rr + e, bv);
       if(x1)
-        st_vec<S, RR>(x1 + e, xo);
+        st_vec<S, R>(x1 + e, xo);
     });
-    reduce_per_rhs<R, Half<double, R, G>::value>(part, sc, [&](int j, double tot)
+    reduce_per_rhs<R>(part, sc, [&](int j, double tot)
     {
       const double d0 = sqrt(tot);
       sc->def_init[j] = d0;
@@ -762,22 +734,21 @@ namespace mr
     #pragma unroll
     for(int r = 0; r < R; ++r)
       part[r] = 0.0;
-    constexpr int RR = Half<double, R, G>::value ? 1 : R;
-    for_rows<double, double, R, G>(A, p, [&](uint32_t row, int j0, int qi, const double (&sum)[RR])
+    for_rows<double, double, R, G>(A, p, [&](uint32_t row, int j0, const double (&sum)[R])
     {
       const bool d = __ldg(dm + row) != 0;
       const size_t e = size_t(row) * K + j0;
-      double pv[RR], qo[RR];
-      ldg_row<double, RR>(p + e, pv);
+      double pv[R], qo[R];
+      ldg_row<double, R>(p + e, pv);
       #pragma unroll
-      for(int r = 0; r < RR; ++r)
+      for(int r = 0; r < R; ++r)
       {
         qo[r] = d ? 0.0 : add(sum[r], 0.0);
-        sum_to(part, qi + r, mul(qo[r], pv[r]));
+        part[r] += mul(qo[r], pv[r]);
       }
-      st_vec<double, RR>(q + e, qo);
+      st_vec<double, R>(q + e, qo);
     });
-    reduce_per_rhs<R, Half<double, R, G>::value>(part, sc, [&](int j, double tot) { sc->alpha[j] = sc->gamma[j] / tot; });
+    reduce_per_rhs<R>(part, sc, [&](int j, double tot) { sc->alpha[j] = sc->gamma[j] / tot; });
   }
 
   // per right-hand side still in progress: x += alpha p, r -= alpha q; ||r||, stopping test; the
