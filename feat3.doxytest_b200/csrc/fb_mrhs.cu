@@ -52,6 +52,38 @@ namespace mr
   __device__ __forceinline__ uint32_t warp_id() { return threadIdx.x >> 5; }
   __device__ __forceinline__ uint32_t warps() { return blockDim.x >> 5; }
 
+  // The rows of this warp: contiguous ranges per block, or (SPREAD) dealt out row by row over all warps, whose
+  // x rows then meet in L2.  Large levels in CSR form take the second, in blocks of 256 with 32 registers, all
+  // the warps an SM holds: ranges let every SM read a region of its own, which saves L1 misses on small levels
+  // and costs L2 hits on large ones.  Contiguous -> dealt out, one
+  // solve, FP32, 32 right-hand sides: 2D level 9 coarse vertices first 7,205 -> 5,574 us, reordered by RCM 6,827 ->
+  // 5,531, lexicographic in CSR form 6,801 -> 5,508, 3D level 6 8,937 -> 6,789; 2D level 8 2,406 -> 2,295; 3D level
+  // 5 with 64 columns 1,602 -> 1,686.
+  template<bool SPREAD>
+  struct Rows
+  {
+    uint32_t first, end, step;
+    __device__ explicit Rows(uint32_t n)
+    {
+      if(SPREAD)
+      {
+        first = blockIdx.x * warps() + warp_id();
+        end = n;
+        step = gridDim.x * warps();
+      }
+      else
+      {
+        const Range r(n);
+        first = r.first + warp_id();
+        end = r.end;
+        step = warps();
+      }
+    }
+  };
+#define MR_ROWS(SPREAD, n) \
+  const Rows<SPREAD> rg_(n); \
+  for(uint32_t row = rg_.first; row < rg_.end; row += rg_.step)
+
   // A matrix in CSR form and, for a system matrix whose stored rows all share one pattern of 9 or
   // 27 column offsets made of triplets (o-1, o, o+1) -- the Q1 stencil of a lexicographically
   // numbered grid -- also in stencil form: dval[k * dn + row] is entry k of the row (zeros for rows
@@ -303,8 +335,8 @@ namespace mr
   }
 
   // epi(row, j0, sum) for every row of A, with sum[r] = (A x)[row][j0 + r]: in the stencil form with G = 9 or
-  // 3 triplets per row, in the CSR form for G = 0.  The form is a template parameter of every matrix pass, so
-  // the CSR instances keep the registers (and the resident warps) of the row kernel.
+  // 3 triplets per row, in the CSR form for G = 0 (contiguous ranges) and G = -1 (rows dealt out).  The form is a
+  // template parameter of every matrix pass, so that each keeps its own registers (and resident warps).
   template<typename V, typename S, int R, int G, class Epi>
   __device__ __forceinline__ void for_rows(const MCsr<V>& A, const S* __restrict__ x, Epi epi)
   {
@@ -316,8 +348,7 @@ namespace mr
       strip_rows<V, S, R, K, G>(A, x, j0, one);
     else
     {
-      const Range rg(A.rows);
-      for(uint32_t row = rg.first + warp_id(); row < rg.end; row += warps())
+      MR_ROWS(G < 0, A.rows)
       {
         Ac sum[R];
         mrow<V, S, R, K>(A, row, x, j0, sum);
@@ -329,11 +360,11 @@ namespace mr
   // block partials per right-hand side (smem), atomically added to sc->acc; the last block calls
   // fin(j, total) for every j < K and clears the accumulators.  part[r] belongs to right-hand side
   // lane R + r.
-  template<int R, class Fin>
+  template<int R, int NW = MW_MAX, class Fin>
   __device__ __forceinline__ void reduce_per_rhs(const double (&part)[R], MScal* sc, Fin fin)
   {
     constexpr int K = 32 * R;
-    __shared__ double red[MW_MAX][K];
+    __shared__ double red[NW][K];
     __shared__ bool last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     #pragma unroll
@@ -365,12 +396,8 @@ namespace mr
       sc->arrive = 0u;
   }
 
-#define MR_ROWS(n) \
-  const Range rg_(n); \
-  for(uint32_t row = rg_.first + warp_id(); row < rg_.end; row += warps())
-
   template<typename V, typename S, int R, int G>
-  __global__ void __launch_bounds__(MNT_BIG, 1) km_smooth(MCsr<V> A, const S* __restrict__ b, const S* __restrict__ x,
+  __global__ void __launch_bounds__(G < 0 ? MNT : MNT_BIG, G < 0 ? 8 : 1) km_smooth(MCsr<V> A, const S* __restrict__ b, const S* __restrict__ x,
     S* __restrict__ xo, const S* __restrict__ dinv, const uint8_t* __restrict__ dm, const int* __restrict__ skip,
     const MScal* __restrict__ sc)
   {
@@ -398,7 +425,7 @@ namespace mr
   }
 
   template<typename V, typename S, int R, int G>
-  __global__ void __launch_bounds__(MNT_BIG, 1) km_defect(MCsr<V> A, const S* __restrict__ b, const S* __restrict__ x,
+  __global__ void __launch_bounds__(G < 0 ? MNT : MNT_BIG, G < 0 ? 8 : 1) km_defect(MCsr<V> A, const S* __restrict__ b, const S* __restrict__ x,
     S* __restrict__ dv, const uint8_t* __restrict__ dm, const MScal* __restrict__ sc)
   {
     typedef typename ValueTraits<V>::acc Ac;
@@ -418,8 +445,8 @@ namespace mr
     });
   }
 
-  template<typename V, typename S, int R>
-  __global__ void __launch_bounds__(MNT_BIG, 1) km_restrict(MCsr<V> Rm, const S* __restrict__ dv, S* __restrict__ bc,
+  template<typename V, typename S, int R, bool SPREAD>
+  __global__ void __launch_bounds__(SPREAD ? MNT : MNT_BIG, SPREAD ? 8 : 1) km_restrict(MCsr<V> Rm, const S* __restrict__ dv, S* __restrict__ bc,
     S* __restrict__ xc, const S* __restrict__ dinvc, const uint8_t* __restrict__ dmc, int* __restrict__ skipc,
     MScal* __restrict__ sc)
   {
@@ -432,7 +459,7 @@ namespace mr
     #pragma unroll
     for(int r = 0; r < R; ++r)
       part[r] = 0.0;
-    MR_ROWS(Rm.rows)
+    MR_ROWS(SPREAD, Rm.rows)
     {
       Ac sum[R];
       mrow<V, S, R, K>(Rm, row, dv, lane * R, sum);
@@ -454,7 +481,7 @@ namespace mr
     }
     if(!xc)
       return;
-    reduce_per_rhs<R>(part, sc, [&](int j, double tot) { skipc[j] = skip_of<S>(sqrt(tot)); });
+    reduce_per_rhs<R, SPREAD ? MW : MW_MAX>(part, sc, [&](int j, double tot) { skipc[j] = skip_of<S>(sqrt(tot)); });
   }
 
   template<typename S, int R>
@@ -477,8 +504,8 @@ namespace mr
     }
   }
 
-  template<typename V, typename S, int R>
-  __global__ void __launch_bounds__(MNT_BIG, 1) km_prolong(MCsr<V> P, const S* __restrict__ xc, S* __restrict__ x,
+  template<typename V, typename S, int R, bool SPREAD>
+  __global__ void __launch_bounds__(SPREAD ? MNT : MNT_BIG, SPREAD ? 8 : 1) km_prolong(MCsr<V> P, const S* __restrict__ xc, S* __restrict__ x,
     const uint8_t* __restrict__ dm, const MScal* __restrict__ sc)
   {
     typedef typename ValueTraits<V>::acc Ac;
@@ -486,7 +513,7 @@ namespace mr
     if(closed(sc))
       return;
     const int lane = threadIdx.x & 31;
-    MR_ROWS(P.rows)
+    MR_ROWS(SPREAD, P.rows)
     {
       Ac sum[R];
       S xv[R];
@@ -505,7 +532,7 @@ namespace mr
   }
 
   template<typename V, typename S, int R, int G>
-  __global__ void __launch_bounds__(MNT_BIG, 1) km_post1(MCsr<V> A, const S* __restrict__ b, const S* __restrict__ x,
+  __global__ void __launch_bounds__(G < 0 ? MNT : MNT_BIG, G < 0 ? 8 : 1) km_post1(MCsr<V> A, const S* __restrict__ b, const S* __restrict__ x,
     S* __restrict__ dv, S* __restrict__ cv, const S* __restrict__ dinv, const uint8_t* __restrict__ dm,
     int* __restrict__ skip, MScal* __restrict__ sc)
   {
@@ -536,11 +563,11 @@ namespace mr
       st_vec<S, R>(dv + e, dvo);
       st_vec<S, R>(cv + e, cvo);
     });
-    reduce_per_rhs<R>(part, sc, [&](int j, double tot) { skip[j] = skip_of<S>(sqrt(tot)); });
+    reduce_per_rhs<R, G < 0 ? MW : MW_MAX>(part, sc, [&](int j, double tot) { skip[j] = skip_of<S>(sqrt(tot)); });
   }
 
   template<typename V, typename S, int R, bool LAST, bool TOP, int G>
-  __global__ void __launch_bounds__(MNT_BIG, 1) km_post2(MCsr<V> A, const S* __restrict__ dv, const S* __restrict__ cv,
+  __global__ void __launch_bounds__(G < 0 ? MNT : MNT_BIG, G < 0 ? 8 : 1) km_post2(MCsr<V> A, const S* __restrict__ dv, const S* __restrict__ cv,
     S* __restrict__ co, S* __restrict__ x, double* __restrict__ z, const double* __restrict__ rr,
     const S* __restrict__ dinv, const uint8_t* __restrict__ dm, const int* __restrict__ skip, MScal* __restrict__ sc)
   {
@@ -593,7 +620,7 @@ namespace mr
     });
     if(!(LAST && TOP))
       return;
-    reduce_per_rhs<R>(part, sc, [&](int j, double tot)
+    reduce_per_rhs<R, G < 0 ? MW : MW_MAX>(part, sc, [&](int j, double tot)
     {
       sc->gamma_prev[j] = sc->gamma[j];
       sc->gamma[j] = tot;
@@ -612,7 +639,7 @@ namespace mr
 
   // r = F(rhs - A x), norms -> def_init, status; FP64 mode: sol1 = F(D .* r)
   template<typename S, int R, int G>
-  __global__ void __launch_bounds__(MNT_BIG, 1) km_pcg_init(MCsr<double> A, const double* __restrict__ rhs,
+  __global__ void __launch_bounds__(G < 0 ? MNT : MNT_BIG, G < 0 ? 8 : 1) km_pcg_init(MCsr<double> A, const double* __restrict__ rhs,
     const double* __restrict__ x, double* __restrict__ rr, const uint8_t* __restrict__ dm, S* __restrict__ x1,
     const S* __restrict__ dinv, int* __restrict__ skip_top, MScal* __restrict__ sc)
   {
@@ -641,7 +668,7 @@ namespace mr
       if(x1)
         st_vec<S, R>(x1 + e, xo);
     });
-    reduce_per_rhs<R>(part, sc, [&](int j, double tot)
+    reduce_per_rhs<R, G < 0 ? MW : MW_MAX>(part, sc, [&](int j, double tot)
     {
       const double d0 = sqrt(tot);
       sc->def_init[j] = d0;
@@ -695,7 +722,7 @@ namespace mr
       scale[r] = pow2_inv(sc->def_cur[lane * R + r]);
       part[r] = 0.0;
     }
-    MR_ROWS(n)
+    MR_ROWS(false, n)
     {
       const bool d = __ldg(dm + row) != 0;
       const size_t e = size_t(row) * K + lane * R;
@@ -724,7 +751,7 @@ namespace mr
 
   // q = F(A p), q.p -> alpha
   template<int R, int G>
-  __global__ void __launch_bounds__(MNT_BIG, 1) km_pcg_q(MCsr<double> A, const double* __restrict__ p, double* __restrict__ q,
+  __global__ void __launch_bounds__(G < 0 ? MNT : MNT_BIG, G < 0 ? 8 : 1) km_pcg_q(MCsr<double> A, const double* __restrict__ p, double* __restrict__ q,
     const uint8_t* __restrict__ dm, MScal* __restrict__ sc)
   {
     constexpr int K = 32 * R;
@@ -748,7 +775,7 @@ namespace mr
       }
       st_vec<double, R>(q + e, qo);
     });
-    reduce_per_rhs<R>(part, sc, [&](int j, double tot) { sc->alpha[j] = sc->gamma[j] / tot; });
+    reduce_per_rhs<R, G < 0 ? MW : MW_MAX>(part, sc, [&](int j, double tot) { sc->alpha[j] = sc->gamma[j] / tot; });
   }
 
   // per right-hand side still in progress: x += alpha p, r -= alpha q; ||r||, stopping test; the
@@ -774,7 +801,7 @@ namespace mr
       scale[r] = CONVERT ? pow2_inv(sc->def_cur[j]) : 1.0;
       part[r] = 0.0;
     }
-    MR_ROWS(n)
+    MR_ROWS(false, n)
     {
       const bool d = __ldg(dm + row) != 0;
       const S di = __ldg(dinv + row);
@@ -837,7 +864,7 @@ namespace mr
     if(closed(sc))
       return;
     const int lane = threadIdx.x & 31;
-    MR_ROWS(n)
+    MR_ROWS(false, n)
     {
       const size_t e = size_t(row) * K + lane * R;
       double zv[R], pv[R];
@@ -899,6 +926,7 @@ struct fb_msolver
     uint32_t dn = 0;
     int nd = 0;
     int goff[9] = {};
+    bool spread = false;                   // CSR form, rows dealt out over all blocks (see upload_stencil)
   };
   struct Level
   {
@@ -1006,7 +1034,9 @@ namespace mr
     // strips to run (18,944 rows on 148 SMs).  Ten iterations, CSR against stencil form: 2D 16,641 rows, 64 right-hand
     // sides FP64 2,547 against 2,906 us; 3D 4,913 rows, 64 FP32 1,223 against 1,353; above the line 2D
     // 66,049 rows, 64 FP32 4,377 against 3,832; 3D 35,937 rows, 64 FP64 4,305 against 3,899
-    if(s->cfg.diagonal == 0 || (s->cfg.diagonal < 0 && d.rows < s->grid / 8u * uint32_t(MW_MAX * STRIP)))
+    const bool large = d.rows >= s->grid / 8u * uint32_t(MW_MAX * STRIP);
+    d.spread = large;   // in CSR form
+    if(s->cfg.diagonal == 0 || (s->cfg.diagonal < 0 && !large))
       return FB_OK;
     std::vector<int64_t> off;
     for(uint32_t r = 0; r < d.rows; ++r)
@@ -1039,6 +1069,7 @@ namespace mr
     }
     if(off.empty())
       return FB_OK;
+    d.spread = false;
     const int nd = int(off.size());
     const uint32_t dn = (d.rows + 7u) & ~7u;
     const size_t vb = prec == FB_PREC_F64 ? 8 : 4;
@@ -1092,7 +1123,7 @@ namespace mr
     template<typename W> Shape ga(const fb_msolver::Mat& m) const
     {
       if(!m.nd)
-        return shape(m.rows);
+        return m.spread ? flat(m.rows) : shape(m.rows);
       constexpr uint32_t M = STRIP;
       const uint32_t nsm = s->grid / 8u, n = (m.rows + M - 1) / M;
       if(n >= nsm * uint32_t(MNT_BIG / 32))
@@ -1110,12 +1141,22 @@ namespace mr
     // f(std::integral_constant<int, G>) with G the stored form of m: 9 or 3 stencil triplets, 0 = CSR
     template<typename W, class F> void by_form(const fb_msolver::Mat& m, F&& f) const
     {
-      if(m.nd == 27)
+      if(m.spread)
+        f(std::integral_constant<int, -1>());
+      else if(m.nd == 27)
         f(std::integral_constant<int, 9>());
       else if(m.nd == 9)
         f(std::integral_constant<int, 3>());
       else
         f(std::integral_constant<int, 0>());
+    }
+    // f(std::bool_constant): whether the level's rows are dealt out over all blocks
+    template<class F> void by_spread(const fb_msolver::Mat& m, F&& f) const
+    {
+      if(m.spread)
+        f(std::true_type());
+      else
+        f(std::false_type());
     }
     double vb(uint32_t n, double count) const { return double(n) * K * sizeof(S) * count; }
 
@@ -1150,8 +1191,11 @@ namespace mr
         bytes += mb(f.A) + vb(f.n, 3);
         const bool coarsest = (l + 2 == nl);
         if(!dry)
-          km_restrict<V, S, R><<<shape(c.n).g, shape(c.n).t, 0, st>>>(mv<V>(f.R), (const S*)f.d, (S*)c.b,
-            coarsest ? (S*)nullptr : (S*)c.x, (const S*)c.dinv, c.dm, c.skip_pre, s->sc);
+          by_spread(f.A, [&](auto sp) {
+            const Shape h = sp.value ? flat(c.n) : shape(c.n);
+            km_restrict<V, S, R, decltype(sp)::value><<<h.g, h.t, 0, st>>>(mv<V>(f.R), (const S*)f.d, (S*)c.b,
+              coarsest ? (S*)nullptr : (S*)c.x, (const S*)c.dinv, c.dm, c.skip_pre, s->sc);
+          });
         ++launches;
         bytes += mb(f.R) + vb(f.n, 1) + vb(c.n, 2);
       }
@@ -1168,7 +1212,11 @@ namespace mr
         fb_msolver::Level& f = s->lv[size_t(l)];
         void* xf = xcur[size_t(l)];
         if(!dry)
-          km_prolong<V, S, R><<<shape(f.n).g, shape(f.n).t, 0, st>>>(mv<V>(f.P), (const S*)xcur[size_t(l + 1)], (S*)xf, f.dm, s->sc);
+          by_spread(f.A, [&](auto sp) {
+            const Shape h = sp.value ? flat(f.n) : shape(f.n);
+            km_prolong<V, S, R, decltype(sp)::value><<<h.g, h.t, 0, st>>>(mv<V>(f.P), (const S*)xcur[size_t(l + 1)],
+              (S*)xf, f.dm, s->sc);
+          });
         if(!dry)
           by_form<V>(f.A, [&](auto gc) {
             km_post1<V, S, R, decltype(gc)::value><<<ga<V>(f.A).g, ga<V>(f.A).t, 0, st>>>(mv<V>(f.A), (const S*)f.b,

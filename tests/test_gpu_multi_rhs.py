@@ -134,3 +134,29 @@ def test_forms_of_large_levels(featlib, cuda, dim, level, K, precision):
         assert moved[None] == moved[False]
     else:
         assert moved[True] < moved[None] < moved[False]
+
+
+# large levels in numberings without the stencil's bands: rows dealt out over all blocks (66,049 and 35,937 rows), and
+# contiguous ranges below 18,944 rows
+@pytest.mark.parametrize("dim,level,ordering,K,precision", [
+    (2, 8, "native", 64, "f64"), (2, 8, "rcm", 32, "f32"), (3, 5, "native", 32, "f64"), (3, 5, "rcm", 64, "f32"),
+    (2, 7, "rcm", 64, "f64")])
+def test_coarse_vertices_first(featlib, cuda, dim, level, ordering, K, precision):
+    """Every right-hand side agrees with its own solve in a numbering with the coarse vertices first."""
+    torch, fb = cuda, featlib
+    from featb200 import assembly as AS
+    from test_gpu_batch import _coarse_first
+    lex, b = AS.poisson_hierarchy(level, dim, rhs="gauss", gauss=AS.gauss_params(9, dim))
+    levels, o = _coarse_first(lex, dim)
+    b = b[o]
+    rhs = torch.tensor(b[:, None] * np.random.default_rng(K).uniform(0.5, 2.0, K), device="cuda")
+    m = fb.MultiRhsPCG(fb.build_hierarchy(levels), K, precision=precision, ordering=ordering)
+    x = torch.zeros_like(rhs)
+    m.solve_device(x, rhs)
+    one = fb.build_pcg_multigrid(levels, precision=precision, ordering=ordering)
+    for j in (0, K // 2 - 1, K // 2, K - 1):
+        ref = torch.zeros(b.size, dtype=torch.float64, device="cuda")
+        assert one.correct_device(ref, rhs[:, j].contiguous()) == fb.Status.success == m.statuses()[j]
+        assert m.iterations()[j] == one.get_num_iter()
+        # only the order of the PCG's sums differs
+        assert rel_err(x[:, j].cpu().numpy(), ref.cpu().numpy()) <= (1e-12 if precision == "f64" else 1e-9)
