@@ -102,8 +102,7 @@ def test_multi_rhs_stencil_form(featlib, cuda, dim, level, precision):
 
 
 # the CSR and the stencil form of the system matrix: levels of 16,641 rows (too few strips to fill the
-# SMs) and of 66,049 and 35,937 (strips of four rows, the last one partial), FP64 with 64 right-hand
-# sides in two sweeps
+# SMs) and of 66,049 and 35,937 (strips of four rows, the last one partial; CSR rows dealt out over all blocks)
 @pytest.mark.parametrize("dim,level,K,precision", [(2, 7, 32, "f64"), (2, 8, 64, "f64"), (2, 8, 32, "f32"), (3, 5, 64, "f32")])
 def test_forms_of_large_levels(featlib, cuda, dim, level, K, precision):
     """Every right-hand side agrees with its own solve (kernel/solver/pcg.hpp:159-286); both forms and the
